@@ -1154,6 +1154,7 @@ static int ensure_plan(spk_handle* h) {
         cudaGetLastError();   // a refused query leaves clusters of 8
     }
     if (std::is_same<T, float>::value) {
+        CU(h, cudaFuncSetAttribute(spk::k_block_lu_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, spk::LuSmem::bytes));
         CU(h, cudaFuncSetAttribute(spk::k_tc_update<spk::TC_TRAIL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    spk::umma::PSMEM));
         CU(h, cudaFuncSetAttribute(spk::k_tc_update<spk::TC_SCHUR, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1371,6 +1372,9 @@ static int factor_launches(spk_handle* h, int fs_nrhs = 0) {
                         fac, h->d_ipiv, h->d_info, S, launch_of(PL, P.blu[t]), (int)t);
                 else if (h->lu_pieces && P.blu_pc[t])
                     spk::k_block_lu_pc<T><<<P.blu[t].tiles, spk::PC_THREADS, spk::PcLu<T>::smem, h->stream>>>(
+                        fac, h->d_ipiv, h->d_info, h->d_bmap, S, launch_of(PL, P.blu[t]), (int)t);
+                else if constexpr (std::is_same<T, float>::value)
+                    spk::k_block_lu_f32<<<P.blu[t].tiles, spk::LU_THREADS, spk::LuSmem::bytes, h->stream>>>(
                         fac, h->d_ipiv, h->d_info, h->d_bmap, S, launch_of(PL, P.blu[t]), (int)t);
                 else
                     spk::k_block_lu<T><<<P.blu[t].tiles, spk::LuThreads<T>::value, 0, h->stream>>>(

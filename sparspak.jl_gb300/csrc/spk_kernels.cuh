@@ -159,10 +159,21 @@ __device__ __forceinline__ int warp_first_max(unsigned long long key) {
 __device__ __forceinline__ float rcp_rn(float x) { return __frcp_rn(x); }
 __device__ __forceinline__ double rcp_rn(double x) { return __drcp_rn(x); }
 
+__device__ __forceinline__ float rcp_approx(float x) {   // normal x whose reciprocal is normal
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // Scaling factor 1 / pivot of the FP32 block LU: the hardware reciprocal
 // (within 2 ulp; the FP32 factor is refined in FP64); FP64 keeps the
-// correctly rounded one.
-__device__ __forceinline__ float lu_recip(float x) { return __fdividef(1.0f, x); }
+// correctly rounded one.  __fdividef covers the pivots whose reciprocal is
+// not normal; everywhere else it costs 140 cycles of a column's chain where
+// the bare instruction takes 20 (measured in a loop of one warp).
+__device__ __forceinline__ float lu_recip(float x) {
+    const float a = fabsf(x);
+    return a >= 1.1754944e-38f && a <= 8.5070592e37f ? rcp_approx(x) : __fdividef(1.0f, x);
+}
 __device__ __forceinline__ double lu_recip(double x) { return rcp_rn(x); }
 
 // The pivot lane of a column (first strict maximum of |x| among the
@@ -403,8 +414,8 @@ __device__ __forceinline__ void block_gather_map(const int* ipiv_blk, const int*
 }
 
 
-// Block LU by a whole CTA (blocks of 33..BlockMax columns; one CTA per
-// front).  Warp w holds the column group [4w, 4w+4) of the block, lane l the
+// Block LU in FP64 by a whole CTA (blocks of 33..BlockMax columns; one CTA
+// per front; FP32: k_block_lu_f32).  Warp w holds the column group [4w, 4w+4) of the block, lane l the
 // rows [RPT l, RPT l + RPT) (RPT = BlockMax / 32), in registers.  The block
 // is factored one column group at a time:
 //   A. the group's owner warp factors its four columns in order, on its own
@@ -658,6 +669,571 @@ __global__ void __launch_bounds__(LuThreads<T>::value, 1) k_block_lu(T* fac, int
     if (tid == 0 && szero != INT_MAX) {
         int p = 0;
         while (q0[p + 1] <= szero) ++p;
+        atomicMin(info, p0 + p + 1);   // first singular piece of the block
+    }
+}
+
+// ---------------------------------------------------------------------------
+// FP32 block LU by a whole CTA (blocks of 33..128 columns; one CTA per
+// front), in groups of at most 32 columns: consecutive whole pieces that
+// fit, or a slice of a wider piece.  The block is in shared memory.  Per
+// group [a, b):
+//   1. warps 0..3 factor the group's rows and columns in registers
+//      (lu_sweep): exactly ggetrf!'s pivots, a lane per row, eight columns
+//      per warp; no row ever moves, a lane records the position its row has
+//      reached;
+//   2. a thread per later row solves its L21 entries (trsm 'r','u','n','n')
+//      and a thread per later column its U12 entries (_luswap! as a gather
+//      of source rows, trsm 'l','l','t','u');
+//   3. the rest of the block takes the rank-w update.  The next group's
+//      diagonal block is updated first, by eight warps, so that warps 0..3
+//      factor it while the others do the rest and write out what is final
+//      (look-ahead).
+// What bounds it is the latency of step 1 (per column a reduction, a vote,
+// the shuffles of the winner's reciprocal and of the next column's entry, a
+// multiply-add), so everything else is kept off that chain: the reciprocal
+// of every candidate is formed beside the reduction, the warp that owns a
+// column only publishes its multipliers and goes on, and the warps of the
+// later columns follow two columns behind.  One block of 120 columns alone
+// on the GPU: 29 us when every pivot is on the diagonal, 37 us with searches
+// (60 us in the column-group form k_block_lu, whose owner warp also moved rows
+// and updated 128 of them per column).
+// ---------------------------------------------------------------------------
+constexpr int LU_THREADS = 512, LU_G = 32, LU_W = 8;   // group, columns per warp of a sweep
+constexpr int LU_LSW = LU_G + 4;   // entries per staged row of a group: 16-byte rows, 4 words apart in the bank cycle
+
+typedef unsigned long long f2;     // two floats, the first in the low half
+__device__ __forceinline__ f2 f2_pack(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float f2_lo(f2 v) { return __uint_as_float((unsigned)v); }
+__device__ __forceinline__ float f2_hi(f2 v) { return __uint_as_float((unsigned)(v >> 32)); }
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// A sweep's outputs in shared memory.
+struct LuSweep {
+    float* lu;    // L and U by position: entry (i, j) at lu + i * LU_LSW + j (up to 64 rows)
+    float* lt;    // the first w rows transposed: entry (i, j) at lt + j * LU_LSW + i
+    float* ex;    // exchange: multipliers of column k by row (ex + k * 64), or work space of the general form
+    float* rd;    // per column, the reciprocal of its pivot (1 for a zero pivot: no scaling)
+    int* piv;     // per column, row | position << 8 of the pivot (position before the interchange)
+    int* lsrc;    // original row now at each position
+    int* at;      // position of each original row
+    int* bad;     // set when the group has to be repeated by a more general form
+};
+
+// Called by warps q = 0 .. cdiv(w, 8) - 1; A is only read, so that a group can
+// be repeated.  RPL: rows per lane (at most 32 RPL rows).  cend: in lane k,
+// the end of the candidate positions of column k (its piece's end; k + 1 in
+// the symmetric form, where the diagonal row is the only candidate).
+//   SEARCH = false: the diagonal row is taken as every column's pivot and
+//     each candidate is checked against it beside the chain; *bad is set when
+//     one is larger.  Nothing of the chain waits for a search then: a column
+//     is two shuffles and a multiply-add.
+//   SEARCH = true: a reduction and a vote find the pivot.
+// Both set *bad for a column whose pivot is not unique, not finite, or not
+// normal (as its reciprocal).
+template <bool SEARCH, int RPL>
+__device__ __forceinline__ void lu_sweep(const float* A, int lda, int nrow, int w, int cend, const LuSweep& O, int q) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, nq = cdiv(w, LU_W);
+    f2 P[RPL][LU_W / 2];
+    int pos[RPL];
+    bool act[RPL], bad = false;
+#pragma unroll
+    for (int s = 0; s < RPL; ++s) {
+        const int r = lane + 32 * s;
+        pos[s] = r;
+        act[s] = r < nrow;
+#pragma unroll
+        for (int i = 0; i < LU_W / 2; ++i) {
+            const int j = q * LU_W + 2 * i;
+            P[s][i] = f2_pack(r < nrow && j < w ? A[j * lda + r] : 0.0f, r < nrow && j + 1 < w ? A[(j + 1) * lda + r] : 0.0f);
+        }
+    }
+    // rank-1 update of pairs i0 .. with the row in lane kl, slot ks
+    auto update = [&](int i0, int kl, int ks, const float (&l)[RPL]) {
+        f2 nl[RPL];
+#pragma unroll
+        for (int s = 0; s < RPL; ++s) nl[s] = f2_pack(-l[s], -l[s]);
+#pragma unroll
+        for (int i = 0; i < LU_W / 2; ++i)
+            if (i >= i0) {
+                const f2 v = RPL == 2 && ks ? P[RPL - 1][i] : P[0][i];
+                const f2 u = f2_pack(__shfl_sync(FULL, f2_lo(v), kl), __shfl_sync(FULL, f2_hi(v), kl));
+#pragma unroll
+                for (int s = 0; s < RPL; ++s)
+                    if (act[s]) P[s][i] = f2_fma(nl[s], u, P[s][i]);
+            }
+    };
+    // row r (lane kl, slot ks) goes to position k
+    auto place = [&](int k, int kl, int ks, int pp) {
+#pragma unroll
+        for (int s = 0; s < RPL; ++s) {
+            if (SEARCH && pos[s] == k) pos[s] = pp;
+            if (lane == kl && s == ks) {
+                pos[s] = k;
+                act[s] = false;
+            }
+        }
+    };
+#pragma unroll 1
+    for (int o = 0; o < q; ++o)   // follow the warps of the earlier columns, two columns at a time
+#pragma unroll
+        for (int t = 0; t < LU_W; t += 2) {
+            const int k = o * LU_W + t;
+            asm volatile("bar.sync %0, %1;" ::"r"(4 + t / 2), "r"(32 * (nq - o)) : "memory");
+            float l[2][RPL];
+            int pv[2] = {0, 0};
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+#pragma unroll
+                for (int s = 0; s < RPL; ++s) l[c][s] = O.ex[(k + c) * 64 + lane + 32 * s];
+                if (SEARCH) pv[c] = O.piv[k + c];
+            }
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const int kr = SEARCH ? pv[c] & 255 : k + c;
+                place(k + c, kr & 31, kr >> 5, pv[c] >> 8);
+                update(0, kr & 31, kr >> 5, l[c]);
+            }
+        }
+#pragma unroll
+    for (int t = 0; t < LU_W; ++t) {
+        const int k = q * LU_W + t;
+        if (k >= w) break;
+        float c[RPL], r[RPL], l[RPL];
+        const int ce = __shfl_sync(FULL, cend, k);
+#pragma unroll
+        for (int s = 0; s < RPL; ++s) {
+            c[s] = (t & 1) ? f2_hi(P[s][t / 2]) : f2_lo(P[s][t / 2]);
+            r[s] = rcp_approx(c[s]);
+        }
+        int kl = k, ks = 0, pp = k;
+        float inv;
+        if constexpr (SEARCH) {
+            unsigned key[RPL], best = 0u, m = 0u, dup = 0u;
+#pragma unroll
+            for (int s = 0; s < RPL; ++s) {
+                key[s] = act[s] && pos[s] < ce ? __float_as_uint(c[s]) & 0x7fffffffu : 0u;   // NaN above infinity: caught below
+                best = max(best, key[s]);
+            }
+            const unsigned mx = __reduce_max_sync(FULL, best);
+#pragma unroll
+            for (int s = 0; s < RPL; ++s) {
+                const unsigned b = __ballot_sync(FULL, key[s] == mx);
+                dup |= (b & (b - 1)) | (b ? m : 0u);
+                if (b) ks = s;
+                m |= b;
+            }
+            kl = 31 - __clz(m);   // the only lane, or the group is repeated
+            bad |= dup != 0u || mx - 0x00800000u > 0x7e000000u - 0x00800000u;
+            inv = __shfl_sync(FULL, RPL == 2 && ks ? r[RPL - 1] : r[0], kl);
+            pp = __shfl_sync(FULL, RPL == 2 && ks ? pos[RPL - 1] : pos[0], kl);
+        } else {
+            inv = __shfl_sync(FULL, r[0], k);
+            const unsigned d = __float_as_uint(__shfl_sync(FULL, c[0], k)) & 0x7fffffffu;
+            bad |= d - 0x00800000u > 0x7e000000u - 0x00800000u;
+#pragma unroll
+            for (int s = 0; s < RPL; ++s)   // a tie keeps the diagonal row, the first candidate; NaN counts as larger
+                bad |= act[s] && pos[s] < ce && (__float_as_uint(c[s]) & 0x7fffffffu) > d;
+        }
+        place(k, kl, ks, pp);
+#pragma unroll
+        for (int s = 0; s < RPL; ++s) {
+            l[s] = c[s] * inv;
+            O.ex[k * 64 + lane + 32 * s] = l[s];
+            if (lane == kl && s == ks) {
+                O.piv[k] = (kl + 32 * ks) | pp << 8;
+                O.rd[k] = r[s];
+            }
+        }
+        if ((t & 1) && q + 1 < nq) asm volatile("bar.arrive %0, %1;" ::"r"(4 + t / 2), "r"(32 * (nq - q)) : "memory");
+        if (!(t & 1)) {
+            const float v = f2_hi(RPL == 2 && ks ? P[RPL - 1][t / 2] : P[0][t / 2]);
+            const float u = __shfl_sync(FULL, v, kl);
+#pragma unroll
+            for (int s = 0; s < RPL; ++s)
+                if (act[s]) P[s][t / 2] = f2_pack(l[s], fmaf(-l[s], u, f2_hi(P[s][t / 2])));
+        } else {
+#pragma unroll
+            for (int s = 0; s < RPL; ++s)
+                if (act[s]) P[s][t / 2] = f2_pack(f2_lo(P[s][t / 2]), l[s]);
+        }
+        update(t / 2 + 1, kl, ks, l);
+    }
+    if (q == nq - 1)   // the last warp knows every row's final position
+#pragma unroll
+        for (int s = 0; s < RPL; ++s)
+            if (lane + 32 * s < nrow) {
+                O.at[lane + 32 * s] = pos[s];
+                O.lsrc[pos[s]] = lane + 32 * s;
+            }
+    if (bad) *O.bad = 1;
+    asm volatile("bar.sync 12, %0;" ::"r"(32 * nq) : "memory");
+#pragma unroll
+    for (int s = 0; s < RPL; ++s)
+        if (lane + 32 * s < nrow) {
+            const int i = O.at[lane + 32 * s];
+            ulonglong2* d = reinterpret_cast<ulonglong2*>(O.lu + i * LU_LSW + q * LU_W);
+            d[0] = make_ulonglong2(P[s][0], P[s][1]);
+            d[1] = make_ulonglong2(P[s][2], P[s][3]);
+            if (i < LU_G)
+#pragma unroll
+                for (int j = 0; j < LU_W; ++j)
+                    O.lt[(q * LU_W + j) * LU_LSW + i] = (j & 1) ? f2_hi(P[s][j / 2]) : f2_lo(P[s][j / 2]);
+        }
+}
+
+// General form, by one warp (up to 64 rows, at slots lane and lane + 32): the
+// same with ties (the first position wins), zero pivots (no scaling), NaN
+// (never wins, except on the diagonal) and reciprocals outside the normal
+// range.  The rows stay in O.ex, column k of row r at ex[k * 64 + r].
+// Returns the first step with a zero pivot, or LU_G.
+__device__ __noinline__ int lu_sweep_general(const float* A, int lda, int nrow, int w, int cend, const LuSweep& O, bool sym) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    int pos[2] = {lane, lane + 32}, zero = LU_G;
+    bool act[2] = {lane < nrow, lane + 32 < nrow};
+    for (int j = 0; j < w; ++j)
+        for (int s = 0; s < 2; ++s)
+            if (lane + 32 * s < nrow) O.ex[j * 64 + lane + 32 * s] = A[j * lda + lane + 32 * s];
+    __syncwarp();
+    for (int k = 0; k < w; ++k) {
+        const int ce = __shfl_sync(FULL, cend, k);
+        float c[2];
+        unsigned key[2];
+        for (int s = 0; s < 2; ++s) {
+            c[s] = act[s] ? O.ex[k * 64 + lane + 32 * s] : 0.0f;
+            key[s] = pivot_key32(c[s], act[s] && (sym ? pos[s] == k : pos[s] < ce), pos[s] == k);
+        }
+        const unsigned mx = __reduce_max_sync(FULL, max(key[0], key[1]));
+        unsigned p = 0xffffffffu;   // the first position holding it
+        for (int s = 0; s < 2; ++s)
+            if (key[s] == mx) p = min(p, (unsigned)pos[s]);
+        p = __reduce_min_sync(FULL, p);
+        const unsigned b0 = __ballot_sync(FULL, act[0] && pos[0] == (int)p), b1 = __ballot_sync(FULL, act[1] && pos[1] == (int)p);
+        const int kr = b0 ? __ffs(b0) - 1 : 31 + __ffs(b1);   // the pivot row
+        const float pv = O.ex[k * 64 + kr];
+        const float inv = pv != 0.0f ? lu_recip(pv) : 1.0f;
+        if (pv == 0.0f) zero = min(zero, k);
+        if (lane == 0) {
+            O.piv[k] = kr | (int)p << 8;
+            O.rd[k] = inv;
+        }
+        for (int s = 0; s < 2; ++s) {
+            if (pos[s] == k) pos[s] = (int)p;
+            if (lane + 32 * s == kr) {
+                pos[s] = k;
+                act[s] = false;
+            }
+            if (act[s]) {
+                const float l = c[s] * inv;
+                O.ex[k * 64 + lane + 32 * s] = l;
+                for (int j = k + 1; j < w; ++j) O.ex[j * 64 + lane + 32 * s] -= l * O.ex[j * 64 + kr];
+            }
+        }
+        __syncwarp();
+    }
+    for (int s = 0; s < 2; ++s)
+        if (lane + 32 * s < nrow) {
+            O.at[lane + 32 * s] = pos[s];
+            O.lsrc[pos[s]] = lane + 32 * s;
+            for (int j = 0; j < w; ++j) {
+                const float v = O.ex[j * 64 + lane + 32 * s];
+                O.lu[pos[s] * LU_LSW + j] = v;
+                if (pos[s] < LU_G) O.lt[j * LU_LSW + pos[s]] = v;
+            }
+        }
+    return zero;
+}
+
+struct LuSmem {   // offsets in floats
+    static constexpr int BM = 128, LD = BM + 1, SLB = BM + 4;   // a slab's last row is read up to 28 entries past its end
+    static constexpr int a = 0;                          // A(i, j) at a + j * LD + i
+    static constexpr int lu = (BM * LD + 3) / 4 * 4;     // LuSweep::lu
+    static constexpr int lt = lu + 2 * LU_G * LU_LSW;    // LuSweep::lt
+    static constexpr int ex = lt + LU_G * LU_LSW;        // LuSweep::ex
+    static constexpr int sl = ex + LU_G * 2 * LU_G;      // L21 by column: sl + k * SLB + row - b
+    static constexpr int su = sl + LU_G * SLB;           // U12 by row: su + k * SLB + column - b
+    static constexpr int bytes = (su + LU_G * SLB + 32) * 4;
+};
+
+// A(i, j) -= sum_k sl[k][i] su[k][j], one warp: rows r0 + lane + 32 m (m < M,
+// below r1) and columns [4 c, 4 c + 4) below q1 (relative to the slabs).
+// Lanes run along the rows, so that every access is free of bank conflicts.
+template <int M>
+__device__ __forceinline__ void lu_rank_tile(float* A, const float* sl, const float* su, int w, int r0, int r1, int c, int q1) {
+    constexpr int LD = LuSmem::LD, SLB = LuSmem::SLB;
+    const int lane = threadIdx.x & 31;
+    f2 acc[M][2];
+#pragma unroll
+    for (int m = 0; m < M; ++m) acc[m][0] = acc[m][1] = 0ull;
+    const float* x = sl + r0 + lane;
+    const float* y = su + 4 * c;
+#pragma unroll 4
+    for (int k = 0; k < w; ++k) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(y + k * SLB);   // past r1 (q1): read, never stored
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+            const float xm = x[k * SLB + 32 * m];
+            const f2 xx = f2_pack(xm, xm);
+            acc[m][0] = f2_fma(xx, v.x, acc[m][0]);
+            acc[m][1] = f2_fma(xx, v.y, acc[m][1]);
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+        const int i = r0 + lane + 32 * m;
+        const float d[4] = {f2_lo(acc[m][0]), f2_hi(acc[m][0]), f2_lo(acc[m][1]), f2_hi(acc[m][1])};
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (i < r1 && 4 * c + j < q1) A[(4 * c + j) * LD + i] -= d[j];
+    }
+}
+// Rows [r0, r1) (at most 128), one quad of columns.
+__device__ __forceinline__ void lu_rank_quad(float* A, const float* sl, const float* su, int w, int r0, int r1, int c, int q1) {
+    const int m = cdiv(r1 - r0, 32);
+    if (m == 1) lu_rank_tile<1>(A, sl, su, w, r0, r1, c, q1);
+    else if (m == 2) lu_rank_tile<2>(A, sl, su, w, r0, r1, c, q1);
+    else if (m >= 3) {
+        lu_rank_tile<3>(A, sl, su, w, r0, r1, c, q1);
+        if (m > 3) lu_rank_tile<1>(A, sl, su, w, r0 + 96, r1, c, q1);
+    }
+}
+
+__global__ void __launch_bounds__(LU_THREADS, 1) k_block_lu_f32(float* fac, int* ipiv, int* info, int* bmap, Sched S,
+                                                                Launch L, int step) {
+    using SM = LuSmem;
+    constexpr int BM = SM::BM, LD = SM::LD, SLB = SM::SLB, NW = LU_THREADS / 32;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float* sm = reinterpret_cast<float*>(smem_raw);
+    float *A = sm + SM::a, *lu = sm + SM::lu, *sl = sm + SM::sl, *su = sm + SM::su;
+    __shared__ int cpa[BM], cpb[BM];          // piece of each column
+    __shared__ int gs[BM + 1], ge[BM];        // groups: first column, end of the rows that take part
+    __shared__ __align__(16) float srd[LU_G];   // reciprocals of the group's pivots
+    __shared__ __align__(16) int lsrc[2 * LU_G];
+    __shared__ int spv[LU_G], sat[2 * LU_G], sbad;
+    __shared__ int spiv[BM], gmap[BM];        // gmap: row sources of the block's interchanges
+    __shared__ int szero, ngrp;
+    int fid, tile;
+    locate(L, blockIdx.x, fid, tile);
+    const DFront F = S.fronts[fid];
+    const int blk = F.block0 + step;
+    const int c0 = S.blk_c0[blk], c1 = S.blk_c1[blk], bw = c1 - c0;
+    const int p0 = S.blk_p0[blk], np = S.blk_np[blk];
+    const int tid = threadIdx.x, wp = tid >> 5, lane = tid & 31;
+    const bool sym = S.sym != 0;
+    float* blkp = fac + F.loff + (ll)c0 * F.ld + c0;   // block (i, j) at blkp[j * ld + i]
+    {
+        float v[BM / NW][4];
+#pragma unroll
+        for (int q = 0; q < BM / NW; ++q)
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+                const int C = wp + q * NW, R = lane + 32 * s;
+                v[q][s] = (C < bw && R < bw && (!sym || R >= C)) ? blkp[(ll)C * F.ld + R] : 0.0f;
+            }
+        for (int pc = tid; pc < np; pc += LU_THREADS) {
+            const int a = S.xsuper[p0 + pc] - F.f - c0, b = S.xsuper[p0 + pc + 1] - F.f - c0;
+            for (int k = a; k < b; ++k) {
+                cpa[k] = a;
+                cpb[k] = b;
+            }
+        }
+        if (tid < BM) gmap[tid] = tid;
+        if (tid == 0) {
+            szero = INT_MAX;
+            sbad = 0;
+        }
+#pragma unroll
+        for (int q = 0; q < BM / NW; ++q)
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+                const int C = wp + q * NW, R = lane + 32 * s;
+                if (C < bw && R < bw && (!sym || R >= C)) {
+                    A[C * LD + R] = v[q][s];
+                    if (sym) A[R * LD + C] = v[q][s];   // symmetric form: the upper triangle mirrors the lower one
+                }
+            }
+    }
+    __syncthreads();
+    if (tid == 0) {   // groups: whole pieces up to LU_G columns, or LU_G-column slices of a wider piece
+        int n = 0, a = 0;
+        while (a < bw) {
+            int b = a, e;
+            while (b < bw && cpb[b] - a <= LU_G) b = cpb[b];
+            e = b;
+            if (b == a) {
+                e = cpb[a];
+                b = a + LU_G;
+            }
+            gs[n] = a;
+            ge[n++] = e;
+            a = b;
+        }
+        gs[n] = bw;
+        ngrp = n;
+    }
+    const LuSweep O{lu, sm + SM::lt, sm + SM::ex, srd, spv, lsrc, sat, &sbad};
+    // part 1 of group [a, b), rows to e (warps 0..3)
+    auto sweep = [&](int a, int b, int e, bool search) {
+        const int w = b - a, nrow = e - a;
+        if (wp >= cdiv(w, LU_W)) return;
+        const int cend = lane < w ? (sym ? lane + 1 : cpb[a + lane] - a) : 0;
+        const float* D = A + a * LD + a;
+        if (nrow <= 32) {
+            if (search) lu_sweep<true, 1>(D, LD, nrow, w, cend, O, wp);
+            else lu_sweep<false, 1>(D, LD, nrow, w, cend, O, wp);
+        } else {
+            lu_sweep<true, 2>(D, LD, nrow, w, cend, O, wp);
+        }
+    };
+    __syncthreads();
+    const int ng = ngrp;
+    bool search = false;   // once a group needed an interchange, look for the pivots of the next ones
+    if (wp < 4) sweep(gs[0], gs[1], ge[0], search);
+    __syncthreads();
+    int done = 0;   // columns [0, done) and their rows are written out
+#pragma unroll 1
+    for (int g = 0; g < ng; ++g) {
+        const int a = gs[g], b = gs[g + 1], w = b - a, e = ge[g], nrow = e - a;
+        const bool moved = e > b || cpa[a] < a;
+        if (sbad) {   // the diagonal was not every column's pivot: search
+            const bool again = !search && !sym && nrow <= 32;
+            __syncthreads();
+            if (again) {
+                if (tid == 0) sbad = 0;
+                search = true;
+                __syncthreads();
+                if (wp < 4) sweep(a, b, e, true);
+                __syncthreads();
+            }
+            if (!again || sbad) {   // an exceptional pivot
+                if (wp == 0) {
+                    const int z = lu_sweep_general(A + a * LD + a, LD, nrow, w, lane < w ? cpb[a + lane] - a : 0, O, sym);
+                    if (lane == 0 && z < LU_G) szero = min(szero, a + z);
+                }
+                __syncthreads();
+                if (tid == 0) sbad = 0;
+            }
+        }
+        if (moved) {
+            // a slice of a wide piece: its interchanges move whole rows, over
+            // the columns right of the group and those of the piece left of it
+            const int left = a - cpa[a], nc = left + (bw - b);
+            for (int c = wp; c < nc; c += NW) {
+                float* col = A + (c < left ? cpa[a] + c : b + c - left) * LD + a;
+                const int lim = c < left ? cpb[a] - a : nrow;   // left: the rows of this piece only
+                const float v0 = lane < lim ? col[lsrc[lane]] : 0.0f, v1 = lane + 32 < lim ? col[lsrc[lane + 32]] : 0.0f;
+                __syncwarp();
+                if (lane < lim) col[lane] = v0;
+                if (lane + 32 < lim) col[lane + 32] = v1;
+            }
+            __syncthreads();
+        }
+        // part 2: warps 0, 2, 4 (.. by 32) the rows below, warps 1, 3, 5 the columns right
+        const int nr = bw - b;
+        if (wp < 2 * cdiv(nr, 32)) {
+            const int x = (wp >> 1) * 32 + lane;
+            // Both are x := x T^-1 with the rows of T in order: T = U for a
+            // row of L21 (entries scaled by 1 / U(k, k)), T = L^T for a
+            // column of U12 (unit diagonal), so they share their code.
+            const bool isU = wp & 1;
+            float* line = isU ? A + (b + x) * LD + a : A + a * LD + b + x;   // entry k at line[k * ls]
+            const int ls = isU ? 1 : LD;
+            float* out = (isU ? su : sl) + x;
+            const float* T = isU ? O.lt : lu;
+            if (x < nr && !isU && b + x < e) {   // a row of the sliced piece: its multipliers are known
+                for (int k = 0; k < w; ++k) {
+                    const float v = lu[(b + x - a) * LU_LSW + k];
+                    line[k * ls] = v;
+                    out[k * SLB] = v;
+                }
+            } else if (x < nr) {
+                const bool gather = isU && !moved;   // the interchanges of whole pieces, as a gather
+                f2 y[LU_G / 2];
+#pragma unroll
+                for (int k = 0; k < LU_G; k += 4) {
+                    const int4 src = gather ? *reinterpret_cast<const int4*>(lsrc + k) : make_int4(k, k + 1, k + 2, k + 3);
+                    y[k / 2] = f2_pack(k < w ? line[src.x * ls] : 0.0f, k + 1 < w ? line[src.y * ls] : 0.0f);
+                    y[k / 2 + 1] = f2_pack(k + 2 < w ? line[src.z * ls] : 0.0f, k + 3 < w ? line[src.w * ls] : 0.0f);
+                }
+#pragma unroll
+                for (int k = 0; k < LU_G; ++k) {   // past w: zeros, times whatever is there, never stored
+                    const float v = (k & 1 ? f2_hi(y[k / 2]) : f2_lo(y[k / 2])) * (isU ? 1.0f : srd[k]);
+                    const f2 nv = f2_pack(-v, -v);
+                    const ulonglong2* tr = reinterpret_cast<const ulonglong2*>(T + k * LU_LSW);
+                    if (!(k & 1)) y[k / 2] = f2_pack(v, f2_hi(y[k / 2]) - v * T[k * LU_LSW + k + 1]);
+                    else y[k / 2] = f2_pack(f2_lo(y[k / 2]), v);
+#pragma unroll
+                    for (int q = (k / 2 + 1) / 2; q < LU_G / 4; ++q) {
+                        const ulonglong2 u = tr[q];
+                        if (2 * q > k / 2) y[2 * q] = f2_fma(nv, u.x, y[2 * q]);
+                        y[2 * q + 1] = f2_fma(nv, u.y, y[2 * q + 1]);
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < LU_G; ++k)
+                    if (k < w) {
+                        const float v = k & 1 ? f2_hi(y[k / 2]) : f2_lo(y[k / 2]);
+                        line[k * ls] = v;
+                        out[k * SLB] = v;
+                    }
+            }
+        } else if (wp >= 8) {
+            // the group's own part of the factor (the multipliers left of a
+            // row's piece are never interchanged), pivots and row sources
+            for (int j = wp - 8; j < w; j += NW - 8)
+                if (lane < w) {
+                    const int i = lane;
+                    const int s = i <= j || a + j >= cpa[a + i] ? i : sat[i];
+                    A[(a + j) * LD + a + i] = lu[s * LU_LSW + j];
+                }
+            if (wp == 13 && lane < w) spiv[a + lane] = a + (spv[lane] >> 8) - cpa[a + lane];
+            if (wp >= 14) {   // row sources: composed over the slices of a wide piece
+                const int i = tid - (LU_THREADS - 64);
+                const int v = i < nrow ? gmap[a + lsrc[i]] : 0;
+                asm volatile("bar.sync 3, 64;" ::: "memory");
+                if (i < nrow) gmap[a + i] = v;
+            }
+        }
+        __syncthreads();
+        if (g + 1 == ng) break;
+        // part 3, the next group's diagonal block first
+        // (its rows rounded up to 32, its columns to 4)
+        const int b2 = gs[g + 2], e2 = ge[g + 1], rn = min(cdiv(e2 - b, 32) * 32, nr), cn = cdiv(b2 - b, 4);
+        float* D = A + b * LD + b;
+        if (wp < 8) {
+            for (int c = wp; c < cn; c += 8) lu_rank_quad(D, sl, su, w, 0, rn, c, nr);
+            asm volatile("bar.sync 1, 256;" ::: "memory");
+        }
+        if (wp < 4) {
+            sweep(b, b2, e2, search);
+        } else {
+            for (int c = wp - 4; c < cdiv(nr, 4); c += NW - 4) lu_rank_quad(D, sl, su, w, c < cn ? rn : 0, nr, c, nr);
+            if (e == b) {   // whole pieces: their columns, and their rows right of them, are final
+                for (int C = done + wp - 4; C < bw; C += NW - 4)
+                    for (int R = done + lane; R < (C < b ? bw : b); R += 32) blkp[(ll)C * F.ld + R] = A[C * LD + R];
+            }
+        }
+        if (e == b) done = b;
+        __syncthreads();
+    }
+    for (int C = done + wp; C < bw; C += NW)
+        for (int R = done + lane; R < bw; R += 32) blkp[(ll)C * F.ld + R] = A[C * LD + R];
+    if (tid < bw) {
+        ipiv[F.f + c0 + tid] = spiv[tid];
+        bmap[F.f + c0 + tid] = gmap[tid] | (cpa[tid] << 8);
+    }
+    if (tid == 0 && szero != INT_MAX) {
+        int p = 0;
+        while (S.xsuper[p0 + p + 1] - F.f - c0 <= szero) ++p;
         atomicMin(info, p0 + p + 1);   // first singular piece of the block
     }
 }
