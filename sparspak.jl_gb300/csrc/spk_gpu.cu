@@ -1114,6 +1114,8 @@ static int ensure_plan(spk_handle* h) {
                                (int)spk::LeafSmem<T, 16>::bytes));
     CU(h, cudaFuncSetAttribute(spk::k_leaf_factor<T, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)spk::LeafSmem<T, 32>::bytes));
+    CU(h, cudaFuncSetAttribute(spk::k_leaf_factor_set<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)spk::LeafSmem<T, 32>::bytes));
     CU(h, cudaFuncSetAttribute(spk::k_leaf_queue<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)spk::LeafSmem<T, 32>::bytes));
     {   // the queue's persistent grid: every CTA the SMs hold at once
@@ -1262,6 +1264,27 @@ static cudaError_t launch_leaf(int c, const spk::Launch& la, T* fac, int* ipiv, 
     return cudaGetLastError();
 }
 
+// A level's lists of small fronts go out as one launch (k_leaf_factor_set,
+// k_solve_leaf_set) while they hold at most this many fronts per SM, i.e. one
+// wave or so of warps: the launches would run one after the other, mostly
+// idle.  Wider lists keep a launch per width class, whose registers and shared
+// memory are sized to the class.
+constexpr int LEAF_MERGE = 16;
+
+static spk::LeafSet leaf_set(const Plan& PL, const LaunchRec* const (&lists)[spk::LEAF_LISTS], int& total, int& used) {
+    spk::LeafSet s{};
+    total = used = 0;
+    for (int i = 0; i < spk::LEAF_LISTS; ++i) {
+        if (lists[i] && lists[i]->tiles > 0) {
+            s.ids[i] = PL.d_sched_ids + lists[i]->off;
+            total += lists[i]->count;
+            ++used;
+        }
+        s.end[i] = total;
+    }
+    return s;
+}
+
 template <typename T>
 static int solve_fwd_levels(spk_handle* h, int nrhs, size_t l0, size_t l1, cudaStream_t st);
 
@@ -1353,14 +1376,35 @@ static int factor_launches(spk_handle* h, int fs_nrhs = 0) {
             CU(h, cudaEventRecord(h->evI, h->side2));
             pending_inv = true;
         }
-        for (int c = 0; c < spk::LF_CLASSES; ++c) {
-            if (P.leaf_factor[c].tiles > 0) {
-                LaunchScope ls(h, SPK_K_GETRF, P.leaf_factor[c].flops, P.leaf_factor[c].words * sizeof(T));
-                CU(h, launch_leaf<T>(c, launch_of(PL, P.leaf_factor[c]), fac, h->d_ipiv, h->d_info, S, h->stream));
+        {
+            const LaunchRec* lists[spk::LEAF_LISTS];
+            for (int c = 0; c < spk::LF_CLASSES; ++c) {
+                lists[c] = &P.leaf_factor[c];
+                lists[spk::LF_CLASSES + c] = queue ? nullptr : &P.leaf_q[c];
             }
-            if (!queue && P.leaf_q[c].tiles > 0) {
-                LaunchScope ls(h, SPK_K_GETRF, P.leaf_q[c].flops, P.leaf_q[c].words * sizeof(T));
-                CU(h, launch_leaf<T>(c, launch_of(PL, P.leaf_q[c]), fac, h->d_ipiv, h->d_info, S, h->stream));
+            int total = 0, used = 0;
+            const spk::LeafSet set = leaf_set(PL, lists, total, used);
+            if (used > 1 && total <= LEAF_MERGE * h->nsm) {
+                double fl = 0.0, wl = 0.0;
+                size_t wb = 0;
+                for (int i = 0; i < spk::LEAF_LISTS; ++i)
+                    if (lists[i] && lists[i]->tiles > 0) {
+                        fl += lists[i]->flops;
+                        wl += lists[i]->words;
+                        const size_t need[] = {spk::LeafSmem<T, 4>::warp_bytes, spk::LeafSmem<T, 8>::warp_bytes,
+                                               spk::LeafSmem<T, 16>::warp_bytes, spk::LeafSmem<T, 32>::warp_bytes};
+                        wb = std::max(wb, need[i % spk::LF_CLASSES]);
+                    }
+                LaunchScope ls(h, SPK_K_GETRF, fl, wl * sizeof(T));
+                spk::k_leaf_factor_set<T><<<spk::cdiv(total, spk::LF_WARPS), 32 * spk::LF_WARPS, spk::LF_WARPS * wb,
+                                            h->stream>>>(fac, h->d_ipiv, h->d_info, S, set, (unsigned)wb);
+            } else {
+                for (int i = 0; i < spk::LEAF_LISTS; ++i)
+                    if (lists[i] && lists[i]->tiles > 0) {
+                        LaunchScope ls(h, SPK_K_GETRF, lists[i]->flops, lists[i]->words * sizeof(T));
+                        CU(h, launch_leaf<T>(i % spk::LF_CLASSES, launch_of(PL, *lists[i]), fac, h->d_ipiv, h->d_info, S,
+                                             h->stream));
+                    }
             }
         }
         for (size_t t = 0; t < P.blu.size(); ++t) {
@@ -1534,6 +1578,41 @@ static cudaError_t launch_solve_leaf(int c, int count, cudaStream_t st, const T*
     }
 }
 
+// A level's small fronts, forward or backward: one launch for all width
+// classes, or one each (LEAF_MERGE).
+template <typename T, bool FWD>
+static int solve_leaf_level(spk_handle* h, const Plan& PL, const LevelPlan& P, int kind, cudaStream_t st, T* in, T* out,
+                            const T* xs, int nrhs) {
+    const T* fac = storage<T>(h).d;
+    const T* inv = storage<T>(h).inv2;
+    const int n = (int)h->n;
+    const LaunchRec* lists[spk::LEAF_LISTS] = {};
+    for (int c = 0; c < spk::LF_CLASSES; ++c) lists[c] = &P.front_leaf[c];
+    int total = 0, used = 0;
+    const spk::LeafSet set = leaf_set(PL, lists, total, used);
+    if (used > 1 && total <= LEAF_MERGE * h->nsm) {
+        double fl = 0.0, wl = 0.0;
+        for (const LaunchRec& R : P.front_leaf) {
+            fl += R.tiles > 0 ? R.flops : 0.0;
+            wl += R.tiles > 0 ? R.words : 0.0;
+        }
+        LaunchScope ls(h, kind, fl * nrhs, wl * sizeof(T));
+        const int grid = spk::cdiv(total, 8);
+        CU(h, nrhs == 1 ? launch_chained(spk::k_solve_leaf_set<T, FWD, 1>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs,
+                                         PL.sched, set)
+                        : launch_chained(spk::k_solve_leaf_set<T, FWD, 4>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs,
+                                         PL.sched, set));
+        return SPK_OK;
+    }
+    for (int c = 0; c < spk::LF_CLASSES; ++c) {
+        const LaunchRec& R = P.front_leaf[c];
+        if (R.tiles == 0) continue;
+        LaunchScope ls(h, kind, R.flops * nrhs, R.words * sizeof(T));
+        CU(h, (launch_solve_leaf<T, FWD>(c, R.count, st, fac, inv, in, out, xs, n, nrhs, PL.sched, launch_of(PL, R))));
+    }
+    return SPK_OK;
+}
+
 // The forward substitution over levels [l0, l1) on the permuted work
 // vectors (wb, consumed, -> wy), launched on `st`.
 template <typename T>
@@ -1548,13 +1627,7 @@ static int solve_fwd_levels(spk_handle* h, int nrhs, size_t l0, size_t l1, cudaS
     constexpr size_t fc_smem = spk::FcSmem<T>::bytes;
     for (size_t l = l0; l < l1; ++l) {
         const LevelPlan& P = PL.levels[l];
-        for (int c = 0; c < spk::LF_CLASSES; ++c) {
-            const LaunchRec& R = P.front_leaf[c];
-            if (R.tiles == 0) continue;
-            LaunchScope ls(h, SPK_K_FWD, R.flops * nrhs, R.words * sizeof(T));
-            CU(h, (launch_solve_leaf<T, true>(c, R.count, st, fac, inv, b, y, (const T*)nullptr, n, nrhs, S,
-                                              launch_of(PL, R))));
-        }
+        if (int rc = solve_leaf_level<T, true>(h, PL, P, SPK_K_FWD, st, b, y, (const T*)nullptr, nrhs)) return rc;
         if (P.front_big.tiles > 0) {
             LaunchScope ls(h, SPK_K_FWD, P.front_big.flops * nrhs, P.front_big.words * sizeof(T));
             if (h->fc16)
@@ -1615,13 +1688,7 @@ static int solve_bwd_levels(spk_handle* h, int nrhs, cudaStream_t st) {
     constexpr size_t fc_smem = spk::FcSmem<T>::bytes;
     for (size_t l = PL.levels.size(); l-- > 0;) {
         const LevelPlan& P = PL.levels[l];
-        for (int c = 0; c < spk::LF_CLASSES; ++c) {
-            const LaunchRec& R = P.front_leaf[c];
-            if (R.tiles == 0) continue;
-            LaunchScope ls(h, SPK_K_BWD, R.flops * nrhs, R.words * sizeof(T));
-            CU(h, (launch_solve_leaf<T, false>(c, R.count, st, fac, inv, y, x, (const T*)x, n, nrhs, S,
-                                               launch_of(PL, R))));
-        }
+        if (int rc = solve_leaf_level<T, false>(h, PL, P, SPK_K_BWD, st, y, x, (const T*)x, nrhs)) return rc;
         if (P.bwdu_small.tiles > 0) {
             LaunchScope ls(h, SPK_K_BWD, P.bwdu_small.flops * nrhs, P.bwdu_small.words * sizeof(T));
             CU(h, launch_chained(spk::k_bwd_u12<T>, P.bwdu_small.tiles, 256, 0, st, fac, y, x, n, nrhs, S,

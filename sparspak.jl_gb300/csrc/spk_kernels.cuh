@@ -155,6 +155,14 @@ __device__ __forceinline__ int warp_first_max(unsigned long long key) {
     return __ffs(ballot) - 1;
 }
 
+// 32-bit pivot key of a float (same order as pivot_key).
+__device__ __forceinline__ unsigned pivot_key32(float x, bool cand, bool diag) {
+    if (!cand) return 0u;
+    const unsigned b = __float_as_uint(x) & 0x7fffffffu;
+    if (b > 0x7f800000u) return diag ? 0xffffffffu : 1u;
+    return b + 2u;
+}
+
 // Correctly rounded reciprocal (the value of T(1) / x).
 __device__ __forceinline__ float rcp_rn(float x) { return __frcp_rn(x); }
 __device__ __forceinline__ double rcp_rn(double x) { return __drcp_rn(x); }
@@ -222,106 +230,134 @@ __device__ bool warp_lu_sweep(T (&r)[W], int nrows, int ncols, const int* q0, in
     const int lane = threadIdx.x & 31;
     bool sing = false;
     int pc = 0;
-    if constexpr (W <= 8) {
-        // Narrow blocks: unrolled over the column index, so that r[k] and the
-        // columns after k are compile-time registers.
-#pragma unroll
-        for (int k = 0; k < W; ++k) {
-            if (k < ncols) {
-                while (q0[pc + 1] <= k) ++pc;
-                const int a = q0[pc], b = q0[pc + 1];
-                const int kp = warp_pivot_lane(r[k], sym ? lane == k : (lane >= k && lane < b), lane == k);
-                if (lane == 0) piv[k] = kp - a;
-                const T pv = __shfl_sync(FULL, r[k], kp);
-                if (pv != T(0)) {
-                    if (kp != k) {
-#pragma unroll
-                        for (int j = 0; j < W; ++j) {
-                            const T vk = __shfl_sync(FULL, r[j], k), vp = __shfl_sync(FULL, r[j], kp);
-                            if (j >= a) {
-                                if (lane == k) r[j] = vp;
-                                else if (lane == kp) r[j] = vk;
-                            }
-                        }
-                    }
-                    const T inv = lu_recip(pv);
-                    if (lane > k && lane < nrows) r[k] *= inv;
-                } else {
-                    sing = true;
-                }
-                const T lk = r[k];
-                const bool upd = lane > k && lane < nrows;
-#pragma unroll
-                for (int j = k + 1; j < W; ++j) {
-                    const T u = __shfl_sync(FULL, r[j], k);
-                    if (upd) r[j] -= lk * u;
-                }
-            }
-        }
-    } else {
-        // Wider blocks: a rolled loop (the unrolled form's code outgrows the
-        // instruction cache), r[k] picked by a tree of selects.
+    // a rolled loop (the unrolled form's code outgrows the instruction cache),
+    // r[k] picked by a tree of selects
 #pragma unroll 1
-        for (int k = 0; k < ncols; ++k) {
-            while (q0[pc + 1] <= k) ++pc;
-            const int a = q0[pc], b = q0[pc + 1];
-            const T rk0 = pickw<W>(r, k);
-            const int kp = warp_pivot_lane(rk0, sym ? lane == k : (lane >= k && lane < b), lane == k);
-            if (lane == 0) piv[k] = kp - a;
-            const T pv = __shfl_sync(FULL, rk0, kp);
-            if (pv != T(0)) {
-                if (kp != k) {
+    for (int k = 0; k < ncols; ++k) {
+        while (q0[pc + 1] <= k) ++pc;
+        const int a = q0[pc], b = q0[pc + 1];
+        const T rk0 = pickw<W>(r, k);
+        const int kp = warp_pivot_lane(rk0, sym ? lane == k : (lane >= k && lane < b), lane == k);
+        if (lane == 0) piv[k] = kp - a;
+        const T pv = __shfl_sync(FULL, rk0, kp);
+        if (pv != T(0)) {
+            if (kp != k) {
 #pragma unroll
-                    for (int j = 0; j < W; ++j) {
-                        const T vk = __shfl_sync(FULL, r[j], k), vp = __shfl_sync(FULL, r[j], kp);
-                        if (j >= a) {
-                            if (lane == k) r[j] = vp;
-                            else if (lane == kp) r[j] = vk;
-                        }
+                for (int j = 0; j < W; ++j) {
+                    const T vk = __shfl_sync(FULL, r[j], k), vp = __shfl_sync(FULL, r[j], kp);
+                    if (j >= a) {
+                        if (lane == k) r[j] = vp;
+                        else if (lane == kp) r[j] = vk;
                     }
                 }
-                const T inv = lu_recip(pv);
-                if (lane > k && lane < nrows) {
-#pragma unroll
-                    for (int j = 0; j < W; ++j)
-                        if (j == k) r[j] *= inv;
-                }
-            } else {
-                sing = true;
             }
-            const T lk = pickw<W>(r, k);
-            const bool upd = lane > k && lane < nrows;
+            const T inv = lu_recip(pv);
+            if (lane > k && lane < nrows) {
 #pragma unroll
-            for (int j = 0; j < W; ++j) {
-                const T u = __shfl_sync(FULL, r[j], k);
-                if (upd && j > k) r[j] -= lk * u;
+                for (int j = 0; j < W; ++j)
+                    if (j == k) r[j] *= inv;
             }
+        } else {
+            sing = true;
+        }
+        const T lk = pickw<W>(r, k);
+        const bool upd = lane > k && lane < nrows;
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+            const T u = __shfl_sync(FULL, r[j], k);
+            if (upd && j > k) r[j] -= lk * u;
         }
     }
     return sing;
 }
 
-// A whole block of at most 32 columns factored by one warp in registers
-// (lane i holds row i) as one right-looking sweep over its columns.  For
-// column k in piece [a, b): the pivot is the first strict maximum among rows
-// [k, b) (ggetrf!), the interchange moves whole rows over columns [a, bw)
-// (the piece's own columns, then _luswap! of its U rows), column k is scaled
+// A whole block of at most W <= 32 columns factored by one warp in registers
+// (a lane per row) as one right-looking sweep over its columns.  For column
+// k in piece [a, b): the pivot is the first strict maximum among rows [k, b)
+// (ggetrf!), the interchange acts on whole rows over columns [a, bw) (the
+// piece's own columns, then _luswap! of its U rows), column k is scaled
 // below the diagonal (ggetrf! scaling for rows in the piece, the L-panel
 // trsm 'r','u','n','n' for rows below it) and the rank-1 update covers rows
 // and columns after k (ggetrf!, the U-panel trsm 'r','l','t','u' and the
 // block-local update).  Columns left of the piece are never interchanged.
-template <typename T, int W = 32>
-__device__ bool warp_block_lu32(T* A, int lda, int bw, const int* q0, int np, int* piv, bool sym) {
+// No row moves during the sweep: a lane keeps the position its row has
+// reached, and the block is put in order when it is written back: entry j
+// of lane's row belongs at row (j >= p0 ? pos : lane).  Unrolled, so that
+// only the columns after k are touched (in FP64 a multiply-add takes a warp
+// 64 cycles).  Lanes bw .. nrow - 1 may hold rows below the block: the sweep
+// turns them into their L21 rows.  piv: local pivot rows; gm[i]: the row now
+// at position i; pa[i]: the first row of the piece of position i.
+template <typename T, int W>
+__device__ __forceinline__ bool warp_block_lu(T (&r)[W], int bw, int nrow, const int* q0, int* piv, int* gm, int* pa, bool sym,
+                                              int& pos, int& p0) {
+    const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    (void)np;
-    T r[W];
-#pragma unroll
-    for (int j = 0; j < W; ++j) r[j] = (lane < bw && j < bw) ? A[j * lda + lane] : T(0);
-    const bool sing = warp_lu_sweep<T, W>(r, bw, bw, q0, piv, sym);
+    p0 = 0;
+    int p1 = 0;   // the piece of row (and column) `lane`
     if (lane < bw) {
+        int pc = 0;
+        while (q0[pc + 1] <= lane) ++pc;
+        p0 = q0[pc];
+        p1 = q0[pc + 1];
+    }
+    pos = lane;
+    bool act = lane < nrow, sing = false;
 #pragma unroll
-        for (int j = 0; j < W; ++j)
-            if (j < bw) A[j * lda + lane] = r[j];
+    for (int k = 0; k < W; ++k)
+        if (k < bw) {
+            const T c = r[k];
+            const int ce = __shfl_sync(FULL, p1, k);
+            const bool diag = pos == k, cand = act && (sym ? diag : pos < ce);
+            T rc;   // every candidate's reciprocal, beside the search
+            if constexpr (sizeof(T) == 4) rc = rcp_approx(c);
+            else rc = lu_recip(cand ? c : T(1));
+            unsigned m;
+            if constexpr (sizeof(T) == 4) {
+                const unsigned key = pivot_key32(c, cand, diag);
+                m = __ballot_sync(FULL, key == __reduce_max_sync(FULL, key));
+            } else {
+                const unsigned long long key = pivot_key(c, cand, diag);
+                const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
+                const unsigned mh = __reduce_max_sync(FULL, hi);
+                m = __ballot_sync(FULL, hi == mh);
+                if (m & (m - 1)) {
+                    const unsigned ml = __reduce_max_sync(FULL, hi == mh ? lo : 0u);
+                    m = __ballot_sync(FULL, hi == mh && lo == ml);
+                }
+            }
+            if (m & (m - 1)) {   // equal values: the first position
+                const bool tied = (m >> lane) & 1u;
+                const unsigned p = __reduce_min_sync(FULL, tied ? (unsigned)pos : 0xffffffffu);
+                m = __ballot_sync(FULL, tied && (unsigned)pos == p);
+            }
+            const int kl = 31 - __clz(m);
+            const T pv = __shfl_sync(FULL, c, kl);
+            T inv = __shfl_sync(FULL, rc, kl);
+            const int pp = __shfl_sync(FULL, pos, kl);
+            if constexpr (sizeof(T) == 4) {
+                if (!(tabs(pv) >= 1.1754944e-38f && tabs(pv) <= 8.5070592e37f)) inv = lu_recip(pv);
+            }
+            if (pv == T(0)) {   // no scaling
+                inv = T(1);
+                sing = true;
+            }
+            if (pos == k) pos = pp;
+            if (lane == kl) {
+                pos = k;
+                act = false;
+                piv[k] = pp - p0;
+            }
+            const T l = c * inv;
+            if (act) r[k] = l;
+#pragma unroll
+            for (int j = k + 1; j < W; ++j) {
+                const T u = __shfl_sync(FULL, r[j], kl);
+                if (act) r[j] -= l * u;
+            }
+        }
+    if (lane < bw) {
+        gm[pos] = lane;
+        pa[lane] = p0;
     }
     __syncwarp();
     return sing;
@@ -331,34 +367,42 @@ __device__ bool warp_block_lu32(T* A, int lda, int bw, const int* q0, int np, in
 // launch holds one block per front).  Same outputs as k_block_lu.
 template <typename T>
 __global__ void __launch_bounds__(128) k_block_lu_small(T* fac, int* ipiv, int* info, Sched S, Launch L, int step) {
-    __shared__ T sA[4][32 * 33];
     __shared__ int sq[4][33];
-    __shared__ int spiv[4][32];
+    __shared__ int spiv[4][32], sgm[4][32], spa[4][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int idx = blockIdx.x * 4 + warp;
     if (idx >= L.count) return;
     const DFront F = S.fronts[L.front_ids[idx]];
     const int blk = F.block0 + step;
-    const int c0 = S.blk_c0[blk], c1 = S.blk_c1[blk], bw = c1 - c0, lda = 33;
+    const int c0 = S.blk_c0[blk], c1 = S.blk_c1[blk], bw = c1 - c0;
     const int p0 = S.blk_p0[blk], np = S.blk_np[blk];
-    T* A = sA[warp];
     int* q0 = sq[warp];
     int* piv = spiv[warp];
     for (int k = lane; k <= np; k += 32) q0[k] = S.xsuper[p0 + k] - F.f - c0;
-    for (int j = 0; j < bw; ++j)   // symmetric form: the upper triangle mirrors the lower one
-        if (lane < bw)
-            A[j * lda + lane] = (S.sym && lane < j) ? fac[F.loff + (ll)(c0 + lane) * F.ld + c0 + j]
-                                                    : fac[F.loff + (ll)(c0 + j) * F.ld + c0 + lane];
+    T* blkp = fac + F.loff + (ll)c0 * F.ld + c0;   // block (i, j) at blkp[j * ld + i]
+    T r[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j)   // symmetric form: the upper triangle mirrors the lower one
+        r[j] = lane < bw && j < bw ? ((S.sym && lane < j) ? blkp[(ll)lane * F.ld + j] : blkp[(ll)j * F.ld + lane]) : T(0);
     __syncwarp();
-    const bool sing = warp_block_lu32(A, lda, bw, q0, np, piv, S.sym != 0);
-    for (int j = 0; j < bw; ++j)
-        if (lane < bw) fac[F.loff + (ll)(c0 + j) * F.ld + c0 + lane] = A[j * lda + lane];
-    if (lane < bw) ipiv[F.f + c0 + lane] = piv[lane];
-    if (lane == 0 && sing) {   // sing is uniform across the warp
-        for (int pc = 0; pc < np; ++pc) {
-            bool z = false;
-            for (int k = q0[pc]; k < q0[pc + 1]; ++k) z |= A[k * lda + k] == T(0);
-            if (z) { atomicMin(info, p0 + pc + 1); break; }
+    int pos, pa0;
+    const bool sing = warp_block_lu<T, 32>(r, bw, bw, q0, piv, sgm[warp], spa[warp], S.sym != 0, pos, pa0);
+    bool zero = false;   // this row's pivot
+    if (lane < bw) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+            if (j < bw) {
+                blkp[(ll)j * F.ld + (j >= pa0 ? pos : lane)] = r[j];
+                zero |= j == pos && r[j] == T(0);
+            }
+        ipiv[F.f + c0 + lane] = piv[lane];
+    }
+    if (sing) {   // uniform across the warp: the first piece with a zero pivot
+        const unsigned first = __reduce_min_sync(0xffffffffu, zero ? (unsigned)pos : 0xffffffffu);
+        if (lane == 0 && first != 0xffffffffu) {
+            int pc = 0;
+            while (q0[pc + 1] <= (int)first) ++pc;
+            atomicMin(info, p0 + pc + 1);
         }
     }
 }
@@ -371,18 +415,6 @@ __device__ __forceinline__ int warp_first_max_row(unsigned long long key, int id
     const unsigned mh = __reduce_max_sync(FULL, hi);
     const unsigned ml = __reduce_max_sync(FULL, hi == mh ? lo : 0u);
     return (int)__reduce_min_sync(FULL, (hi == mh && lo == ml) ? (unsigned)idx : 0xffffffffu);
-}
-__device__ __forceinline__ int warp_first_max_row(unsigned key, int idx) {
-    const unsigned FULL = 0xffffffffu;
-    const unsigned m = __reduce_max_sync(FULL, key);
-    return (int)__reduce_min_sync(FULL, key == m ? (unsigned)idx : 0xffffffffu);
-}
-// 32-bit pivot key of a float (same order as pivot_key).
-__device__ __forceinline__ unsigned pivot_key32(float x, bool cand, bool diag) {
-    if (!cand) return 0u;
-    const unsigned b = __float_as_uint(x) & 0x7fffffffu;
-    if (b > 0x7f800000u) return diag ? 0xffffffffu : 1u;
-    return b + 2u;
 }
 template <typename T> struct PivotKey;
 template <> struct PivotKey<float> {
@@ -2511,7 +2543,7 @@ constexpr int LF_CLASSES = 4;   // W = 4 << class
 __host__ __device__ constexpr int leaf_class(int bw) { return bw <= 4 ? 0 : bw <= 8 ? 1 : bw <= 16 ? 2 : 3; }
 template <typename T, int W> struct LeafSmem {
     static constexpr int LD = W + 1;
-    static constexpr size_t warp_bytes = (((size_t)(W + LF_M) * LD + W) * sizeof(T) + LF_M * sizeof(ScatterRow) +
+    static constexpr size_t warp_bytes = (((size_t)(W + 2 * LF_M) * LD + W) * sizeof(T) + LF_M * sizeof(ScatterRow) +
                                           (W + 1 + 3 * W) * sizeof(int) + 15) / 16 * 16;
     static constexpr size_t bytes = LF_WARPS * warp_bytes;
 };
@@ -2534,7 +2566,8 @@ __device__ __forceinline__ void leaf_front(T* fac, int* ipiv, int* info, const S
     ScatterRow* tab = reinterpret_cast<ScatterRow*>(base);
     T* sD = reinterpret_cast<T*>(tab + LF_M);          // diagonal block, D(i, j) at sD[j * LD + i]
     T* sL = sD + W * LD;                               // L21 rows, L21(r, k) at sL[r * LD + k]
-    T* srv = sL + LF_M * LD;                           // 1 / U(k, k)
+    T* sV = sL + LF_M * LD;                            // U12 columns, U12(k, c) at sV[c * LD + k]
+    T* srv = sV + LF_M * LD;                           // 1 / U(k, k)
     int* q0 = reinterpret_cast<int*>(srv + W);
     int* piv = q0 + W + 1;
     int* gm = piv + W;
@@ -2543,19 +2576,34 @@ __device__ __forceinline__ void leaf_front(T* fac, int* ipiv, int* info, const S
     const int p0 = S.blk_p0[blk], np = S.blk_np[blk];
     const bool sym = S.sym != 0;
     for (int k = lane; k <= np; k += 32) q0[k] = S.xsuper[p0 + k] - F.f;
-    for (int j = 0; j < bw; ++j)   // symmetric form: the upper triangle mirrors the lower one
-        if (lane < bw)
-            sD[j * LD + lane] = (sym && lane < j) ? ld_fac<COH>(fac + F.loff + (ll)lane * F.ld + j)
-                                                  : ld_fac<COH>(fac + F.loff + (ll)j * F.ld + lane);
+    // the block, with the rows below it where a warp holds both
+    const bool fit = bw + m <= 32;
+    const int nrow = fit ? bw + m : bw;
+    T r0[W];
+#pragma unroll
+    for (int j = 0; j < W; ++j)   // symmetric form: the upper triangle mirrors the lower one
+        r0[j] = lane < nrow && j < bw ? ((sym && lane < j) ? ld_fac<COH>(fac + F.loff + (ll)lane * F.ld + j)
+                                                           : ld_fac<COH>(fac + F.loff + (ll)j * F.ld + lane))
+                                      : T(0);
     for (int x = lane; x < m; x += 32) tab[x] = scatter_row<T>(S, F, x);
     __syncwarp();
     // block LU (ggetrf! pivots inside each piece; none in the symmetric form)
-    const bool sing = warp_block_lu32<T, W>(sD, LD, bw, q0, np, piv, sym);
-    for (int j = 0; j < bw; ++j)
-        if (lane < bw) fac[F.loff + (ll)j * F.ld + lane] = sD[j * LD + lane];
+    int pos, pa0;
+    const bool sing = warp_block_lu<T, W>(r0, bw, nrow, q0, piv, gm, pam, sym, pos, pa0);
+    if (lane < nrow) {
+#pragma unroll
+        for (int j = 0; j < W; ++j)
+            if (j < bw) {
+                const int i = lane >= bw || j < pa0 ? lane : pos;
+                fac[F.loff + (ll)j * F.ld + i] = r0[j];
+                if (lane < bw) sD[j * LD + i] = r0[j];
+                else sL[(lane - bw) * LD + j] = r0[j];
+            }
+    }
+    __syncwarp();
     if (lane < bw) {
         ipiv[F.f + lane] = piv[lane];
-        srv[lane] = rcp_rn(sD[lane * LD + lane]);   // as the panel's 1 / U(k, k)
+        srv[lane] = fit ? T(1) : rcp_rn(sD[lane * LD + lane]);   // as the panel's 1 / U(k, k)
     }
     if (lane == 0 && sing) {
         for (int pc = 0; pc < np; ++pc) {
@@ -2564,24 +2612,11 @@ __device__ __forceinline__ void leaf_front(T* fac, int* ipiv, int* info, const S
             if (z) { atomicMin(info, p0 + pc + 1); break; }
         }
     }
-    for (int pc = lane; pc < np; pc += 32) {   // row sources of the interchanges (block_gather_map)
-        const int a = q0[pc], b = q0[pc + 1];
-        for (int i = a; i < b; ++i) {
-            gm[i] = i;
-            pam[i] = a;
-        }
-        for (int k = a; k < b; ++k) {
-            const int kp = a + piv[k];
-            const int t = gm[k];
-            gm[k] = gm[kp];
-            gm[kp] = t;
-        }
-    }
     __syncwarp();
     // L21 rows (m <= 32: a lane per row): x := x U^-1 (left-looking: entry j
     // gets k = 0, 1, .. then its scaling)
     const int r = lane;
-    if (r < m) {
+    if (!fit && r < m) {
         T x[W];
 #pragma unroll
         for (int k = 0; k < W; ++k) x[k] = k < bw ? ld_fac<COH>(fac + F.loff + (ll)k * F.ld + bw + r) : T(0);
@@ -2622,26 +2657,31 @@ __device__ __forceinline__ void leaf_front(T* fac, int* ipiv, int* info, const S
     if (c < m)
 #pragma unroll
         for (int k = 0; k < W; ++k)
-            if (k < bw) fac[F.uoff + (ll)k * m + c] = y[k];
+            if (k < bw) {
+                fac[F.uoff + (ll)k * m + c] = y[k];
+                sV[c * LD + k] = y[k];
+            }
     __syncwarp();
-    // Schur complement, a lane per column c, rows in order
-    if (c < m) {
-        for (int rr = sym ? c : 0; rr < m; ++rr) {   // the symmetric form forms the lower part only
-            T acc = T(0);
+    // Schur complement, entries (rr, cc) over the lanes, rows fastest: every
+    // lane works whatever m is, and the adds to a column of an ancestor are
+    // contiguous
+    for (int e = lane; e < m * m; e += 32) {
+        const int cc = e / m, rr = e - cc * m;
+        if (sym && rr < cc) continue;   // the symmetric form forms the lower part only
+        T acc = T(0);
 #pragma unroll
-            for (int k = 0; k < W; ++k)
-                if (k < bw) acc += sL[rr * LD + k] * y[k];
-            if (rr >= c) {   // L entry of the front of R_F[c]
-                const ScatterRow& Cc = tab[c];
-                const int p = S.rel[Cc.rel0 + rr];
-                if (Cc.pos >= 0 && p >= 0) atomicAdd(&fac[Cc.loff + (ll)Cc.pos * Cc.ld + p], -acc);
-            } else {   // entry of the front of R_F[rr] (not in the symmetric form)
-                const ScatterRow& R = tab[rr];
-                const int p = S.rel[R.rel0 + c];
-                if (R.pos >= 0 && p >= 0) {
-                    const ll addr = p < R.nf ? R.loff + (ll)p * R.ld + R.pos : R.uoff + (ll)R.pos * R.m + (p - R.nf);
-                    atomicAdd(&fac[addr], -acc);
-                }
+        for (int k = 0; k < W; ++k)
+            if (k < bw) acc += sL[rr * LD + k] * sV[cc * LD + k];
+        if (rr >= cc) {   // L entry of the front of R_F[cc]
+            const ScatterRow& Cc = tab[cc];
+            const int p = S.rel[Cc.rel0 + rr];
+            if (Cc.pos >= 0 && p >= 0) atomicAdd(&fac[Cc.loff + (ll)Cc.pos * Cc.ld + p], -acc);
+        } else {          // entry of the front of R_F[rr]
+            const ScatterRow& R = tab[rr];
+            const int p = S.rel[R.rel0 + cc];
+            if (R.pos >= 0 && p >= 0) {
+                const ll addr = p < R.nf ? R.loff + (ll)p * R.ld + R.pos : R.uoff + (ll)R.pos * R.m + (p - R.nf);
+                atomicAdd(&fac[addr], -acc);
             }
         }
     }
@@ -2655,6 +2695,45 @@ __global__ void __launch_bounds__(32 * LF_WARPS) k_leaf_factor(T* fac, int* ipiv
     const int idx = blockIdx.x * LF_WARPS + warp;
     if (idx >= L.count) return;   // whole warp; the kernel has no CTA barrier
     leaf_front<T, false, W>(fac, ipiv, info, S, S.fronts[L.front_ids[idx]], base);
+}
+
+// Small fronts of every width class in one launch, for levels with few of
+// them: lists ids[i] (class i % LF_CLASSES) hold the fronts up to the running
+// count end[i].
+constexpr int LEAF_LISTS = 2 * LF_CLASSES;
+struct LeafSet {
+    const int* ids[LEAF_LISTS];
+    int end[LEAF_LISTS];
+};
+__device__ __forceinline__ int leaf_of(const LeafSet& L, int idx, int& list) {
+    int first = 0, front = -1;
+    list = LEAF_LISTS;
+#pragma unroll
+    for (int i = 0; i < LEAF_LISTS; ++i) {
+        if (list == LEAF_LISTS && idx < L.end[i]) {
+            list = i;
+            front = L.ids[i][idx - first];
+        }
+        first = L.end[i];
+    }
+    return front;
+}
+template <typename T>
+__global__ void __launch_bounds__(32 * LF_WARPS) k_leaf_factor_set(T* fac, int* ipiv, int* info, Sched S, LeafSet L,
+                                                                   unsigned warp_bytes) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int warp = threadIdx.x >> 5;
+    unsigned char* base = smem_raw + (size_t)warp * warp_bytes;
+    int list;
+    const int fid = leaf_of(L, blockIdx.x * LF_WARPS + warp, list);
+    if (fid < 0) return;   // whole warp; the kernel has no CTA barrier
+    const DFront F = S.fronts[fid];
+    switch (list % LF_CLASSES) {
+    case 0: leaf_front<T, false, 4>(fac, ipiv, info, S, F, base); break;
+    case 1: leaf_front<T, false, 8>(fac, ipiv, info, S, F, base); break;
+    case 2: leaf_front<T, false, 16>(fac, ipiv, info, S, F, base); break;
+    default: leaf_front<T, false, 32>(fac, ipiv, info, S, F, base); break;
+    }
 }
 
 // The bottom subtrees of small fronts (every front of the subtree factored
@@ -3637,15 +3716,12 @@ __device__ __forceinline__ T warp_reduce_scatter(T (&v)[N]) {
     return v[0];
 }
 
+// RG: right-hand sides per pass (1 for a single one, else 4).
 template <typename T, bool FWD, int W, int RG>
-__global__ void __launch_bounds__(256) k_solve_leaf(const T* fac, const T* inv2, T* in, T* out, const T* xs, int n,
-                                                     int nrhs, Sched S, Launch L) {
-    // RG: right-hand sides per pass (1 for a single one, else 4)
+__device__ __forceinline__ void solve_leaf_front(const T* fac, const T* inv2, T* in, T* out, const T* xs, int n, int nrhs,
+                                                 const Sched& S, const DFront& F) {
     const unsigned FULL = 0xffffffffu;
-    griddep_launch();
-    const int lane = threadIdx.x & 31, idx = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (idx >= L.count) return;   // whole warp
-    const DFront F = S.fronts[L.front_ids[idx]];
+    const int lane = threadIdx.x & 31;
     const int blk = F.block0, bw = F.nf;
     const T* Mi = inv2 + S.blk_inv2[blk] + (FWD ? 0 : (ll)bw * bw);
     const int* rows = S.rows + F.rows_off;
@@ -3774,6 +3850,33 @@ __global__ void __launch_bounds__(256) k_solve_leaf(const T* fac, const T* inv2,
                         if (r < nr) atomicAdd(&in[(ll)(r0 + r) * n + rows[i]], -acc[r]);
             }
         }
+    }
+}
+
+template <typename T, bool FWD, int W, int RG>
+__global__ void __launch_bounds__(256) k_solve_leaf(const T* fac, const T* inv2, T* in, T* out, const T* xs, int n,
+                                                     int nrhs, Sched S, Launch L) {
+    griddep_launch();
+    const int idx = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (idx >= L.count) return;   // whole warp
+    const DFront F = S.fronts[L.front_ids[idx]];
+    solve_leaf_front<T, FWD, W, RG>(fac, inv2, in, out, xs, n, nrhs, S, F);
+}
+
+// Every width class in one launch, for levels with few of these fronts.
+template <typename T, bool FWD, int RG>
+__global__ void __launch_bounds__(256) k_solve_leaf_set(const T* fac, const T* inv2, T* in, T* out, const T* xs, int n,
+                                                         int nrhs, Sched S, LeafSet L) {
+    griddep_launch();
+    int list;
+    const int fid = leaf_of(L, blockIdx.x * 8 + (threadIdx.x >> 5), list);
+    if (fid < 0) return;   // whole warp
+    const DFront F = S.fronts[fid];
+    switch (list % LF_CLASSES) {
+    case 0: solve_leaf_front<T, FWD, 4, RG>(fac, inv2, in, out, xs, n, nrhs, S, F); break;
+    case 1: solve_leaf_front<T, FWD, 8, RG>(fac, inv2, in, out, xs, n, nrhs, S, F); break;
+    case 2: solve_leaf_front<T, FWD, 16, RG>(fac, inv2, in, out, xs, n, nrhs, S, F); break;
+    default: solve_leaf_front<T, FWD, 32, RG>(fac, inv2, in, out, xs, n, nrhs, S, F); break;
     }
 }
 
