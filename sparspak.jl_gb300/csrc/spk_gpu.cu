@@ -94,6 +94,10 @@ constexpr int TC_SCHUR_M = 96, TC_TRAIL_ROWS = 128;
 // it gives up and records a timeout.
 constexpr long long WAIT_BUDGET = 1 << 20;
 
+// Fronts of at most SMALL_NF columns and SMALL_M rows below them merge along
+// their chain whatever the padding (analyse).
+constexpr int SMALL_NF = 16, SMALL_M = spk::LF_M;
+
 // Block partition and schedule for one precision (block width BlockMax<T>).
 struct Plan {
     bool built = false;
@@ -502,6 +506,14 @@ static int analyse(spk_handle* h, const int64_t* xsuper, const int64_t* snode, c
     // most the amalgamation allowance.  Exact fundamental chains need no
     // padding; padded positions are structural zeros and stay exactly zero
     // (every product that reaches them has a structurally zero factor).
+    // Small fronts merge whatever their padding: a warp factors or solves one
+    // whole front in one launch, so a longer chain of smaller ones only adds
+    // launches (a tridiagonal system of 1101 unknowns: 551 levels of one- and
+    // two-column fronts without this, 4.7 ms a refactorisation and solve, 36
+    // levels with it, 1.8 ms; 512 batched systems: 1.44 M fronts in 18 levels,
+    // 17.8 ms, 451,000 in 14 levels, 14.3 ms).  Up to 8 columns takes 1.4 and
+    // 15.0 ms, up to 32 columns 2.6 and 14.9 ms, up to 64 rows below them 24.9
+    // instead of 24.1 ms for a 64^3 step.
     h->col_front.assign(n, -1);
     h->fronts.clear();
     auto exact_entries = [&](i64 t) {
@@ -518,7 +530,8 @@ static int analyse(spk_handle* h, const int64_t* xsuper, const int64_t* snode, c
             double ex2 = exact + exact_entries(e + 1);
             double nf = h->xs[e + 2] - h->xs[s];
             double m = (double)(h->xlindx0[e + 2] - h->xlindx0[e + 1]) - (h->xs[e + 2] - h->xs[e + 1]);
-            if (nf * nf + 2.0 * nf * m > (1.0 + h->amalgamation) * ex2) break;
+            const bool small = nf <= SMALL_NF && m <= SMALL_M;
+            if (!small && nf * nf + 2.0 * nf * m > (1.0 + h->amalgamation) * ex2) break;
             exact = ex2;
             ++e;
         }
