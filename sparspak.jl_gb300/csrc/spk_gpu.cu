@@ -1043,6 +1043,38 @@ static size_t panel_smem() {
     return sweep_smem<T, W>(1) + ((std::is_same<T, float>::value && W == 128) ? (size_t)spk::PT_SMEM : 0);
 }
 
+// Shared memory of the cluster front solves for RG right-hand sides at a
+// time, and whether clusters of 16 (a non-portable size) can be held.
+template <typename T, int RG>
+static int prepare_front_solve(spk_handle* h) {
+    constexpr int bytes = (int)spk::FcSmem<T, RG>::bytes;
+    CU(h, (cudaFuncSetAttribute(spk::k_front_solve<T, true, spk::FC, RG>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)));
+    CU(h, (cudaFuncSetAttribute(spk::k_front_solve<T, false, spk::FC, RG>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)));
+    h->fc16 = false;
+    auto k16f = spk::k_front_solve<T, true, 16, RG>;
+    auto k16b = spk::k_front_solve<T, false, 16, RG>;
+    if (cudaFuncSetAttribute(k16f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaFuncSetAttribute(k16b, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+        cudaFuncSetAttribute(k16f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess &&
+        cudaFuncSetAttribute(k16b, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(16);
+        cfg.blockDim = dim3(spk::FC_THREADS);
+        cfg.dynamicSmemBytes = bytes;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = 16;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int nclusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&nclusters, (void*)k16f, &cfg) == cudaSuccess && nclusters >= 1) h->fc16 = true;
+    }
+    cudaGetLastError();   // a refused query leaves clusters of 8
+    return SPK_OK;
+}
+
 template <typename T>
 static int ensure_plan(spk_handle* h) {
     Plan& P = h->plan[plan_index<T>(h)];
@@ -1137,37 +1169,7 @@ static int ensure_plan(spk_handle* h) {
                                                             spk::LeafSmem<T, 32>::bytes));
         P.q_grid = std::max(1, std::min(h->nsm * std::max(per_sm, 1), spk::cdiv(std::max(P.nq, 1), spk::LF_WARPS)));
     }
-    CU(h, cudaFuncSetAttribute(spk::k_front_solve<T, true, spk::FC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)spk::FcSmem<T>::bytes));
-    CU(h, cudaFuncSetAttribute(spk::k_front_solve<T, false, spk::FC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)spk::FcSmem<T>::bytes));
-    {   // clusters of 16 (a non-portable size) where the GPU can hold one
-        h->fc16 = false;
-        auto k16f = spk::k_front_solve<T, true, 16>;
-        auto k16b = spk::k_front_solve<T, false, 16>;
-        if (cudaFuncSetAttribute(k16f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-            cudaFuncSetAttribute(k16b, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-            cudaFuncSetAttribute(k16f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)spk::FcSmem<T>::bytes) ==
-                cudaSuccess &&
-            cudaFuncSetAttribute(k16b, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)spk::FcSmem<T>::bytes) ==
-                cudaSuccess) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(16);
-            cfg.blockDim = dim3(spk::FC_THREADS);
-            cfg.dynamicSmemBytes = spk::FcSmem<T>::bytes;
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim.x = 16;
-            at[0].val.clusterDim.y = 1;
-            at[0].val.clusterDim.z = 1;
-            cfg.attrs = at;
-            cfg.numAttrs = 1;
-            int nclusters = 0;
-            if (cudaOccupancyMaxActiveClusters(&nclusters, (void*)k16f, &cfg) == cudaSuccess && nclusters >= 1)
-                h->fc16 = true;
-        }
-        cudaGetLastError();   // a refused query leaves clusters of 8
-    }
+    if ((rc = prepare_front_solve<T, 1>(h)) || (rc = prepare_front_solve<T, 4>(h))) return rc;
     if (std::is_same<T, float>::value) {
         CU(h, cudaFuncSetAttribute(spk::k_block_lu_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, spk::LuSmem::bytes));
         CU(h, cudaFuncSetAttribute(spk::k_tc_update<spk::TC_TRAIL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1626,6 +1628,31 @@ static int solve_leaf_level(spk_handle* h, const Plan& PL, const LevelPlan& P, i
     return SPK_OK;
 }
 
+// k_front_solve over `fronts` fronts, k_front_gemv (one right-hand side, or
+// four at a time: in FP64 the arithmetic of the three unused ones would cost
+// more than the factor's bytes).
+template <typename T, bool FWD>
+static void launch_front_solve(const spk_handle* h, int fronts, cudaStream_t st, const T* fac, const T* inv, T* in, T* out,
+                               int nrhs, const spk::Sched& S, const spk::Launch& la) {
+    const int n = (int)h->n, nc = h->fc16 ? 16 : spk::FC, grid = nc * fronts;
+    if (nrhs == 1) {
+        constexpr size_t sm = spk::FcSmem<T, 1>::bytes;
+        if (h->fc16) spk::k_front_solve<T, FWD, 16, 1><<<grid, spk::FC_THREADS, sm, st>>>(fac, inv, in, out, n, nrhs, S, la);
+        else spk::k_front_solve<T, FWD, spk::FC, 1><<<grid, spk::FC_THREADS, sm, st>>>(fac, inv, in, out, n, nrhs, S, la);
+    } else {
+        constexpr size_t sm = spk::FcSmem<T, 4>::bytes;
+        if (h->fc16) spk::k_front_solve<T, FWD, 16, 4><<<grid, spk::FC_THREADS, sm, st>>>(fac, inv, in, out, n, nrhs, S, la);
+        else spk::k_front_solve<T, FWD, spk::FC, 4><<<grid, spk::FC_THREADS, sm, st>>>(fac, inv, in, out, n, nrhs, S, la);
+    }
+}
+template <typename T>
+static void launch_front_gemv(const spk_handle* h, const HFront& F, cudaStream_t st, const T* fac, T* out, const T* in, int nrhs,
+                              int r0, int r1, int c0, int c1) {
+    const int grid = spk::cdiv(r1 - r0, spk::L21_ROWS) * spk::cdiv(c1 - c0, spk::L21_COLS);
+    auto kern = nrhs == 1 ? spk::k_front_gemv<T, 1> : spk::k_front_gemv<T, 4>;
+    kern<<<grid, 256, 0, st>>>(fac, out, in, (int)h->n, nrhs, F.loff, F.nf + F.m, (int)F.f, r0, r1, c0, c1);
+}
+
 // The forward substitution over levels [l0, l1) on the permuted work
 // vectors (wb, consumed, -> wy), launched on `st`.
 template <typename T>
@@ -1637,44 +1664,30 @@ static int solve_fwd_levels(spk_handle* h, int nrhs, size_t l0, size_t l1, cudaS
     T* b = (T*)h->d_wb;
     T* y = (T*)h->d_wy;
     const int n = (int)h->n;
-    constexpr size_t fc_smem = spk::FcSmem<T>::bytes;
     for (size_t l = l0; l < l1; ++l) {
         const LevelPlan& P = PL.levels[l];
         if (int rc = solve_leaf_level<T, true>(h, PL, P, SPK_K_FWD, st, b, y, (const T*)nullptr, nrhs)) return rc;
         if (P.front_big.tiles > 0) {
             LaunchScope ls(h, SPK_K_FWD, P.front_big.flops * nrhs, P.front_big.words * sizeof(T));
-            if (h->fc16)
-                spk::k_front_solve<T, true, 16><<<16 * P.front_big.tiles, spk::FC_THREADS, fc_smem, st>>>(
-                    fac, inv, b, y, n, nrhs, S, launch_of(PL, P.front_big));
-            else
-                spk::k_front_solve<T, true, spk::FC><<<spk::FC * P.front_big.tiles, spk::FC_THREADS, fc_smem,
-                                                       st>>>(fac, inv, b, y, n, nrhs, S,
-                                                                    launch_of(PL, P.front_big));
+            launch_front_solve<T, true>(h, P.front_big.tiles, st, fac, inv, b, y, nrhs, S, launch_of(PL, P.front_big));
         }
         if (P.front_l21.tiles > 0) {
             LaunchScope ls(h, SPK_K_FWD, P.front_l21.flops * nrhs, P.front_l21.words * sizeof(T));
-            CU(h, launch_chained(spk::k_fwd_l21<T>, P.front_l21.tiles, 256, 0, st, fac, b, (const T*)y, n, nrhs,
+            CU(h, launch_chained(nrhs == 1 ? spk::k_fwd_l21<T, 1> : spk::k_fwd_l21<T, 4>, P.front_l21.tiles, 256, 0, st, fac, b, (const T*)y, n, nrhs,
                                  S, launch_of(PL, P.front_l21)));
         }
         for (size_t c = 0; c < P.chunks.size(); ++c) {   // chunked root fronts, chunks in order
             const LevelPlan::SolveChunk& ch = P.chunks[c];
             {
                 LaunchScope ls(h, SPK_K_FWD, ch.rec.flops * nrhs, ch.rec.words * sizeof(T));
-                if (h->fc16)
-                    spk::k_front_solve<T, true, 16><<<16, spk::FC_THREADS, fc_smem, st>>>(fac, inv, b, y, n, nrhs, S,
-                                                                                         launch_of(PL, ch.rec));
-                else
-                    spk::k_front_solve<T, true, spk::FC><<<spk::FC, spk::FC_THREADS, fc_smem, st>>>(
-                        fac, inv, b, y, n, nrhs, S, launch_of(PL, ch.rec));
+                launch_front_solve<T, true>(h, 1, st, fac, inv, b, y, nrhs, S, launch_of(PL, ch.rec));
             }
             if (c + 1 < P.chunks.size() && P.chunks[c + 1].front == ch.front) {   // rows below the chunk
                 const HFront& F = h->fronts[ch.front];
                 const int r0 = ch.hi, r1 = F.nf;
                 LaunchScope ls(h, SPK_K_FWD, 2.0 * (r1 - r0) * (ch.hi - ch.lo) * nrhs,
                                (double)(r1 - r0) * (ch.hi - ch.lo) * sizeof(T));
-                const int grid = spk::cdiv(r1 - r0, spk::L21_ROWS) * spk::cdiv(ch.hi - ch.lo, spk::L21_COLS);
-                spk::k_front_gemv<T><<<grid, 256, 0, st>>>(fac, b, (const T*)y, n, nrhs, F.loff, F.nf + F.m,
-                                                          (int)F.f, r0, r1, ch.lo, ch.hi);
+                launch_front_gemv<T>(h, F, st, fac, b, y, nrhs, r0, r1, ch.lo, ch.hi);
             }
         }
         for (size_t t = 0; t < P.fwd_small.size(); ++t)
@@ -1698,44 +1711,30 @@ static int solve_bwd_levels(spk_handle* h, int nrhs, cudaStream_t st) {
     T* y = (T*)h->d_wy;
     T* x = (T*)h->d_wx;
     const int n = (int)h->n;
-    constexpr size_t fc_smem = spk::FcSmem<T>::bytes;
     for (size_t l = PL.levels.size(); l-- > 0;) {
         const LevelPlan& P = PL.levels[l];
         if (int rc = solve_leaf_level<T, false>(h, PL, P, SPK_K_BWD, st, y, x, (const T*)x, nrhs)) return rc;
         if (P.bwdu_small.tiles > 0) {
             LaunchScope ls(h, SPK_K_BWD, P.bwdu_small.flops * nrhs, P.bwdu_small.words * sizeof(T));
-            CU(h, launch_chained(spk::k_bwd_u12<T>, P.bwdu_small.tiles, 256, 0, st, fac, y, x, n, nrhs, S,
+            CU(h, launch_chained(nrhs == 1 ? spk::k_bwd_u12<T, 1> : spk::k_bwd_u12<T, 4>, P.bwdu_small.tiles, 256, 0, st, fac, y, x, n, nrhs, S,
                                  launch_of(PL, P.bwdu_small)));
         }
         if (P.front_big.tiles > 0) {
             LaunchScope ls(h, SPK_K_BWD, P.front_big.flops * nrhs, P.front_big.words * sizeof(T));
-            if (h->fc16)
-                spk::k_front_solve<T, false, 16><<<16 * P.front_big.tiles, spk::FC_THREADS, fc_smem, st>>>(
-                    fac, inv, y, x, n, nrhs, S, launch_of(PL, P.front_big));
-            else
-                spk::k_front_solve<T, false, spk::FC><<<spk::FC * P.front_big.tiles, spk::FC_THREADS, fc_smem,
-                                                        st>>>(fac, inv, y, x, n, nrhs, S,
-                                                                     launch_of(PL, P.front_big));
+            launch_front_solve<T, false>(h, P.front_big.tiles, st, fac, inv, y, x, nrhs, S, launch_of(PL, P.front_big));
         }
         for (size_t c = P.chunks.size(); c-- > 0;) {   // chunked root fronts, chunks in reverse
             const LevelPlan::SolveChunk& ch = P.chunks[c];
             {
                 LaunchScope ls(h, SPK_K_BWD, ch.rec.flops * nrhs, ch.rec.words * sizeof(T));
-                if (h->fc16)
-                    spk::k_front_solve<T, false, 16><<<16, spk::FC_THREADS, fc_smem, st>>>(fac, inv, y, x, n, nrhs,
-                                                                                          S, launch_of(PL, ch.rec));
-                else
-                    spk::k_front_solve<T, false, spk::FC><<<spk::FC, spk::FC_THREADS, fc_smem, st>>>(
-                        fac, inv, y, x, n, nrhs, S, launch_of(PL, ch.rec));
+                launch_front_solve<T, false>(h, 1, st, fac, inv, y, x, nrhs, S, launch_of(PL, ch.rec));
             }
             if (c > 0 && P.chunks[c - 1].front == ch.front) {   // rows above the chunk
                 const HFront& F = h->fronts[ch.front];
                 const int r0 = 0, r1 = ch.lo;
                 LaunchScope ls(h, SPK_K_BWD, 2.0 * (r1 - r0) * (ch.hi - ch.lo) * nrhs,
                                (double)(r1 - r0) * (ch.hi - ch.lo) * sizeof(T));
-                const int grid = spk::cdiv(r1 - r0, spk::L21_ROWS) * spk::cdiv(ch.hi - ch.lo, spk::L21_COLS);
-                spk::k_front_gemv<T><<<grid, 256, 0, st>>>(fac, y, (const T*)x, n, nrhs, F.loff, F.nf + F.m,
-                                                          (int)F.f, r0, r1, ch.lo, ch.hi);
+                launch_front_gemv<T>(h, F, st, fac, y, x, nrhs, r0, r1, ch.lo, ch.hi);
             }
         }
         for (size_t t = 0; t < P.bwd_small.size(); ++t)
@@ -1772,7 +1771,7 @@ static int run_solve_permuted(spk_handle* h, int nrhs, bool transpose) {
             const LevelPlan& P = PL.levels[l];
             if (P.bwdu.tiles > 0) {
                 LaunchScope ls(h, SPK_K_BWD, P.bwdu.flops * nrhs, P.bwdu.words * sizeof(T));
-                CU(h, launch_chained(spk::k_tbwd_l21<T>, P.bwdu.tiles, 256, 0, h->stream, fac, y, x, n, nrhs, S,
+                CU(h, launch_chained(nrhs == 1 ? spk::k_tbwd_l21<T, 1> : spk::k_tbwd_l21<T, 4>, P.bwdu.tiles, 256, 0, h->stream, fac, y, x, n, nrhs, S,
                                      launch_of(PL, P.bwdu)));
             }
             for (size_t t = 0; t < P.bwd.size(); ++t)

@@ -163,6 +163,22 @@ __device__ __forceinline__ unsigned pivot_key32(float x, bool cand, bool diag) {
     return b + 2u;
 }
 
+// 16-byte loads of N entries (N * sizeof(T) a multiple of 16) from shared memory.
+template <int N, typename T>
+__device__ __forceinline__ void sm_load(const T* p, T* v) {
+    constexpr int E = 16 / sizeof(T);
+#pragma unroll
+    for (int q = 0; q < N / E; ++q) {
+        if constexpr (sizeof(T) == 4) {
+            const float4 t = *reinterpret_cast<const float4*>(p + q * E);
+            v[q * E] = t.x; v[q * E + 1] = t.y; v[q * E + 2] = t.z; v[q * E + 3] = t.w;
+        } else {
+            const double2 t = *reinterpret_cast<const double2*>(p + q * E);
+            v[q * E] = t.x; v[q * E + 1] = t.y;
+        }
+    }
+}
+
 // Correctly rounded reciprocal (the value of T(1) / x).
 __device__ __forceinline__ float rcp_rn(float x) { return __frcp_rn(x); }
 __device__ __forceinline__ double rcp_rn(double x) { return __drcp_rn(x); }
@@ -3291,29 +3307,29 @@ __global__ void __launch_bounds__(TS) k_fwd(const T* fac, const T* inv2, T* b, T
 // to y with atomics.  The tile count of a front is
 // cdiv(F.nf, U12_ROWS) * cdiv(F.m, U12_COLS), enough CTAs to keep HBM busy
 // on the wide fronts near the root.
-constexpr int U12_ROWS = 32, U12_COLS = 512, U12_RG = 4;
-template <typename T>
+constexpr int U12_ROWS = 32, U12_COLS = 512;
+template <typename T, int RG>
 __device__ __forceinline__ void front_line_dots(const T* base, ll stride, T* y, const T* x, int n, int nrhs,
                                                 const DFront& F, const int* rows, int tile) {
-    __shared__ T sx[U12_COLS * U12_RG];   // sx[c * U12_RG + r]
+    __shared__ T sx[U12_COLS * RG];   // sx[c * RG + r]
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int ncc = cdiv(F.m, U12_COLS);
     const int i0 = (tile / ncc) * U12_ROWS + wid, c0 = (tile % ncc) * U12_COLS;
     const int nc = min(U12_COLS, F.m - c0);
-    for (int r0 = 0; r0 < nrhs; r0 += U12_RG) {
-        const int nr = min(U12_RG, nrhs - r0);
+    for (int r0 = 0; r0 < nrhs; r0 += RG) {
+        const int nr = min(RG, nrhs - r0);
         if (r0 > 0) __syncthreads();
         for (int c = threadIdx.x; c < nc; c += 256) {
             const int g = rows[c0 + c];
 #pragma unroll
-            for (int r = 0; r < U12_RG; ++r) sx[c * U12_RG + r] = r < nr ? x[(ll)(r0 + r) * n + g] : T(0);
+            for (int r = 0; r < RG; ++r) sx[c * RG + r] = r < nr ? x[(ll)(r0 + r) * n + g] : T(0);
         }
         __syncthreads();
-        T acc[4][U12_RG];
+        T acc[4][RG];
 #pragma unroll
         for (int a = 0; a < 4; ++a)
 #pragma unroll
-            for (int r = 0; r < U12_RG; ++r) acc[a][r] = T(0);
+            for (int r = 0; r < RG; ++r) acc[a][r] = T(0);
         const T* u[4];
         bool live[4];
 #pragma unroll
@@ -3326,18 +3342,18 @@ __device__ __forceinline__ void front_line_dots(const T* base, ll stride, T* y, 
             T uv[4];
 #pragma unroll
             for (int a = 0; a < 4; ++a) uv[a] = live[a] ? u[a][c] : T(0);
-            T xv[U12_RG];
+            T xv[RG];
 #pragma unroll
-            for (int r = 0; r < U12_RG; ++r) xv[r] = sx[c * U12_RG + r];
+            for (int r = 0; r < RG; ++r) xv[r] = sx[c * RG + r];
 #pragma unroll
             for (int a = 0; a < 4; ++a)
 #pragma unroll
-                for (int r = 0; r < U12_RG; ++r) acc[a][r] += uv[a] * xv[r];
+                for (int r = 0; r < RG; ++r) acc[a][r] += uv[a] * xv[r];
         }
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
 #pragma unroll
-            for (int r = 0; r < U12_RG; ++r) {
+            for (int r = 0; r < RG; ++r) {
                 T v = acc[a][r];
 #pragma unroll
                 for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
@@ -3348,14 +3364,14 @@ __device__ __forceinline__ void front_line_dots(const T* base, ll stride, T* y, 
 }
 
 // Backward, part 1: y[F's columns] -= U12 * x[R_F] (U12 row i contiguous in Uf).
-template <typename T>
+template <typename T, int RG>
 __global__ void __launch_bounds__(256) k_bwd_u12(const T* fac, T* y, const T* x, int n, int nrhs, Sched S, Launch L) {
     griddep_launch();
     int fid, tile;
     locate(L, blockIdx.x, fid, tile);
     const DFront F = S.fronts[fid];
     griddep_wait();
-    front_line_dots<T>(fac + F.uoff, F.m, y, x, n, nrhs, F, S.rows + F.rows_off, tile);
+    front_line_dots<T, RG>(fac + F.uoff, F.m, y, x, n, nrhs, F, S.rows + F.rows_off, tile);
 }
 
 // Backward, part 2, for the block `step`-th from the last, tiled as (128
@@ -3461,42 +3477,34 @@ __global__ void __launch_bounds__(TS) k_bwd(const T* fac, const T* inv2, T* y, T
 // owner of the next step after publishing it), so that only the next
 // owner's work is on the chain.  Same operations as k_fwd / k_bwd per step
 // inside the front; forward, the R_F rows get L21 y_F afterwards from
-// k_fwd_l21 (all the GPU's SMs).  Right-hand sides FC_RG at a time.  Fronts
+// k_fwd_l21 (all the GPU's SMs).  Right-hand sides RG at a time.  Fronts
 // with at least FC_MINB and at most FC * FC_OWN blocks take this path (the
 // plan decides).
 // ---------------------------------------------------------------------------
-constexpr int FC = 8, FC_MINB = 4, FC_OWN = 16, FC_RG = 4, FC_THREADS = 1024;
+constexpr int FC = 8, FC_MINB = 4, FC_OWN = 16, FC_THREADS = 1024;
 
-// Vectors of a block for FC_RG right-hand sides: entry (k, r) at k * FC_RG + r.
-template <typename T> struct RgVec;
-template <> struct RgVec<float> {
-    using type = float4;
-    __device__ static void get(const float* p, float (&v)[FC_RG]) {
-        const float4 q = *reinterpret_cast<const float4*>(p);
-        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-    }
-};
-template <> struct RgVec<double> {
-    __device__ static void get(const double* p, double (&v)[FC_RG]) {
-        const double2 q0 = *reinterpret_cast<const double2*>(p), q1 = *reinterpret_cast<const double2*>(p + 2);
-        v[0] = q0.x; v[1] = q0.y; v[2] = q1.x; v[3] = q1.y;
-    }
-};
+// Vectors of a block for RG right-hand sides (4, or 1 for a single one):
+// entry (k, r) at k * RG + r.
+template <int RG, typename T>
+__device__ __forceinline__ void rg_get(const T* p, T (&v)[RG]) {
+    if constexpr (RG == 1) v[0] = p[0];
+    else sm_load<RG>(p, v);
+}
 
-template <typename T>
+template <typename T, int RG>
 struct FcSmem {
     static constexpr int BM = BlockMax<T>::value, CS = FC_THREADS / BM;
-    static constexpr size_t ypub = 0, ycur = ypub + BM * FC_RG, own = ycur + BM * FC_RG,
-                            part = own + (size_t)FC_OWN * BM * FC_RG, preA = part + (size_t)CS * BM * FC_RG,
+    static constexpr size_t ypub = 0, ycur = ypub + BM * RG, own = ycur + BM * RG,
+                            part = own + (size_t)FC_OWN * BM * RG, preA = part + (size_t)CS * BM * RG,
                             preM = preA + (size_t)BM * BM, total = preM + (size_t)BM * BM;   // in T's
     static constexpr size_t bytes = total * sizeof(T);
 };
 
-// v[i * FC_RG + r] -= sum_j A(i, j) w[j * FC_RG + r], i < nrow, j < ncol,
+// v[i * RG + r] -= sum_j A(i, j) w[j * RG + r], i < nrow, j < ncol,
 // with A(i, j) = a[j * lda + i] (a block of the factor in global memory, or
 // its prefetched copy in shared memory).  Thread (i, cs) takes columns
 // cs, cs + CS, ...; all its loads are issued before the first use.
-template <typename T>
+template <typename T, int RG>
 __device__ __forceinline__ void fc_tile_update(const T* a, ll lda, int nrow, int ncol, T* v, const T* w, T* part) {
     constexpr int BM = BlockMax<T>::value, CS = FC_THREADS / BM, NJ = BM / CS;
     const int i = threadIdx.x % BM, cs = threadIdx.x / BM;
@@ -3506,68 +3514,68 @@ __device__ __forceinline__ void fc_tile_update(const T* a, ll lda, int nrow, int
         const int j = cs + q * CS;
         av[q] = (i < nrow && j < ncol) ? a[(ll)j * lda + i] : T(0);
     }
-    T acc[FC_RG];
+    T acc[RG];
 #pragma unroll
-    for (int r = 0; r < FC_RG; ++r) acc[r] = T(0);
+    for (int r = 0; r < RG; ++r) acc[r] = T(0);
 #pragma unroll
     for (int q = 0; q < NJ; ++q) {
-        T wv[FC_RG];
-        RgVec<T>::get(w + (cs + q * CS) * FC_RG, wv);
+        T wv[RG];
+        rg_get<RG>(w + (cs + q * CS) * RG, wv);
 #pragma unroll
-        for (int r = 0; r < FC_RG; ++r) acc[r] += av[q] * wv[r];
+        for (int r = 0; r < RG; ++r) acc[r] += av[q] * wv[r];
     }
 #pragma unroll
-    for (int r = 0; r < FC_RG; ++r) part[(cs * BM + i) * FC_RG + r] = acc[r];
+    for (int r = 0; r < RG; ++r) part[(cs * BM + i) * RG + r] = acc[r];
     __syncthreads();
-    for (int e = threadIdx.x; e < nrow * FC_RG; e += FC_THREADS) {
+    for (int e = threadIdx.x; e < nrow * RG; e += FC_THREADS) {
         T sum = T(0);
 #pragma unroll
-        for (int c = 0; c < CS; ++c) sum += part[c * BM * FC_RG + e];
+        for (int c = 0; c < CS; ++c) sum += part[c * BM * RG + e];
         v[e] -= sum;
     }
     __syncthreads();
 }
 
-// out[j * FC_RG + r] = sum_k op(j, k) v[k * FC_RG + r] for the block's solve
+// out[j * RG + r] = sum_k op(j, k) v[k * RG + r] for the block's solve
 // operator (forward Minv, backward Uinv; op(j, k) at m[k * BM + j]).
-template <typename T, bool FWD>
+template <typename T, bool FWD, int RG>
 __device__ __forceinline__ void fc_block_solve(const T* m, int bw, const T* v, T* out, T* part, int nr) {
     constexpr int BM = BlockMax<T>::value, CS = FC_THREADS / BM;
     const int j = threadIdx.x % BM, cs = threadIdx.x / BM;
-    T acc[FC_RG];
+    T acc[RG];
 #pragma unroll
-    for (int r = 0; r < FC_RG; ++r) acc[r] = T(0);
+    for (int r = 0; r < RG; ++r) acc[r] = T(0);
     if (j < bw) {
 #pragma unroll 4
         for (int k = (FWD ? 0 : j) + cs; k < bw; k += CS) {
             const T mv = m[k * BM + j];
-            T vv[FC_RG];
-            RgVec<T>::get(v + k * FC_RG, vv);
+            T vv[RG];
+            rg_get<RG>(v + k * RG, vv);
 #pragma unroll
-            for (int r = 0; r < FC_RG; ++r) acc[r] += mv * vv[r];
+            for (int r = 0; r < RG; ++r) acc[r] += mv * vv[r];
         }
     }
 #pragma unroll
-    for (int r = 0; r < FC_RG; ++r) part[(cs * BM + j) * FC_RG + r] = acc[r];
+    for (int r = 0; r < RG; ++r) part[(cs * BM + j) * RG + r] = acc[r];
     __syncthreads();
-    for (int e = threadIdx.x; e < BM * FC_RG; e += FC_THREADS) {
-        const int jj = e / FC_RG, r = e % FC_RG;
+    for (int e = threadIdx.x; e < BM * RG; e += FC_THREADS) {
+        const int jj = e / RG, r = e % RG;
         T sum = T(0);
         if (jj < bw && r < nr)
 #pragma unroll
-            for (int c = 0; c < CS; ++c) sum += part[c * BM * FC_RG + e];
+            for (int c = 0; c < CS; ++c) sum += part[c * BM * RG + e];
         out[e] = sum;
     }
     __syncthreads();
 }
 
-template <typename T, bool FWD, int NC>
+template <typename T, bool FWD, int NC, int RG>
 __global__ void __cluster_dims__(NC, 1, 1) __launch_bounds__(FC_THREADS, 1)
     k_front_solve(const T* fac, const T* inv2, T* in, T* out, int n, int nrhs, Sched S, Launch L) {
     constexpr int FC = NC;   // CTAs of the cluster
     namespace cg = cooperative_groups;
     constexpr int BM = BlockMax<T>::value;
-    using SM = FcSmem<T>;
+    using SM = FcSmem<T, RG>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* sm = reinterpret_cast<T*>(smem_raw);
     T* ypub = sm + SM::ypub;
@@ -3603,27 +3611,27 @@ __global__ void __cluster_dims__(NC, 1, 1) __launch_bounds__(FC_THREADS, 1)
             }
         }
     };
-    for (int r0 = 0; r0 < nrhs; r0 += FC_RG) {
-        const int nr = min(FC_RG, nrhs - r0);
+    for (int r0 = 0; r0 < nrhs; r0 += RG) {
+        const int nr = min(RG, nrhs - r0);
         prefetch(rank);
         for (int st = rank, o = 0; st < nb; st += FC, ++o) {   // the owned blocks' right-hand sides
             const int blk = blk_of(st), c0 = S.blk_c0[blk], bw = S.blk_c1[blk] - c0;
-            T* v = own + (size_t)o * BM * FC_RG;
-            for (int e = tid; e < BM * FC_RG; e += FC_THREADS) {
-                const int k = e / FC_RG, r = e % FC_RG;
+            T* v = own + (size_t)o * BM * RG;
+            for (int e = tid; e < BM * RG; e += FC_THREADS) {
+                const int k = e / RG, r = e % RG;
                 v[e] = (k < bw && r < nr) ? in[(ll)(r0 + r) * n + F.f + c0 + k] : T(0);
             }
         }
         __syncthreads();
         auto solve_step = [&](int st) {   // owner: publish the solution of step st
             const int blk = blk_of(st), bw = S.blk_c1[blk] - S.blk_c0[blk];
-            fc_block_solve<T, FWD>(preM, bw, own + (size_t)(st / FC) * BM * FC_RG, ypub, part, nr);
+            fc_block_solve<T, FWD, RG>(preM, bw, own + (size_t)(st / FC) * BM * RG, ypub, part, nr);
         };
         auto finish_step = [&](int st) {   // owner, after the barrier arrival: output and next prefetch
             const int blk = blk_of(st), c0 = S.blk_c0[blk], bw = S.blk_c1[blk] - c0;
             for (int e = tid; e < bw * nr; e += FC_THREADS) {
                 const int j = e % bw, r = e / bw;
-                out[(ll)(r0 + r) * n + F.f + c0 + j] = ypub[j * FC_RG + r];
+                out[(ll)(r0 + r) * n + F.f + c0 + j] = ypub[j * RG + r];
             }
             prefetch(st + FC);   // preM / preA are free again
         };
@@ -3637,7 +3645,7 @@ __global__ void __cluster_dims__(NC, 1, 1) __launch_bounds__(FC_THREADS, 1)
         for (int t = 0; t < nb; ++t) {
             cl.barrier_wait();
             const T* src = cl.map_shared_rank(ypub, t % FC);
-            for (int e = tid; e < BM * FC_RG; e += FC_THREADS) ycur[e] = src[e];
+            for (int e = tid; e < BM * RG; e += FC_THREADS) ycur[e] = src[e];
             __syncthreads();
             const int bt = blk_of(t), ncol = S.blk_c1[bt] - S.blk_c0[bt];
             const bool next = t + 1 < nb && (t + 1) % FC == rank;
@@ -3645,8 +3653,8 @@ __global__ void __cluster_dims__(NC, 1, 1) __launch_bounds__(FC_THREADS, 1)
                 cp_wait_all();
                 __syncthreads();
                 const int bs = blk_of(t + 1);
-                fc_tile_update<T>(preA, BM, S.blk_c1[bs] - S.blk_c0[bs], ncol,
-                                  own + (size_t)((t + 1) / FC) * BM * FC_RG, ycur, part);
+                fc_tile_update<T, RG>(preA, BM, S.blk_c1[bs] - S.blk_c0[bs], ncol,
+                                  own + (size_t)((t + 1) / FC) * BM * RG, ycur, part);
                 solve_step(t + 1);
             }
             cl.barrier_arrive();
@@ -3654,8 +3662,8 @@ __global__ void __cluster_dims__(NC, 1, 1) __launch_bounds__(FC_THREADS, 1)
             for (int st = rank, o = 0; st < nb; st += FC, ++o)
                 if (st > t && !(next && st == t + 1)) {
                     const int bs = blk_of(st);
-                    fc_tile_update<T>(a_of(bs, bt), F.ld, S.blk_c1[bs] - S.blk_c0[bs], ncol,
-                                      own + (size_t)o * BM * FC_RG, ycur, part);
+                    fc_tile_update<T, RG>(a_of(bs, bt), F.ld, S.blk_c1[bs] - S.blk_c0[bs], ncol,
+                                      own + (size_t)o * BM * RG, ycur, part);
                 }
             __syncthreads();
         }
@@ -3885,9 +3893,9 @@ __global__ void __launch_bounds__(256) k_solve_leaf_set(const T* fac, const T* i
 // (L21 column k contiguous in Lf), y_F of the tile's columns in shared
 // memory, partial sums added to b with atomics.
 constexpr int L21_ROWS = 256, L21_COLS = 64;   // 64 columns: twice the CTAs and loads in flight of 128
-template <typename T>
+template <typename T, int RG>
 __global__ void __launch_bounds__(256) k_fwd_l21(const T* fac, T* b, const T* y, int n, int nrhs, Sched S, Launch L) {
-    __shared__ T sy[L21_COLS * FC_RG];
+    __shared__ T sy[L21_COLS * RG];
     griddep_launch();
     int fid, tile;
     locate(L, blockIdx.x, fid, tile);
@@ -3898,26 +3906,26 @@ __global__ void __launch_bounds__(256) k_fwd_l21(const T* fac, T* b, const T* y,
     const int grow = ok ? S.rows[F.rows_off + i] : 0;
     const T* a = fac + F.loff + (ll)k0 * F.ld + F.nf + (ok ? i : 0);
     griddep_wait();
-    for (int r0 = 0; r0 < nrhs; r0 += FC_RG) {
-        const int nr = min(FC_RG, nrhs - r0);
+    for (int r0 = 0; r0 < nrhs; r0 += RG) {
+        const int nr = min(RG, nrhs - r0);
         if (r0 > 0) __syncthreads();
-        for (int e = threadIdx.x; e < L21_COLS * FC_RG; e += blockDim.x) {
+        for (int e = threadIdx.x; e < L21_COLS * RG; e += blockDim.x) {
             const int k = e % L21_COLS, r = e / L21_COLS;
             sy[e] = (k < nk && r < nr) ? y[(ll)(r0 + r) * n + F.f + k0 + k] : T(0);
         }
         __syncthreads();
-        T acc[FC_RG];
+        T acc[RG];
 #pragma unroll
-        for (int r = 0; r < FC_RG; ++r) acc[r] = T(0);
+        for (int r = 0; r < RG; ++r) acc[r] = T(0);
         if (ok) {
 #pragma unroll 16
             for (int k = 0; k < nk; ++k) {
                 const T av = a[(ll)k * F.ld];
 #pragma unroll
-                for (int r = 0; r < FC_RG; ++r) acc[r] += av * sy[r * L21_COLS + k];
+                for (int r = 0; r < RG; ++r) acc[r] += av * sy[r * L21_COLS + k];
             }
 #pragma unroll
-            for (int r = 0; r < FC_RG; ++r)
+            for (int r = 0; r < RG; ++r)
                 if (r < nr) atomicAdd(&b[(ll)(r0 + r) * n + grow], -acc[r]);
         }
     }
@@ -3931,35 +3939,35 @@ __global__ void __launch_bounds__(256) k_fwd_l21(const T* fac, T* b, const T* y,
 // r]; forward the L rows below the chunk, backward the U rows above it).
 // Tiles of L21_ROWS rows x L21_COLS columns, atomics as k_fwd_l21.
 constexpr int FC_CHUNK = 16;   // blocks per chunk at most
-template <typename T>
+template <typename T, int RG>
 __global__ void __launch_bounds__(256) k_front_gemv(const T* fac, T* out, const T* in, int n, int nrhs, ll loff, int ld,
                                                     int f, int r0, int r1, int c0, int c1) {
-    __shared__ T sv[L21_COLS * FC_RG];
+    __shared__ T sv[L21_COLS * RG];
     const int nrt = cdiv(r1 - r0, L21_ROWS);
     const int i0 = r0 + (int)(blockIdx.x % nrt) * L21_ROWS, k0 = c0 + (int)(blockIdx.x / nrt) * L21_COLS;
     const int nk = min(L21_COLS, c1 - k0), i = i0 + threadIdx.x;
     const bool ok = i < r1;
     const T* a = fac + loff + (ll)k0 * ld + (ok ? i : 0);
-    for (int q0 = 0; q0 < nrhs; q0 += FC_RG) {
-        const int nr = min(FC_RG, nrhs - q0);
+    for (int q0 = 0; q0 < nrhs; q0 += RG) {
+        const int nr = min(RG, nrhs - q0);
         if (q0 > 0) __syncthreads();
-        for (int e = threadIdx.x; e < L21_COLS * FC_RG; e += blockDim.x) {
+        for (int e = threadIdx.x; e < L21_COLS * RG; e += blockDim.x) {
             const int k = e % L21_COLS, r = e / L21_COLS;
             sv[e] = (k < nk && r < nr) ? in[(ll)(q0 + r) * n + f + k0 + k] : T(0);
         }
         __syncthreads();
-        T acc[FC_RG];
+        T acc[RG];
 #pragma unroll
-        for (int r = 0; r < FC_RG; ++r) acc[r] = T(0);
+        for (int r = 0; r < RG; ++r) acc[r] = T(0);
         if (ok) {
 #pragma unroll 16
             for (int k = 0; k < nk; ++k) {
                 const T av = a[(ll)k * ld];
 #pragma unroll
-                for (int r = 0; r < FC_RG; ++r) acc[r] += av * sv[r * L21_COLS + k];
+                for (int r = 0; r < RG; ++r) acc[r] += av * sv[r * L21_COLS + k];
             }
 #pragma unroll
-            for (int r = 0; r < FC_RG; ++r)
+            for (int r = 0; r < RG; ++r)
                 if (r < nr) atomicAdd(&out[(ll)(q0 + r) * n + f + i], -acc[r]);
         }
     }
@@ -4062,14 +4070,14 @@ __global__ void __launch_bounds__(TS) k_tfwd(const T* fac, const T* inv2, T* b, 
 }
 
 // Pass 2, per front: z[F's columns] -= L21^T x[R_F] (L21 column k contiguous in Lf).
-template <typename T>
+template <typename T, int RG>
 __global__ void __launch_bounds__(256) k_tbwd_l21(const T* fac, T* z, const T* x, int n, int nrhs, Sched S, Launch L) {
     griddep_launch();
     int fid, tile;
     locate(L, blockIdx.x, fid, tile);
     const DFront F = S.fronts[fid];
     griddep_wait();
-    front_line_dots<T>(fac + F.loff + F.nf, F.ld, z, x, n, nrhs, F, S.rows + F.rows_off, tile);
+    front_line_dots<T, RG>(fac + F.loff + F.nf, F.ld, z, x, n, nrhs, F, S.rows + F.rows_off, tile);
 }
 
 // Pass 2, block `step`-th from the last: x_chunk = (Minv^T)[chunk, :] z_B,
