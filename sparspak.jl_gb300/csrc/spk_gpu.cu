@@ -53,20 +53,20 @@ struct Timed {
 // panel and trailing kernels; then the Schur complements; for the solves
 // the forward block steps, and backward the U12 product and block steps.
 struct LevelPlan {
-    LaunchRec schur, schur_tc, bwdu;
+    LaunchRec schur, schur_tc;
     // schur_tc in two parts: the tiles whose targets the next level factors
     // (near) and the others (far, beside the next level's factorisation)
     LaunchRec schur_tc_near, schur_tc_far;
     // btrail_tc0: tile 0 of each packed front's trailing update (it holds the
     // next block's diagonal block); btrail_tc: its tiles 1..
-    std::vector<LaunchRec> blu, bpanel, btrail, btrail_tc0, btrail_tc, fwd, bwd;
+    std::vector<LaunchRec> blu, bpanel, btrail, btrail_tc0, btrail_tc;
     // bpanel split in two parts: the near tiles (the first 128 rows below the
     // block and columns right of it, which tile 0 reads) and the far ones
     std::vector<LaunchRec> bpanel_near, bpanel_far;
     std::vector<char> blu_pc;   // every piece of the step's blocks is at most 32 columns (k_block_lu_pc)
     // Solves: fronts with many blocks by one cluster launch each direction
     // (front_big, one tile per front), the others by block steps
-    // (fwd_small / bwd_small); the transposed solves use fwd / bwd.
+    // (fwd_small / bwd_small); the transposed solves likewise.
     // fronts factored whole by k_leaf_factor (a warp each), by width class;
     // leaf_q: the leaf queue's fronts of this level, for when the queue is off
     LaunchRec leaf_factor[spk::LF_CLASSES], leaf_q[spk::LF_CLASSES];
@@ -775,8 +775,6 @@ static void build_plan(const spk_handle* h, Plan& P, int bmax, bool tc, bool sym
         L.btrail.resize(maxb);
         L.btrail_tc0.resize(maxb);
         L.btrail_tc.resize(maxb);
-        L.fwd.resize(maxb);
-        L.bwd.resize(maxb);
         L.fwd_small.resize(maxb);
         L.bwd_small.resize(maxb);
         std::vector<char> big(nid, 0), leaf(nid, 0);
@@ -959,8 +957,6 @@ static void build_plan(const spk_handle* h, Plan& P, int bmax, bool tc, bool sym
                 add_launch(&P, L.btrail_tc0[t], ids, ttc0, f0, w0);
                 add_launch(&P, L.btrail_tc[t], ids, ttc, f1, w1);
             }
-            add_launch(&P, L.fwd[t], ids, tf, ff, wf);
-            add_launch(&P, L.bwd[t], ids, tb, fb, wb);
             for (size_t k = 0; k < nid; ++k)
                 if (big[k] || leaf[k]) tf[k] = tb[k] = 0;
             add_launch(&P, L.fwd_small[t], ids, tf, ff, wf);
@@ -1005,7 +1001,6 @@ static void build_plan(const spk_handle* h, Plan& P, int bmax, bool tc, bool sym
             add_launch(&P, L.schur_tc_near, ids, tn, fn, wn);
             add_launch(&P, L.schur_tc_far, ids, tfar, ffar, wfar);
         }
-        add_launch(&P, L.bwdu, ids, tbu, fu, wu);
         for (size_t k = 0; k < nid; ++k)
             if (leaf[k]) tbu[k] = 0;
         add_launch(&P, L.bwdu_small, ids, tbu, fu, wu);
@@ -1045,14 +1040,14 @@ static size_t panel_smem() {
 
 // Shared memory of the cluster front solves for RG right-hand sides at a
 // time, and whether clusters of 16 (a non-portable size) can be held.
-template <typename T, int RG>
+template <typename T, int RG, bool TRANS>
 static int prepare_front_solve(spk_handle* h) {
     constexpr int bytes = (int)spk::FcSmem<T, RG>::bytes;
-    CU(h, (cudaFuncSetAttribute(spk::k_front_solve<T, true, spk::FC, RG>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)));
-    CU(h, (cudaFuncSetAttribute(spk::k_front_solve<T, false, spk::FC, RG>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)));
+    CU(h, (cudaFuncSetAttribute(spk::k_front_solve<T, true, spk::FC, RG, TRANS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)));
+    CU(h, (cudaFuncSetAttribute(spk::k_front_solve<T, false, spk::FC, RG, TRANS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)));
     h->fc16 = false;
-    auto k16f = spk::k_front_solve<T, true, 16, RG>;
-    auto k16b = spk::k_front_solve<T, false, 16, RG>;
+    auto k16f = spk::k_front_solve<T, true, 16, RG, TRANS>;
+    auto k16b = spk::k_front_solve<T, false, 16, RG, TRANS>;
     if (cudaFuncSetAttribute(k16f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
         cudaFuncSetAttribute(k16b, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
         cudaFuncSetAttribute(k16f, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess &&
@@ -1169,7 +1164,9 @@ static int ensure_plan(spk_handle* h) {
                                                             spk::LeafSmem<T, 32>::bytes));
         P.q_grid = std::max(1, std::min(h->nsm * std::max(per_sm, 1), spk::cdiv(std::max(P.nq, 1), spk::LF_WARPS)));
     }
-    if ((rc = prepare_front_solve<T, 1>(h)) || (rc = prepare_front_solve<T, 4>(h))) return rc;
+    if ((rc = prepare_front_solve<T, 1, false>(h)) || (rc = prepare_front_solve<T, 4, false>(h)) ||
+        (rc = prepare_front_solve<T, 1, true>(h)) || (rc = prepare_front_solve<T, 4, true>(h)))
+        return rc;
     if (std::is_same<T, float>::value) {
         CU(h, cudaFuncSetAttribute(spk::k_block_lu_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, spk::LuSmem::bytes));
         CU(h, cudaFuncSetAttribute(spk::k_tc_update<spk::TC_TRAIL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1300,7 +1297,7 @@ static spk::LeafSet leaf_set(const Plan& PL, const LaunchRec* const (&lists)[spk
     return s;
 }
 
-template <typename T>
+template <typename T, bool TRANS>
 static int solve_fwd_levels(spk_handle* h, int nrhs, size_t l0, size_t l1, cudaStream_t st);
 
 // Levels whose forward substitution a fused factorisation + solve runs
@@ -1385,7 +1382,7 @@ static int factor_launches(spk_handle* h, int fs_nrhs = 0) {
                 LaunchScope ls(h, SPK_K_PERMUTE, 0.0, (double)tot * (8 + 4 + sizeof(T)));
                 spk::k_permute<double, T><<<(int)((tot + 255) / 256), 256, 0, h->side2>>>(
                     h->d_rhs, h->n, (T*)h->d_wb, (int)h->n, h->d_rperm, (int)h->n, fs_nrhs);
-                int rc = solve_fwd_levels<T>(h, fs_nrhs, 0, lvl, h->side2);
+                int rc = solve_fwd_levels<T, false>(h, fs_nrhs, 0, lvl, h->side2);
                 if (rc) return rc;
             }
             CU(h, cudaEventRecord(h->evI, h->side2));
@@ -1573,29 +1570,29 @@ static int run_factor(spk_handle* h) {
 }
 
 // k_solve_leaf of width class c over `count` fronts (chained launch).
-template <typename T, bool FWD>
+template <typename T, bool FWD, bool TRANS>
 static cudaError_t launch_solve_leaf(int c, int count, cudaStream_t st, const T* fac, const T* inv, T* in, T* out,
                                      const T* xs, int n, int nrhs, const spk::Sched& S, const spk::Launch& la) {
     const int grid = (count + 7) / 8;
     if (nrhs == 1) {   // one right-hand side: passes of one
         switch (c) {
-        case 0: return launch_chained(spk::k_solve_leaf<T, FWD, 4, 1>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs, S, la);
-        case 1: return launch_chained(spk::k_solve_leaf<T, FWD, 8, 1>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs, S, la);
-        case 2: return launch_chained(spk::k_solve_leaf<T, FWD, 16, 1>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs, S, la);
-        default: return launch_chained(spk::k_solve_leaf<T, FWD, 32, 1>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs, S, la);
+        case 0: return launch_chained(spk::k_solve_leaf<T, FWD, 4, 1, TRANS>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs, S, la);
+        case 1: return launch_chained(spk::k_solve_leaf<T, FWD, 8, 1, TRANS>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs, S, la);
+        case 2: return launch_chained(spk::k_solve_leaf<T, FWD, 16, 1, TRANS>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs, S, la);
+        default: return launch_chained(spk::k_solve_leaf<T, FWD, 32, 1, TRANS>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs, S, la);
         }
     }
     switch (c) {
-    case 0: return launch_chained(spk::k_solve_leaf<T, FWD, 4, 4>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs, S, la);
-    case 1: return launch_chained(spk::k_solve_leaf<T, FWD, 8, 4>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs, S, la);
-    case 2: return launch_chained(spk::k_solve_leaf<T, FWD, 16, 4>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs, S, la);
-    default: return launch_chained(spk::k_solve_leaf<T, FWD, 32, 4>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs, S, la);
+    case 0: return launch_chained(spk::k_solve_leaf<T, FWD, 4, 4, TRANS>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs, S, la);
+    case 1: return launch_chained(spk::k_solve_leaf<T, FWD, 8, 4, TRANS>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs, S, la);
+    case 2: return launch_chained(spk::k_solve_leaf<T, FWD, 16, 4, TRANS>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs, S, la);
+    default: return launch_chained(spk::k_solve_leaf<T, FWD, 32, 4, TRANS>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs, S, la);
     }
 }
 
 // A level's small fronts, forward or backward: one launch for all width
 // classes, or one each (LEAF_MERGE).
-template <typename T, bool FWD>
+template <typename T, bool FWD, bool TRANS>
 static int solve_leaf_level(spk_handle* h, const Plan& PL, const LevelPlan& P, int kind, cudaStream_t st, T* in, T* out,
                             const T* xs, int nrhs) {
     const T* fac = storage<T>(h).d;
@@ -1613,9 +1610,9 @@ static int solve_leaf_level(spk_handle* h, const Plan& PL, const LevelPlan& P, i
         }
         LaunchScope ls(h, kind, fl * nrhs, wl * sizeof(T));
         const int grid = spk::cdiv(total, 8);
-        CU(h, nrhs == 1 ? launch_chained(spk::k_solve_leaf_set<T, FWD, 1>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs,
+        CU(h, nrhs == 1 ? launch_chained(spk::k_solve_leaf_set<T, FWD, 1, TRANS>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs,
                                          PL.sched, set)
-                        : launch_chained(spk::k_solve_leaf_set<T, FWD, 4>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs,
+                        : launch_chained(spk::k_solve_leaf_set<T, FWD, 4, TRANS>, grid, 256, 0, st, fac, inv, in, out, xs, n, nrhs,
                                          PL.sched, set));
         return SPK_OK;
     }
@@ -1623,7 +1620,7 @@ static int solve_leaf_level(spk_handle* h, const Plan& PL, const LevelPlan& P, i
         const LaunchRec& R = P.front_leaf[c];
         if (R.tiles == 0) continue;
         LaunchScope ls(h, kind, R.flops * nrhs, R.words * sizeof(T));
-        CU(h, (launch_solve_leaf<T, FWD>(c, R.count, st, fac, inv, in, out, xs, n, nrhs, PL.sched, launch_of(PL, R))));
+        CU(h, (launch_solve_leaf<T, FWD, TRANS>(c, R.count, st, fac, inv, in, out, xs, n, nrhs, PL.sched, launch_of(PL, R))));
     }
     return SPK_OK;
 }
@@ -1631,31 +1628,36 @@ static int solve_leaf_level(spk_handle* h, const Plan& PL, const LevelPlan& P, i
 // k_front_solve over `fronts` fronts, k_front_gemv (one right-hand side, or
 // four at a time: in FP64 the arithmetic of the three unused ones would cost
 // more than the factor's bytes).
-template <typename T, bool FWD>
+template <typename T, bool FWD, bool TRANS>
 static void launch_front_solve(const spk_handle* h, int fronts, cudaStream_t st, const T* fac, const T* inv, T* in, T* out,
                                int nrhs, const spk::Sched& S, const spk::Launch& la) {
     const int n = (int)h->n, nc = h->fc16 ? 16 : spk::FC, grid = nc * fronts;
     if (nrhs == 1) {
         constexpr size_t sm = spk::FcSmem<T, 1>::bytes;
-        if (h->fc16) spk::k_front_solve<T, FWD, 16, 1><<<grid, spk::FC_THREADS, sm, st>>>(fac, inv, in, out, n, nrhs, S, la);
-        else spk::k_front_solve<T, FWD, spk::FC, 1><<<grid, spk::FC_THREADS, sm, st>>>(fac, inv, in, out, n, nrhs, S, la);
+        if (h->fc16) spk::k_front_solve<T, FWD, 16, 1, TRANS><<<grid, spk::FC_THREADS, sm, st>>>(fac, inv, in, out, n, nrhs, S, la);
+        else spk::k_front_solve<T, FWD, spk::FC, 1, TRANS><<<grid, spk::FC_THREADS, sm, st>>>(fac, inv, in, out, n, nrhs, S, la);
     } else {
         constexpr size_t sm = spk::FcSmem<T, 4>::bytes;
-        if (h->fc16) spk::k_front_solve<T, FWD, 16, 4><<<grid, spk::FC_THREADS, sm, st>>>(fac, inv, in, out, n, nrhs, S, la);
-        else spk::k_front_solve<T, FWD, spk::FC, 4><<<grid, spk::FC_THREADS, sm, st>>>(fac, inv, in, out, n, nrhs, S, la);
+        if (h->fc16) spk::k_front_solve<T, FWD, 16, 4, TRANS><<<grid, spk::FC_THREADS, sm, st>>>(fac, inv, in, out, n, nrhs, S, la);
+        else spk::k_front_solve<T, FWD, spk::FC, 4, TRANS><<<grid, spk::FC_THREADS, sm, st>>>(fac, inv, in, out, n, nrhs, S, la);
     }
 }
-template <typename T>
+template <typename T, bool TRANS>
 static void launch_front_gemv(const spk_handle* h, const HFront& F, cudaStream_t st, const T* fac, T* out, const T* in, int nrhs,
                               int r0, int r1, int c0, int c1) {
+    if constexpr (TRANS) {
+        auto kern = nrhs == 1 ? spk::k_front_gemv_t<T, 1> : spk::k_front_gemv_t<T, 4>;
+        kern<<<spk::cdiv(r1 - r0, spk::GT_ROWS), 256, 0, st>>>(fac, out, in, (int)h->n, nrhs, F.loff, F.nf + F.m, (int)F.f, r0, r1, c0, c1);
+        return;
+    }
     const int grid = spk::cdiv(r1 - r0, spk::L21_ROWS) * spk::cdiv(c1 - c0, spk::L21_COLS);
     auto kern = nrhs == 1 ? spk::k_front_gemv<T, 1> : spk::k_front_gemv<T, 4>;
     kern<<<grid, 256, 0, st>>>(fac, out, in, (int)h->n, nrhs, F.loff, F.nf + F.m, (int)F.f, r0, r1, c0, c1);
 }
 
-// The forward substitution over levels [l0, l1) on the permuted work
+// The forward substitution (TRANS: by U^T) over levels [l0, l1) on the permuted work
 // vectors (wb, consumed, -> wy), launched on `st`.
-template <typename T>
+template <typename T, bool TRANS>
 static int solve_fwd_levels(spk_handle* h, int nrhs, size_t l0, size_t l1, cudaStream_t st) {
     const T* fac = storage<T>(h).d;
     const T* inv = storage<T>(h).inv2;
@@ -1666,34 +1668,34 @@ static int solve_fwd_levels(spk_handle* h, int nrhs, size_t l0, size_t l1, cudaS
     const int n = (int)h->n;
     for (size_t l = l0; l < l1; ++l) {
         const LevelPlan& P = PL.levels[l];
-        if (int rc = solve_leaf_level<T, true>(h, PL, P, SPK_K_FWD, st, b, y, (const T*)nullptr, nrhs)) return rc;
+        if (int rc = solve_leaf_level<T, true, TRANS>(h, PL, P, SPK_K_FWD, st, b, y, (const T*)nullptr, nrhs)) return rc;
         if (P.front_big.tiles > 0) {
             LaunchScope ls(h, SPK_K_FWD, P.front_big.flops * nrhs, P.front_big.words * sizeof(T));
-            launch_front_solve<T, true>(h, P.front_big.tiles, st, fac, inv, b, y, nrhs, S, launch_of(PL, P.front_big));
+            launch_front_solve<T, true, TRANS>(h, P.front_big.tiles, st, fac, inv, b, y, nrhs, S, launch_of(PL, P.front_big));
         }
         if (P.front_l21.tiles > 0) {
             LaunchScope ls(h, SPK_K_FWD, P.front_l21.flops * nrhs, P.front_l21.words * sizeof(T));
-            CU(h, launch_chained(nrhs == 1 ? spk::k_fwd_l21<T, 1> : spk::k_fwd_l21<T, 4>, P.front_l21.tiles, 256, 0, st, fac, b, (const T*)y, n, nrhs,
+            CU(h, launch_chained(nrhs == 1 ? spk::k_fwd_l21<T, 1, TRANS> : spk::k_fwd_l21<T, 4, TRANS>, P.front_l21.tiles, 256, 0, st, fac, b, (const T*)y, n, nrhs,
                                  S, launch_of(PL, P.front_l21)));
         }
         for (size_t c = 0; c < P.chunks.size(); ++c) {   // chunked root fronts, chunks in order
             const LevelPlan::SolveChunk& ch = P.chunks[c];
             {
                 LaunchScope ls(h, SPK_K_FWD, ch.rec.flops * nrhs, ch.rec.words * sizeof(T));
-                launch_front_solve<T, true>(h, 1, st, fac, inv, b, y, nrhs, S, launch_of(PL, ch.rec));
+                launch_front_solve<T, true, TRANS>(h, 1, st, fac, inv, b, y, nrhs, S, launch_of(PL, ch.rec));
             }
             if (c + 1 < P.chunks.size() && P.chunks[c + 1].front == ch.front) {   // rows below the chunk
                 const HFront& F = h->fronts[ch.front];
                 const int r0 = ch.hi, r1 = F.nf;
                 LaunchScope ls(h, SPK_K_FWD, 2.0 * (r1 - r0) * (ch.hi - ch.lo) * nrhs,
                                (double)(r1 - r0) * (ch.hi - ch.lo) * sizeof(T));
-                launch_front_gemv<T>(h, F, st, fac, b, y, nrhs, r0, r1, ch.lo, ch.hi);
+                launch_front_gemv<T, TRANS>(h, F, st, fac, b, y, nrhs, r0, r1, ch.lo, ch.hi);
             }
         }
         for (size_t t = 0; t < P.fwd_small.size(); ++t)
             if (P.fwd_small[t].tiles > 0) {
                 LaunchScope ls(h, SPK_K_FWD, P.fwd_small[t].flops * nrhs, P.fwd_small[t].words * sizeof(T));
-                CU(h, launch_chained(spk::k_fwd<T>, P.fwd_small[t].tiles, spk::TS, 0, st, fac, inv, b, y, n,
+                CU(h, launch_chained(TRANS ? spk::k_tfwd<T> : spk::k_fwd<T>, P.fwd_small[t].tiles, spk::TS, 0, st, fac, inv, b, y, n,
                                      nrhs, S, launch_of(PL, P.fwd_small[t]), (int)t));
             }
     }
@@ -1701,8 +1703,8 @@ static int solve_fwd_levels(spk_handle* h, int nrhs, size_t l0, size_t l1, cudaS
     return SPK_OK;
 }
 
-// The backward substitution over every level (wy -> wx), launched on `st`.
-template <typename T>
+// The backward substitution (TRANS: by L^T) over every level (wy -> wx), launched on `st`.
+template <typename T, bool TRANS>
 static int solve_bwd_levels(spk_handle* h, int nrhs, cudaStream_t st) {
     const T* fac = storage<T>(h).d;
     const T* inv = storage<T>(h).inv2;
@@ -1713,34 +1715,36 @@ static int solve_bwd_levels(spk_handle* h, int nrhs, cudaStream_t st) {
     const int n = (int)h->n;
     for (size_t l = PL.levels.size(); l-- > 0;) {
         const LevelPlan& P = PL.levels[l];
-        if (int rc = solve_leaf_level<T, false>(h, PL, P, SPK_K_BWD, st, y, x, (const T*)x, nrhs)) return rc;
+        if (int rc = solve_leaf_level<T, false, TRANS>(h, PL, P, SPK_K_BWD, st, y, x, (const T*)x, nrhs)) return rc;
         if (P.bwdu_small.tiles > 0) {
             LaunchScope ls(h, SPK_K_BWD, P.bwdu_small.flops * nrhs, P.bwdu_small.words * sizeof(T));
-            CU(h, launch_chained(nrhs == 1 ? spk::k_bwd_u12<T, 1> : spk::k_bwd_u12<T, 4>, P.bwdu_small.tiles, 256, 0, st, fac, y, x, n, nrhs, S,
+            const auto lines = TRANS ? (nrhs == 1 ? spk::k_tbwd_l21<T, 1> : spk::k_tbwd_l21<T, 4>)
+                                     : (nrhs == 1 ? spk::k_bwd_u12<T, 1> : spk::k_bwd_u12<T, 4>);
+            CU(h, launch_chained(lines, P.bwdu_small.tiles, 256, 0, st, fac, y, (const T*)x, n, nrhs, S,
                                  launch_of(PL, P.bwdu_small)));
         }
         if (P.front_big.tiles > 0) {
             LaunchScope ls(h, SPK_K_BWD, P.front_big.flops * nrhs, P.front_big.words * sizeof(T));
-            launch_front_solve<T, false>(h, P.front_big.tiles, st, fac, inv, y, x, nrhs, S, launch_of(PL, P.front_big));
+            launch_front_solve<T, false, TRANS>(h, P.front_big.tiles, st, fac, inv, y, x, nrhs, S, launch_of(PL, P.front_big));
         }
         for (size_t c = P.chunks.size(); c-- > 0;) {   // chunked root fronts, chunks in reverse
             const LevelPlan::SolveChunk& ch = P.chunks[c];
             {
                 LaunchScope ls(h, SPK_K_BWD, ch.rec.flops * nrhs, ch.rec.words * sizeof(T));
-                launch_front_solve<T, false>(h, 1, st, fac, inv, y, x, nrhs, S, launch_of(PL, ch.rec));
+                launch_front_solve<T, false, TRANS>(h, 1, st, fac, inv, y, x, nrhs, S, launch_of(PL, ch.rec));
             }
             if (c > 0 && P.chunks[c - 1].front == ch.front) {   // rows above the chunk
                 const HFront& F = h->fronts[ch.front];
                 const int r0 = 0, r1 = ch.lo;
                 LaunchScope ls(h, SPK_K_BWD, 2.0 * (r1 - r0) * (ch.hi - ch.lo) * nrhs,
                                (double)(r1 - r0) * (ch.hi - ch.lo) * sizeof(T));
-                launch_front_gemv<T>(h, F, st, fac, y, x, nrhs, r0, r1, ch.lo, ch.hi);
+                launch_front_gemv<T, TRANS>(h, F, st, fac, y, x, nrhs, r0, r1, ch.lo, ch.hi);
             }
         }
         for (size_t t = 0; t < P.bwd_small.size(); ++t)
             if (P.bwd_small[t].tiles > 0) {
                 LaunchScope ls(h, SPK_K_BWD, P.bwd_small[t].flops * nrhs, P.bwd_small[t].words * sizeof(T));
-                CU(h, launch_chained(spk::k_bwd<T>, P.bwd_small[t].tiles, spk::TS, 0, st, fac, inv, y, x, n,
+                CU(h, launch_chained(TRANS ? spk::k_tbwd<T> : spk::k_bwd<T>, P.bwd_small[t].tiles, spk::TS, 0, st, fac, inv, y, x, n,
                                      nrhs, S, launch_of(PL, P.bwd_small[t]), (int)t));
             }
     }
@@ -1751,42 +1755,10 @@ static int solve_bwd_levels(spk_handle* h, int nrhs, cudaStream_t st) {
 // Solve in place on the permuted work vectors: wb (rhs, consumed) -> wx.
 template <typename T>
 static int run_solve_permuted(spk_handle* h, int nrhs, bool transpose) {
-    const T* fac = storage<T>(h).d;
-    const T* inv = storage<T>(h).inv2;
-    const Plan& PL = h->plan[plan_index<T>(h)];
-    const spk::Sched& S = PL.sched;
-    T* b = (T*)h->d_wb;
-    T* y = (T*)h->d_wy;
-    T* x = (T*)h->d_wx;
-    const int n = (int)h->n;
-    if (transpose) {   // A^T: U^T pass in block order, then L^T pass top-down with blocks reversed
-        for (const LevelPlan& P : PL.levels)
-            for (size_t t = 0; t < P.fwd.size(); ++t)
-                if (P.fwd[t].tiles > 0) {
-                    LaunchScope ls(h, SPK_K_FWD, P.fwd[t].flops * nrhs, P.fwd[t].words * sizeof(T));
-                    CU(h, launch_chained(spk::k_tfwd<T>, P.fwd[t].tiles, spk::TS, 0, h->stream, fac, inv, b, y, n, nrhs, S,
-                                         launch_of(PL, P.fwd[t]), (int)t));
-                }
-        for (size_t l = PL.levels.size(); l-- > 0;) {
-            const LevelPlan& P = PL.levels[l];
-            if (P.bwdu.tiles > 0) {
-                LaunchScope ls(h, SPK_K_BWD, P.bwdu.flops * nrhs, P.bwdu.words * sizeof(T));
-                CU(h, launch_chained(nrhs == 1 ? spk::k_tbwd_l21<T, 1> : spk::k_tbwd_l21<T, 4>, P.bwdu.tiles, 256, 0, h->stream, fac, y, x, n, nrhs, S,
-                                     launch_of(PL, P.bwdu)));
-            }
-            for (size_t t = 0; t < P.bwd.size(); ++t)
-                if (P.bwd[t].tiles > 0) {
-                    LaunchScope ls(h, SPK_K_BWD, P.bwd[t].flops * nrhs, P.bwd[t].words * sizeof(T));
-                    CU(h, launch_chained(spk::k_tbwd<T>, P.bwd[t].tiles, spk::TS, 0, h->stream, fac, inv, y, x, n, nrhs, S,
-                                         launch_of(PL, P.bwd[t]), (int)t));
-                }
-        }
-        CU(h, cudaGetLastError());
-        return SPK_OK;
-    }
-    int rc = solve_fwd_levels<T>(h, nrhs, 0, PL.levels.size(), h->stream);
+    const size_t nl = h->plan[plan_index<T>(h)].levels.size();
+    const int rc = transpose ? solve_fwd_levels<T, true>(h, nrhs, 0, nl, h->stream) : solve_fwd_levels<T, false>(h, nrhs, 0, nl, h->stream);
     if (rc) return rc;
-    return solve_bwd_levels<T>(h, nrhs, h->stream);
+    return transpose ? solve_bwd_levels<T, true>(h, nrhs, h->stream) : solve_bwd_levels<T, false>(h, nrhs, h->stream);
 }
 
 // x(:, 0:nrhs) (=|+=) A^{-1} rhs(:, 0:nrhs) (A^{-T} with `transpose`), both
@@ -2756,8 +2728,8 @@ static int factor_refine_first(spk_handle* h, int nrhs, double* dx, i64 ldx, int
             spk::k_permute<double, T><<<(int)((tot + 255) / 256), 256, 0, h->stream>>>(
                 h->d_rhs, h->n, (T*)h->d_wb, (int)h->n, h->d_rperm, (int)h->n, nrhs);
         }
-        int r = solve_fwd_levels<T>(h, nrhs, split, PL.levels.size(), h->stream);
-        return r ? r : solve_bwd_levels<T>(h, nrhs, h->stream);
+        int r = solve_fwd_levels<T, false>(h, nrhs, split, PL.levels.size(), h->stream);
+        return r ? r : solve_bwd_levels<T, false>(h, nrhs, h->stream);
     });
     if (rc) return rc;
     const ll tot = (ll)h->n * nrhs;

@@ -3201,6 +3201,41 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc_update(float* fac, const u
     if (warp == 1) umma::tmem_dealloc(tmem, G::TMEM_COLS);
 }
 
+// Warp reduce-scatter: N (a power of 2, at most 32) values per lane, summed
+// over the 32 lanes; each step keeps the half of the values picked by a
+// lane bit and adds the partner's copy of it, and once one value is left
+// the remaining lane bits are summed by a butterfly (N/2 + N/4 + ... + the
+// rest shuffles instead of 5 N).  Lane l ends with the sum of value
+// l * N / 32.
+template <int N, int OFF, typename T>
+__device__ __forceinline__ void rs_halve(T* v, int lane) {
+    const bool hi = (lane & OFF) != 0;
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) {
+        const T keep = hi ? v[i + N / 2] : v[i];
+        const T send = hi ? v[i] : v[i + N / 2];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, OFF);
+    }
+}
+template <int N, int OFF, typename T>
+__device__ __forceinline__ void rs_rec(T* v, int lane) {
+    if constexpr (OFF > 0) {
+        if constexpr (N > 1) {
+            rs_halve<N, OFF>(v, lane);
+            rs_rec<N / 2, OFF / 2>(v, lane);
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], OFF);
+            rs_rec<1, OFF / 2>(v, lane);
+        }
+    }
+}
+template <int N, typename T>
+__device__ __forceinline__ T warp_reduce_scatter(T (&v)[N]) {
+    static_assert(N >= 1 && N <= 32 && (N & (N - 1)) == 0, "a power of 2, at most 32 values");
+    rs_rec<N, 16>(v, threadIdx.x & 31);
+    return v[0];
+}
+
 // ---------------------------------------------------------------------------
 // Triangular solves.  Right-hand sides are column-major n x nrhs (ld = n),
 // nrhs <= 16 per launch.
@@ -3494,25 +3529,26 @@ __device__ __forceinline__ void rg_get(const T* p, T (&v)[RG]) {
 template <typename T, int RG>
 struct FcSmem {
     static constexpr int BM = BlockMax<T>::value, CS = FC_THREADS / BM;
+    static constexpr int LDT = BM + 1;   // transposed form: rows of the prefetched blocks, an odd stride
     static constexpr size_t ypub = 0, ycur = ypub + BM * RG, own = ycur + BM * RG,
                             part = own + (size_t)FC_OWN * BM * RG, preA = part + (size_t)CS * BM * RG,
-                            preM = preA + (size_t)BM * BM, total = preM + (size_t)BM * BM;   // in T's
+                            preM = preA + (size_t)BM * LDT, total = preM + (size_t)BM * LDT;   // in T's
     static constexpr size_t bytes = total * sizeof(T);
 };
 
 // v[i * RG + r] -= sum_j A(i, j) w[j * RG + r], i < nrow, j < ncol,
-// with A(i, j) = a[j * lda + i] (a block of the factor in global memory, or
+// with A(i, j) = a[i * si + j * sj] (a block of the factor in global memory, or
 // its prefetched copy in shared memory).  Thread (i, cs) takes columns
 // cs, cs + CS, ...; all its loads are issued before the first use.
 template <typename T, int RG>
-__device__ __forceinline__ void fc_tile_update(const T* a, ll lda, int nrow, int ncol, T* v, const T* w, T* part) {
+__device__ __forceinline__ void fc_tile_update(const T* a, ll si, ll sj, int nrow, int ncol, T* v, const T* w, T* part) {
     constexpr int BM = BlockMax<T>::value, CS = FC_THREADS / BM, NJ = BM / CS;
     const int i = threadIdx.x % BM, cs = threadIdx.x / BM;
     T av[NJ];
 #pragma unroll
     for (int q = 0; q < NJ; ++q) {
         const int j = cs + q * CS;
-        av[q] = (i < nrow && j < ncol) ? a[(ll)j * lda + i] : T(0);
+        av[q] = (i < nrow && j < ncol) ? a[i * si + j * sj] : T(0);
     }
     T acc[RG];
 #pragma unroll
@@ -3536,10 +3572,45 @@ __device__ __forceinline__ void fc_tile_update(const T* a, ll lda, int nrow, int
     __syncthreads();
 }
 
+// The same for the transposed solves' blocks in global memory, A(i, j) =
+// a[i * ld + j]: a warp takes rows i, its lanes run along j, so that the loads
+// are contiguous; the sums over the lanes by a warp reduce-scatter.
+template <typename T, int RG>
+__device__ __forceinline__ void fc_tile_update_t(const T* a, ll ld, int nrow, int ncol, T* v, const T* w) {
+    constexpr int BM = BlockMax<T>::value, NW = FC_THREADS / 32, NI = BM / NW, NJ = BM / 32;
+    const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    T av[NI][NJ];
+#pragma unroll
+    for (int s = 0; s < NI; ++s)
+#pragma unroll
+        for (int q = 0; q < NJ; ++q) {
+            const int i = wp + s * NW, j = lane + 32 * q;
+            av[s][q] = (i < nrow && j < ncol) ? a[i * ld + j] : T(0);
+        }
+    T acc[NI * RG];
+#pragma unroll
+    for (int e = 0; e < NI * RG; ++e) acc[e] = T(0);
+#pragma unroll
+    for (int q = 0; q < NJ; ++q) {
+        T wv[RG];
+        rg_get<RG>(w + (lane + 32 * q) * RG, wv);
+#pragma unroll
+        for (int s = 0; s < NI; ++s)
+#pragma unroll
+            for (int r = 0; r < RG; ++r) acc[s * RG + r] += av[s][q] * wv[r];
+    }
+    const T sum = warp_reduce_scatter<NI * RG>(acc);   // lane l: value l * NI * RG / 32
+    constexpr int per = 32 / (NI * RG);
+    const int e = lane / per, i = wp + (e / RG) * NW;
+    if (lane % per == 0 && i < nrow) v[i * RG + e % RG] -= sum;
+    __syncthreads();
+}
+
 // out[j * RG + r] = sum_k op(j, k) v[k * RG + r] for the block's solve
-// operator (forward Minv, backward Uinv; op(j, k) at m[k * BM + j]).
-template <typename T, bool FWD, int RG>
-__device__ __forceinline__ void fc_block_solve(const T* m, int bw, const T* v, T* out, T* part, int nr) {
+// operator (forward Minv, backward Uinv, TRI: zero for k < j; transposed:
+// Uinv^T, Minv^T); op(j, k) at m[j * sj + k * sk].
+template <typename T, bool TRI, int RG>
+__device__ __forceinline__ void fc_block_solve(const T* m, int sj, int sk, int bw, const T* v, T* out, T* part, int nr) {
     constexpr int BM = BlockMax<T>::value, CS = FC_THREADS / BM;
     const int j = threadIdx.x % BM, cs = threadIdx.x / BM;
     T acc[RG];
@@ -3547,8 +3618,8 @@ __device__ __forceinline__ void fc_block_solve(const T* m, int bw, const T* v, T
     for (int r = 0; r < RG; ++r) acc[r] = T(0);
     if (j < bw) {
 #pragma unroll 4
-        for (int k = (FWD ? 0 : j) + cs; k < bw; k += CS) {
-            const T mv = m[k * BM + j];
+        for (int k = (TRI ? j : 0) + cs; k < bw; k += CS) {
+            const T mv = m[j * sj + k * sk];
             T vv[RG];
             rg_get<RG>(v + k * RG, vv);
 #pragma unroll
@@ -3569,7 +3640,7 @@ __device__ __forceinline__ void fc_block_solve(const T* m, int bw, const T* v, T
     __syncthreads();
 }
 
-template <typename T, bool FWD, int NC, int RG>
+template <typename T, bool FWD, int NC, int RG, bool TRANS = false>
 __global__ void __cluster_dims__(NC, 1, 1) __launch_bounds__(FC_THREADS, 1)
     k_front_solve(const T* fac, const T* inv2, T* in, T* out, int n, int nrhs, Sched S, Launch L) {
     constexpr int FC = NC;   // CTAs of the cluster
@@ -3589,25 +3660,33 @@ __global__ void __cluster_dims__(NC, 1, 1) __launch_bounds__(FC_THREADS, 1)
     const DFront F = S.fronts[L.front_ids[blockIdx.x / FC]];
     const int nb = F.nblocks, tid = threadIdx.x;
     auto blk_of = [&](int step) { return F.block0 + (FWD ? step : nb - 1 - step); };
-    auto a_of = [&](int bs, int bt) { return fac + F.loff + (ll)S.blk_c0[bt] * F.ld + S.blk_c0[bs]; };
+    // A(i, j) of the update of block bs by block bt: L or U (row i of bs, column
+    // j of bt) at a[j * ld + i]; transposed, (row j of bt, column i of bs) at a[i * ld + j]
+    auto a_of = [&](int bs, int bt) {
+        return TRANS ? fac + F.loff + (ll)S.blk_c0[bs] * F.ld + S.blk_c0[bt] : fac + F.loff + (ll)S.blk_c0[bt] * F.ld + S.blk_c0[bs];
+    };
+    // strides of the prefetched copies: element (i, j) at i * PI + j * PJ
+    constexpr int PI = TRANS ? SM::LDT : 1, PJ = TRANS ? 1 : BM;
     // The factor data of owned step st (its operator, and the block linking
     // it to step st - 1) is copied asynchronously while other steps run.
     auto prefetch = [&](int st) {
         if (st >= nb) return;
         const int bs = blk_of(st), bw = S.blk_c1[bs] - S.blk_c0[bs];
-        const T* Mi = inv2 + S.blk_inv2[bs] + (FWD ? 0 : (ll)bw * bw);
+        // forward Minv, backward Uinv; transposed, Uinv^T and Minv^T: the
+        // contiguous index is k there, the row of the untransposed operator
+        const T* Mi = inv2 + S.blk_inv2[bs] + (FWD != TRANS ? 0 : (ll)bw * bw);
         for (int e = tid; e < BM * BM; e += FC_THREADS) {
-            const int j = e % BM, k = e / BM;
-            const bool v = j < bw && k < bw;
-            cp_elem(&preM[e], v ? Mi + (ll)k * bw + j : Mi, v);
+            const int x = e % BM, y = e / BM;
+            const bool v = x < bw && y < bw;
+            cp_elem(&preM[TRANS ? y * PI + x : y * PJ + x], v ? Mi + (ll)y * bw + x : Mi, v);
         }
         if (st > 0) {
             const int bt = blk_of(st - 1), ncol = S.blk_c1[bt] - S.blk_c0[bt];
             const T* a = a_of(bs, bt);
             for (int e = tid; e < BM * BM; e += FC_THREADS) {
-                const int i = e % BM, j = e / BM;
-                const bool v = i < bw && j < ncol;
-                cp_elem(&preA[e], v ? a + (ll)j * F.ld + i : a, v);
+                const int x = e % BM, y = e / BM;   // x contiguous: row i, transposed column j
+                const bool v = x < (TRANS ? ncol : bw) && y < (TRANS ? bw : ncol);
+                cp_elem(&preA[TRANS ? y * PI + x : y * PJ + x], v ? a + (ll)y * F.ld + x : a, v);
             }
         }
     };
@@ -3625,7 +3704,7 @@ __global__ void __cluster_dims__(NC, 1, 1) __launch_bounds__(FC_THREADS, 1)
         __syncthreads();
         auto solve_step = [&](int st) {   // owner: publish the solution of step st
             const int blk = blk_of(st), bw = S.blk_c1[blk] - S.blk_c0[blk];
-            fc_block_solve<T, FWD, RG>(preM, bw, own + (size_t)(st / FC) * BM * RG, ypub, part, nr);
+            fc_block_solve<T, !FWD && !TRANS, RG>(preM, PI, PJ, bw, own + (size_t)(st / FC) * BM * RG, ypub, part, nr);
         };
         auto finish_step = [&](int st) {   // owner, after the barrier arrival: output and next prefetch
             const int blk = blk_of(st), c0 = S.blk_c0[blk], bw = S.blk_c1[blk] - c0;
@@ -3653,7 +3732,7 @@ __global__ void __cluster_dims__(NC, 1, 1) __launch_bounds__(FC_THREADS, 1)
                 cp_wait_all();
                 __syncthreads();
                 const int bs = blk_of(t + 1);
-                fc_tile_update<T, RG>(preA, BM, S.blk_c1[bs] - S.blk_c0[bs], ncol,
+                fc_tile_update<T, RG>(preA, PI, PJ, S.blk_c1[bs] - S.blk_c0[bs], ncol,
                                   own + (size_t)((t + 1) / FC) * BM * RG, ycur, part);
                 solve_step(t + 1);
             }
@@ -3662,8 +3741,10 @@ __global__ void __cluster_dims__(NC, 1, 1) __launch_bounds__(FC_THREADS, 1)
             for (int st = rank, o = 0; st < nb; st += FC, ++o)
                 if (st > t && !(next && st == t + 1)) {
                     const int bs = blk_of(st);
-                    fc_tile_update<T, RG>(a_of(bs, bt), F.ld, S.blk_c1[bs] - S.blk_c0[bs], ncol,
-                                      own + (size_t)o * BM * RG, ycur, part);
+                    T* v = own + (size_t)o * BM * RG;
+                    const int nrow = S.blk_c1[bs] - S.blk_c0[bs];
+                    if constexpr (TRANS) fc_tile_update_t<T, RG>(a_of(bs, bt), F.ld, nrow, ncol, v, ycur);
+                    else fc_tile_update<T, RG>(a_of(bs, bt), 1, F.ld, nrow, ncol, v, ycur, part);
                 }
             __syncthreads();
         }
@@ -3689,49 +3770,22 @@ __global__ void __cluster_dims__(NC, 1, 1) __launch_bounds__(FC_THREADS, 1)
 // k_fwd / k_bwd_u12 / k_bwd.
 constexpr int LEAF_M = 128;
 
-// Warp reduce-scatter: N (a power of 2, at most 32) values per lane, summed
-// over the 32 lanes; each step keeps the half of the values picked by a
-// lane bit and adds the partner's copy of it, and once one value is left
-// the remaining lane bits are summed by a butterfly (N/2 + N/4 + ... + the
-// rest shuffles instead of 5 N).  Lane l ends with the sum of value
-// l * N / 32.
-template <int N, int OFF, typename T>
-__device__ __forceinline__ void rs_halve(T* v, int lane) {
-    const bool hi = (lane & OFF) != 0;
-#pragma unroll
-    for (int i = 0; i < N / 2; ++i) {
-        const T keep = hi ? v[i + N / 2] : v[i];
-        const T send = hi ? v[i] : v[i + N / 2];
-        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, OFF);
-    }
-}
-template <int N, int OFF, typename T>
-__device__ __forceinline__ void rs_rec(T* v, int lane) {
-    if constexpr (OFF > 0) {
-        if constexpr (N > 1) {
-            rs_halve<N, OFF>(v, lane);
-            rs_rec<N / 2, OFF / 2>(v, lane);
-        } else {
-            v[0] += __shfl_xor_sync(0xffffffffu, v[0], OFF);
-            rs_rec<1, OFF / 2>(v, lane);
-        }
-    }
-}
-template <int N, typename T>
-__device__ __forceinline__ T warp_reduce_scatter(T (&v)[N]) {
-    static_assert(N >= 1 && N <= 32 && (N & (N - 1)) == 0, "a power of 2, at most 32 values");
-    rs_rec<N, 16>(v, threadIdx.x & 31);
-    return v[0];
-}
-
-// RG: right-hand sides per pass (1 for a single one, else 4).
-template <typename T, bool FWD, int W, int RG>
+// RG: right-hand sides per pass (1 for a single one, else 4).  TRANS, the
+// transposed solves: forward Uinv^T and U12^T in the places of Minv and L21,
+// backward L21^T and Minv^T in those of U12 and Uinv; only the addresses
+// differ (L21 column k and U12 row k are both contiguous).
+template <typename T, bool FWD, int W, int RG, bool TRANS>
 __device__ __forceinline__ void solve_leaf_front(const T* fac, const T* inv2, T* in, T* out, const T* xs, int n, int nrhs,
                                                  const Sched& S, const DFront& F) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int blk = F.block0, bw = F.nf;
-    const T* Mi = inv2 + S.blk_inv2[blk] + (FWD ? 0 : (ll)bw * bw);
+    const T* Mi = inv2 + S.blk_inv2[blk] + (FWD != TRANS ? 0 : (ll)bw * bw);
+    // entry i of line k of the front's off-diagonal part
+    auto pan = [&](int k, int i) {
+        if constexpr (FWD != TRANS) return fac[F.loff + (ll)k * F.ld + F.nf + i];
+        else return fac[F.uoff + (ll)k * F.m + i];
+    };
     const int* rows = S.rows + F.rows_off;
     griddep_wait();
     for (int r0 = 0; r0 < nrhs; r0 += RG) {
@@ -3741,17 +3795,17 @@ __device__ __forceinline__ void solve_leaf_front(const T* fac, const T* inv2, T*
         // rows), so that a front waits for fewer round trips; wider ones
         // keep them where they are used (registers)
         constexpr bool EARLY = W <= 8;
-        T mv[W];   // op(lane, k), op(j, k) at Mi[k * bw + j]
+        T mv[W];   // op(lane, k), op(j, k) at Mi[k * bw + j] (TRANS: Mi[j * bw + k])
         auto load_mv = [&] {
 #pragma unroll
             for (int k = 0; k < W; ++k)
-                mv[k] = (k < bw && lane < bw && (FWD || k >= lane)) ? Mi[(ll)k * bw + lane] : T(0);
+                mv[k] = (k < bw && lane < bw && (FWD || TRANS || k >= lane)) ? Mi[TRANS ? (ll)lane * bw + k : (ll)k * bw + lane] : T(0);
         };
         if constexpr (EARLY) load_mv();
         T lv0[FWD && EARLY ? W : 1];
         if constexpr (FWD && EARLY) {
 #pragma unroll
-            for (int k = 0; k < W; ++k) lv0[k] = (k < bw && lane < F.m) ? fac[F.loff + (ll)k * F.ld + F.nf + lane] : T(0);
+            for (int k = 0; k < W; ++k) lv0[k] = (k < bw && lane < F.m) ? pan(k, lane) : T(0);
         }
         T v[RG];
 #pragma unroll
@@ -3772,7 +3826,7 @@ __device__ __forceinline__ void solve_leaf_front(const T* fac, const T* inv2, T*
                     const int g = ok ? rows[il] : 0;
                     T uv[W], xv[RG];
 #pragma unroll
-                    for (int j = 0; j < W; ++j) uv[j] = (ok && j < bw) ? fac[F.uoff + (ll)j * F.m + il] : T(0);
+                    for (int j = 0; j < W; ++j) uv[j] = (ok && j < bw) ? pan(j, il) : T(0);
 #pragma unroll
                     for (int r = 0; r < RG; ++r) xv[r] = (ok && r < nr) ? xs[(ll)(r0 + r) * n + g] : T(0);
 #pragma unroll
@@ -3793,7 +3847,7 @@ __device__ __forceinline__ void solve_leaf_front(const T* fac, const T* inv2, T*
                     if (lane < bw) acc[r] = vr;
                 }
             } else {
-                const T* u = fac + F.uoff + (ll)lane * F.m;
+                const T* u = fac + (FWD != TRANS ? F.loff + (ll)lane * F.ld + F.nf : F.uoff + (ll)lane * F.m);
                 for (int i0 = 0; i0 < F.m; i0 += 32) {
                     // lane l: x at row R_F[i0 + l]; lane j: U12(j, i0 ..)
                     const int il = i0 + lane;
@@ -3840,7 +3894,7 @@ __device__ __forceinline__ void solve_leaf_front(const T* fac, const T* inv2, T*
                     if constexpr (EARLY) {
                         if (i0 == 0) { lv[k] = lv0[k]; continue; }
                     }
-                    lv[k] = (k < bw && i < F.m) ? fac[F.loff + (ll)k * F.ld + F.nf + i] : T(0);
+                    lv[k] = (k < bw && i < F.m) ? pan(k, i) : T(0);
                 }
                 T acc[RG];
 #pragma unroll
@@ -3861,18 +3915,18 @@ __device__ __forceinline__ void solve_leaf_front(const T* fac, const T* inv2, T*
     }
 }
 
-template <typename T, bool FWD, int W, int RG>
+template <typename T, bool FWD, int W, int RG, bool TRANS = false>
 __global__ void __launch_bounds__(256) k_solve_leaf(const T* fac, const T* inv2, T* in, T* out, const T* xs, int n,
                                                      int nrhs, Sched S, Launch L) {
     griddep_launch();
     const int idx = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (idx >= L.count) return;   // whole warp
     const DFront F = S.fronts[L.front_ids[idx]];
-    solve_leaf_front<T, FWD, W, RG>(fac, inv2, in, out, xs, n, nrhs, S, F);
+    solve_leaf_front<T, FWD, W, RG, TRANS>(fac, inv2, in, out, xs, n, nrhs, S, F);
 }
 
 // Every width class in one launch, for levels with few of these fronts.
-template <typename T, bool FWD, int RG>
+template <typename T, bool FWD, int RG, bool TRANS = false>
 __global__ void __launch_bounds__(256) k_solve_leaf_set(const T* fac, const T* inv2, T* in, T* out, const T* xs, int n,
                                                          int nrhs, Sched S, LeafSet L) {
     griddep_launch();
@@ -3881,10 +3935,10 @@ __global__ void __launch_bounds__(256) k_solve_leaf_set(const T* fac, const T* i
     if (fid < 0) return;   // whole warp
     const DFront F = S.fronts[fid];
     switch (list % LF_CLASSES) {
-    case 0: solve_leaf_front<T, FWD, 4, RG>(fac, inv2, in, out, xs, n, nrhs, S, F); break;
-    case 1: solve_leaf_front<T, FWD, 8, RG>(fac, inv2, in, out, xs, n, nrhs, S, F); break;
-    case 2: solve_leaf_front<T, FWD, 16, RG>(fac, inv2, in, out, xs, n, nrhs, S, F); break;
-    default: solve_leaf_front<T, FWD, 32, RG>(fac, inv2, in, out, xs, n, nrhs, S, F); break;
+    case 0: solve_leaf_front<T, FWD, 4, RG, TRANS>(fac, inv2, in, out, xs, n, nrhs, S, F); break;
+    case 1: solve_leaf_front<T, FWD, 8, RG, TRANS>(fac, inv2, in, out, xs, n, nrhs, S, F); break;
+    case 2: solve_leaf_front<T, FWD, 16, RG, TRANS>(fac, inv2, in, out, xs, n, nrhs, S, F); break;
+    default: solve_leaf_front<T, FWD, 32, RG, TRANS>(fac, inv2, in, out, xs, n, nrhs, S, F); break;
     }
 }
 
@@ -3893,7 +3947,8 @@ __global__ void __launch_bounds__(256) k_solve_leaf_set(const T* fac, const T* i
 // (L21 column k contiguous in Lf), y_F of the tile's columns in shared
 // memory, partial sums added to b with atomics.
 constexpr int L21_ROWS = 256, L21_COLS = 64;   // 64 columns: twice the CTAs and loads in flight of 128
-template <typename T, int RG>
+// TRANS: U12^T in the place of L21 (the transposed solves).
+template <typename T, int RG, bool TRANS = false>
 __global__ void __launch_bounds__(256) k_fwd_l21(const T* fac, T* b, const T* y, int n, int nrhs, Sched S, Launch L) {
     __shared__ T sy[L21_COLS * RG];
     griddep_launch();
@@ -3904,7 +3959,8 @@ __global__ void __launch_bounds__(256) k_fwd_l21(const T* fac, T* b, const T* y,
     const int nk = min(L21_COLS, F.nf - k0), i = i0 + threadIdx.x;
     const bool ok = i < F.m;
     const int grow = ok ? S.rows[F.rows_off + i] : 0;
-    const T* a = fac + F.loff + (ll)k0 * F.ld + F.nf + (ok ? i : 0);
+    const ll sk = TRANS ? F.m : F.ld;
+    const T* a = fac + (TRANS ? F.uoff : F.loff + F.nf) + k0 * sk + (ok ? i : 0);
     griddep_wait();
     for (int r0 = 0; r0 < nrhs; r0 += RG) {
         const int nr = min(RG, nrhs - r0);
@@ -3920,7 +3976,7 @@ __global__ void __launch_bounds__(256) k_fwd_l21(const T* fac, T* b, const T* y,
         if (ok) {
 #pragma unroll 16
             for (int k = 0; k < nk; ++k) {
-                const T av = a[(ll)k * F.ld];
+                const T av = a[k * sk];
 #pragma unroll
                 for (int r = 0; r < RG; ++r) acc[r] += av * sy[r * L21_COLS + k];
             }
@@ -3973,6 +4029,37 @@ __global__ void __launch_bounds__(256) k_front_gemv(const T* fac, T* out, const 
     }
 }
 
+// The transposed product: out[f + r] -= sum_c A(c, r) in[f + c] (line r is
+// contiguous).  Tiles of GT_ROWS lines, a warp per four of them, lanes along
+// the columns; a line's sum is one warp's, so no atomics.
+constexpr int GT_ROWS = 32;
+template <typename T, int RG>
+__global__ void __launch_bounds__(256) k_front_gemv_t(const T* fac, T* out, const T* in, int n, int nrhs, ll loff, int ld, int f,
+                                                      int r0, int r1, int c0, int c1) {
+    const int lane = threadIdx.x & 31, i0 = r0 + (int)blockIdx.x * GT_ROWS + (int)(threadIdx.x >> 5) * 4;
+    for (int q0 = 0; q0 < nrhs; q0 += RG) {
+        T acc[4 * RG];
+#pragma unroll
+        for (int e = 0; e < 4 * RG; ++e) acc[e] = T(0);
+#pragma unroll 4
+        for (int c = c0 + lane; c < c1; c += 32) {
+            T av[4], x[RG];
+#pragma unroll
+            for (int s = 0; s < 4; ++s) av[s] = i0 + s < r1 ? fac[loff + (ll)(i0 + s) * ld + c] : T(0);
+#pragma unroll
+            for (int r = 0; r < RG; ++r) x[r] = q0 + r < nrhs ? in[(ll)(q0 + r) * n + f + c] : T(0);
+#pragma unroll
+            for (int s = 0; s < 4; ++s)
+#pragma unroll
+                for (int r = 0; r < RG; ++r) acc[s * RG + r] += av[s] * x[r];
+        }
+        const T sum = warp_reduce_scatter<4 * RG>(acc);   // lane l: value l * 4 RG / 32
+        constexpr int per = 32 / (4 * RG);
+        const int e = lane / per, i = i0 + e / RG, r = q0 + e % RG;
+        if (lane % per == 0 && i < r1 && r < nrhs) out[(ll)r * n + f + i] -= sum;
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Transposed solves, A^T x = b with the same factors (no reference kernel:
 // the reference's `transposetriangularsolve` is commented out,
@@ -3986,7 +4073,9 @@ __global__ void __launch_bounds__(256) k_front_gemv(const T* fac, T* out, const 
 //   pass 2, fronts top-down: the front's columns get L21^T x[R_F]
 //     subtracted, then blocks in reverse: x_B = Minv_B^T z_B, and the
 //     front's earlier columns get L_B,earlier^T x_B subtracted.
-// The tiles and launch lists are those of k_fwd / k_bwd_u12 / k_bwd.
+// The launch lists are those of the plain solves: small fronts and fronts of
+// many blocks by k_solve_leaf and k_front_solve in their TRANS forms, the
+// others by the kernels below, with the tiles of k_fwd / k_bwd_u12 / k_bwd.
 // ---------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(TS) k_tfwd(const T* fac, const T* inv2, T* b, T* z, int n, int nrhs, Sched S,
