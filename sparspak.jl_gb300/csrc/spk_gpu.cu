@@ -63,6 +63,7 @@ struct LevelPlan {
     // bpanel split in two parts: the near tiles (the first 128 rows below the
     // block and columns right of it, which tile 0 reads) and the far ones
     std::vector<LaunchRec> bpanel_near, bpanel_far;
+    std::vector<LaunchRec> oz_pack;   // FP64: slices of the step's panels (k_oz_pack)
     std::vector<char> blu_pc;   // every piece of the step's blocks is at most 32 columns (k_block_lu_pc)
     // Solves: fronts with many blocks by one cluster launch each direction
     // (front_big, one tile per front), the others by block steps
@@ -90,6 +91,10 @@ struct LevelPlan {
 // tc_schur_m rows, or more than one block with at least tc_trail_rows rows
 // below the first (spk_handle; defaults below, SPK_OPT_TC_* to change).
 constexpr int TC_SCHUR_M = 96, TC_TRAIL_ROWS = 128;
+// FP64 fronts whose rank updates go to the tensor cores as integer slices
+// (k_oz_update): at least OZ_MIN rows below the front, or below its first
+// block when it has several.
+constexpr int OZ_MIN = 128;
 // Polls of a bounded device wait (the leaf queue's dependency waits) before
 // it gives up and records a timeout.
 constexpr long long WAIT_BUDGET = 1 << 20;
@@ -185,6 +190,7 @@ struct spk_handle {
     ll* d_run_rel = nullptr;
     int* d_ipiv = nullptr;
     int* d_bmap = nullptr;     // row sources of each block's interchanges (k_block_lu -> panels)
+    int* d_rexp = nullptr;     // FP64: exponent field of each U row's largest panel entry (panels -> k_oz_pack)
     int* d_info = nullptr;
 
     // pattern and values
@@ -638,7 +644,7 @@ static void add_launch(Plan* h, LaunchRec& rec, const std::vector<int>& ids, con
 
 // Lines per panel tile: the 128-wide FP32 form (a launch with a block wider
 // than 64 columns) takes spk::PT_LINES, the others 64.
-static int panel_lines(bool fp32, bool wide) { return fp32 && wide ? spk::PT_LINES : 64; }
+static int panel_lines(bool fp32, bool wide) { return !fp32 ? spk::PD_LINES : wide ? spk::PT_LINES : 64; }
 
 // Group each front's pieces into blocks of at most `bmax` columns and lay
 // out the launches of every level.
@@ -674,17 +680,19 @@ static void build_plan(const spk_handle* h, Plan& P, int bmax, bool tc, bool sym
     }
     P.blk_lpack.assign(P.blk_c0.size(), -1);
     P.blk_upack.assign(P.blk_c0.size(), -1);
-    if (tc) {
+    {
         const ll chunk = spk::umma::PCHUNK;
         for (int i = 0; i < nfr; ++i) {
             const HFront& F = h->fronts[i];
             const int b0 = P.block0[i], nb = P.nblocks[i];
-            const bool packed = F.m >= h->tc_schur_m || (nb > 1 && F.nf + F.m - P.blk_c1[b0] >= h->tc_trail_rows);
+            const bool packed = tc ? F.m >= h->tc_schur_m || (nb > 1 && F.nf + F.m - P.blk_c1[b0] >= h->tc_trail_rows)
+                                   : F.m >= OZ_MIN || (nb > 1 && F.nf + F.m - P.blk_c1[b0] >= OZ_MIN);
             if (!packed) continue;
             const int n2 = cdiv(F.m, spk::umma::TM);
             for (int b = b0; b < b0 + nb; ++b) {
                 const int n1 = cdiv(F.nf - P.blk_c1[b], spk::umma::TM);
-                const ll bytes = (ll)(n1 + n2) * cdiv(P.blk_c1[b] - P.blk_c0[b], spk::umma::KCH) * chunk;
+                const int nch = cdiv(P.blk_c1[b] - P.blk_c0[b], spk::umma::KCH);
+                const ll bytes = tc ? (ll)(n1 + n2) * nch * chunk : spk::oz_side_bytes(n1 + n2, nch);
                 P.blk_lpack[b] = P.pack_size;
                 P.blk_upack[b] = P.pack_size + bytes;
                 P.pack_size += 2 * bytes;
@@ -772,6 +780,7 @@ static void build_plan(const spk_handle* h, Plan& P, int bmax, bool tc, bool sym
         L.bpanel.resize(maxb);
         L.bpanel_near.resize(maxb);
         L.bpanel_far.resize(maxb);
+        L.oz_pack.resize(maxb);
         L.btrail.resize(maxb);
         L.btrail_tc0.resize(maxb);
         L.btrail_tc.resize(maxb);
@@ -864,11 +873,12 @@ static void build_plan(const spk_handle* h, Plan& P, int bmax, bool tc, bool sym
             for (int t = 0; t < P.nblocks[id]; ++t)
                 if (P.blk_c1[P.block0[id] + t] - P.blk_c0[P.block0[id] + t] > 64) wide[t] = 1;
         for (int t = 0; t < maxb; ++t) {
-            std::vector<int> tl(nid), tp(nid), tt(nid), ttc(nid), ttc0(nid), tf(nid), tb(nid);
+            std::vector<int> tl(nid), tp(nid), tt(nid), ttc(nid), ttc0(nid), tf(nid), tb(nid), toz(nid, 0);
             std::vector<double> fl(nid), wl(nid), fp(nid), wp(nid), ft(nid), wt(nid), ff(nid), wf(nid), fb(nid), wb(nid);
             for (size_t k = 0; k < nid; ++k) {
                 const HFront& F = h->fronts[ids[k]];
                 const int nb = P.nblocks[ids[k]];
+                toz[k] = 0;
                 if (t >= nb) { tl[k] = tp[k] = tt[k] = ttc[k] = ttc0[k] = tf[k] = tb[k] = 0; continue; }
                 const int blk = P.block0[ids[k]] + t;
                 const int c0 = P.blk_c0[blk], c1 = P.blk_c1[blk];
@@ -888,8 +898,11 @@ static void build_plan(const spk_handle* h, Plan& P, int bmax, bool tc, bool sym
                 ttc[k] = ttc0[k] = 0;
                 if (P.blk_lpack[blk] >= 0) {   // packed front: 128-tiles, row / column regions split at nf
                     const int n1 = cdiv(F.nf - c1, spk::umma::TM), n2 = cdiv(F.m, spk::umma::TM);
-                    const int all = sym ? spk::lower_tiles(n1 + n2, n1) : (n1 + n2) * n1 + n1 * n2;
-                    ttc0[k] = all > 0 ? 1 : 0;
+                    const int oc1 = cdiv(F.nf - c1, spk::OZ_N);
+                    const int all = !tc ? spk::oz_trail_tiles(n1, n2, oc1, cdiv(F.m, spk::OZ_N), sym)
+                                    : sym ? spk::lower_tiles(n1 + n2, n1) : (n1 + n2) * n1 + n1 * n2;
+                    toz[k] = tc ? 0 : 2 * (n1 + n2);
+                    ttc0[k] = !tc ? spk::oz_near(oc1) : all > 0 ? 1 : 0;
                     ttc[k] = all - ttc0[k];
                     tt[k] = 0;
                 }
@@ -945,6 +958,7 @@ static void build_plan(const spk_handle* h, Plan& P, int bmax, bool tc, bool sym
                 }
             L.blu[t].bw = L.bpanel[t].bw = bwl;
             add_launch(&P, L.btrail[t], ids, tt, ft, wt);
+            add_launch(&P, L.oz_pack[t], ids, toz, std::vector<double>(nid, 0.0), wp);
             {   // flops and words of the tensor-core update split by tiles
                 std::vector<double> f0(nid), w0(nid), f1(nid), w1(nid);
                 for (size_t k = 0; k < nid; ++k) {
@@ -970,7 +984,8 @@ static void build_plan(const spk_handle* h, Plan& P, int bmax, bool tc, bool sym
             tsch[k] = F.m > 0 && !leafF[k] ? (sym ? spk::lower_tiles(nts, nts) : nts * nts) : 0;
             tsch_tc[k] = 0;
             if (F.m > 0 && P.blk_lpack[P.block0[ids[k]]] >= 0) {
-                tsch_tc[k] = sym ? spk::lower_tiles_w(ntc, P.schur_nh) : ntc * cdiv(ntc, P.schur_nh);
+                tsch_tc[k] = !tc ? spk::oz_schur_tiles(ntc, cdiv(F.m, spk::OZ_N), sym)
+                             : sym ? spk::lower_tiles_w(ntc, P.schur_nh) : ntc * cdiv(ntc, P.schur_nh);
                 tsch[k] = 0;
             }
             tbu[k] = F.m > 0 ? cdiv(F.nf, spk::U12_ROWS) * cdiv(F.m, spk::U12_COLS) : 0;
@@ -988,7 +1003,7 @@ static void build_plan(const spk_handle* h, Plan& P, int bmax, bool tc, bool sym
             for (size_t k = 0; k < nid; ++k) {
                 tn[k] = tfar[k] = 0;
                 fn[k] = wn[k] = ffar[k] = wfar[k] = 0.0;
-                if (tsch_tc[k] <= 0) continue;
+                if (!tc || tsch_tc[k] <= 0) continue;
                 const int ntc = cdiv(h->fronts[ids[k]].m, spk::umma::TM), q = P.schur_q[ids[k]];
                 tn[k] = spk::schur_part_count(1, ntc, P.schur_nh, q, sym);
                 tfar[k] = spk::schur_part_count(2, ntc, P.schur_nh, q, sym);
@@ -1018,6 +1033,7 @@ static int upload_structure(spk_handle* h) {
     if ((rc = upload(h, &h->d_rel, h->rel))) return rc;
     CU(h, cudaMalloc((void**)&h->d_ipiv, sizeof(int) * std::max<i64>(h->n, 1)));
     CU(h, cudaMalloc((void**)&h->d_bmap, sizeof(int) * std::max<i64>(h->n, 1)));
+    CU(h, cudaMalloc((void**)&h->d_rexp, sizeof(int) * std::max<i64>(h->n, 1)));
     // first singular piece, tensor-core wait timeout, leaf-queue wait timeout
     CU(h, cudaMalloc((void**)&h->d_info, 3 * sizeof(int)));
     return SPK_OK;
@@ -1033,6 +1049,8 @@ template <typename T, int W>
 static int panel_threads() {
     return (std::is_same<T, float>::value && W == 128) ? 4 * spk::PT_LINES : 256;
 }
+template <int W>
+static constexpr size_t panel64_smem() { return sizeof(double) * W * (W + 1); }   // k_block_panel_f64
 template <typename T, int W>
 static size_t panel_smem() {
     return sweep_smem<T, W>(1) + ((std::is_same<T, float>::value && W == 128) ? (size_t)spk::PT_SMEM : 0);
@@ -1140,8 +1158,9 @@ static int ensure_plan(spk_handle* h) {
     S.blk_upack = P.d_blk_upack;
     S.sym = P.sym ? 1 : 0;
     constexpr int BM = spk::BlockMax<T>::value;
-    CU(h, cudaFuncSetAttribute(spk::k_block_panel<T, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)panel_smem<T, BM>()));
+    if constexpr (std::is_same<T, float>::value)
+        CU(h, cudaFuncSetAttribute(spk::k_block_panel<T, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)panel_smem<T, BM>()));
     CU(h, cudaFuncSetAttribute(spk::k_block_lu_pc<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)spk::PcLu<T>::smem));
     CU(h, cudaFuncSetAttribute(spk::k_block_inv<T, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1167,6 +1186,10 @@ static int ensure_plan(spk_handle* h) {
     if ((rc = prepare_front_solve<T, 1, false>(h)) || (rc = prepare_front_solve<T, 4, false>(h)) ||
         (rc = prepare_front_solve<T, 1, true>(h)) || (rc = prepare_front_solve<T, 4, true>(h)))
         return rc;
+    if (std::is_same<T, double>::value) {
+        CU(h, cudaFuncSetAttribute(spk::k_oz_update<spk::TC_TRAIL>, cudaFuncAttributeMaxDynamicSharedMemorySize, spk::OZ_SMEM));
+        CU(h, cudaFuncSetAttribute(spk::k_oz_update<spk::TC_SCHUR>, cudaFuncAttributeMaxDynamicSharedMemorySize, spk::OZ_SMEM));
+    }
     if (std::is_same<T, float>::value) {
         CU(h, cudaFuncSetAttribute(spk::k_block_lu_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, spk::LuSmem::bytes));
         CU(h, cudaFuncSetAttribute(spk::k_tc_update<spk::TC_TRAIL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1352,6 +1375,7 @@ static int factor_launches(spk_handle* h, int fs_nrhs = 0) {
                                                                                   PL.d_blk_front, ent);
         }
     };
+    if (std::is_same<T, double>::value) CU(h, cudaMemsetAsync(h->d_rexp, 0, sizeof(int) * (size_t)h->n, h->stream));
     const bool queue = h->leaf_queue != 0 && PL.nq > 0;
     if (queue) {   // the bottom subtrees first, in one persistent launch
         CU(h, cudaMemcpyAsync(PL.d_q_deps, PL.d_q_deps0, sizeof(int) * h->fronts.size(), cudaMemcpyDeviceToDevice,
@@ -1452,7 +1476,12 @@ static int factor_launches(spk_handle* h, int fs_nrhs = 0) {
                 if (rec.tiles <= 0) return;
                 LaunchScope ls(h, SPK_K_PANEL, rec.flops, rec.words * sizeof(T));
                 const spk::Launch la = launch_of(PL, rec);
-                if (bw <= 32)
+                if constexpr (std::is_same<T, double>::value) {
+                    if (bw <= 32)
+                        spk::k_block_panel_f64<32><<<rec.tiles, 128, panel64_smem<32>(), st>>>(fac, h->d_ipiv, S, la, (int)t, h->d_rexp);
+                    else
+                        spk::k_block_panel_f64<64><<<rec.tiles, 128, panel64_smem<64>(), st>>>(fac, h->d_ipiv, S, la, (int)t, h->d_rexp);
+                } else if (bw <= 32)
                     spk::k_block_panel<T, 32><<<rec.tiles, 256, sweep_smem<T, 32>(1), st>>>(
                         fac, h->d_ipiv, h->d_bmap, S, la, (int)t, storage<T>(h).pack, bf16, part);
                 else if (bw <= 64)
@@ -1475,40 +1504,49 @@ static int factor_launches(spk_handle* h, int fs_nrhs = 0) {
                 spk::k_block_trail<T><<<P.btrail[t].tiles, 256, 0, h->stream>>>(fac, S, launch_of(PL, P.btrail[t]),
                                                                                  (int)t);
             }
-            if constexpr (std::is_same<T, float>::value) {
-                // Tiles 1.. of the tensor-core trailing update: on the side
-                // stream when looking ahead, on as many SMs as the next
-                // block LU and tile 0 leave free; the next panels wait for it.
-                if (P.btrail_tc[t].tiles > 0) {
-                    const int nt = P.btrail_tc[t].tiles;
-                    int grid = std::min(nt, h->nsm);
-                    cudaStream_t st = h->stream;
-                    if (ahead) {
-                        const int reserve = std::max(P.btrail_tc0[t].tiles,
-                                                     t + 1 < P.blu.size() ? P.blu[t + 1].tiles : 0);
-                        grid = std::max(std::min(nt, h->nsm - reserve), std::min(nt, h->nsm / 2));
-                        CU(h, cudaEventRecord(h->evP, h->stream));   // with a split: the near tiles done
-                        CU(h, cudaStreamWaitEvent(h->side, h->evP, 0));
-                        st = h->side;
-                    }
-                    LaunchScope ls(h, SPK_K_TC_TRAIL, P.btrail_tc[t].flops, P.btrail_tc[t].words * sizeof(T));
-                    auto kern = bf16 ? spk::k_tc_update<spk::TC_TRAIL, true> : spk::k_tc_update<spk::TC_TRAIL, false>;
-                    kern<<<grid, spk::TC_THREADS, spk::umma::PSMEM, st>>>(
-                        fac, storage<T>(h).pack, S, launch_of(PL, P.btrail_tc[t]), (int)t, nt, 1, 0, h->d_info + 1);
-                    if (ahead) {
-                        CU(h, cudaEventRecord(h->evB, h->side));
-                        pending = true;
-                    }
-                }
-                // Tile 0 (the next block's diagonal block) on the launch stream.
-                if (P.btrail_tc0[t].tiles > 0) {
-                    LaunchScope ls(h, SPK_K_TC_TRAIL, P.btrail_tc0[t].flops, P.btrail_tc0[t].words * sizeof(T));
-                    const int nt = P.btrail_tc0[t].tiles;
-                    auto kern = bf16 ? spk::k_tc_update<spk::TC_TRAIL, true> : spk::k_tc_update<spk::TC_TRAIL, false>;
-                    kern<<<std::min(nt, h->nsm), spk::TC_THREADS, spk::umma::PSMEM, h->stream>>>(
-                        fac, storage<T>(h).pack, S, launch_of(PL, P.btrail_tc0[t]), (int)t, nt, 0, 0, h->d_info + 1);
+            if constexpr (std::is_same<T, double>::value) {
+                if (P.oz_pack[t].tiles > 0) {
+                    LaunchScope ls(h, SPK_K_PANEL, 0.0, 3.0 * P.oz_pack[t].words * sizeof(T));
+                    spk::k_oz_pack<<<P.oz_pack[t].tiles, 256, 0, h->stream>>>(fac, h->d_rexp, storage<T>(h).pack, S,
+                                                                            launch_of(PL, P.oz_pack[t]), (int)t);
                 }
             }
+            // The tensor-core trailing update, on `grid` SMs: part 1 the near
+            // tiles (the next block's diagonal block), 2 the others.
+            auto trail = [&](const LaunchRec& rec, int part, int grid, cudaStream_t st) {
+                LaunchScope ls(h, SPK_K_TC_TRAIL, rec.flops, rec.words * sizeof(T));
+                const spk::Launch la = launch_of(PL, rec);
+                if constexpr (std::is_same<T, float>::value) {
+                    auto kern = bf16 ? spk::k_tc_update<spk::TC_TRAIL, true> : spk::k_tc_update<spk::TC_TRAIL, false>;
+                    kern<<<grid, spk::TC_THREADS, spk::umma::PSMEM, st>>>(fac, storage<T>(h).pack, S, la, (int)t, rec.tiles,
+                                                                        part - 1, 0, h->d_info + 1);
+                } else {
+                    spk::k_oz_update<spk::TC_TRAIL><<<grid, spk::TC_THREADS, spk::OZ_SMEM, st>>>(
+                        fac, storage<T>(h).pack, S, la, (int)t, rec.tiles, part, h->d_info + 1);
+                }
+            };
+            // The other tiles: on the side stream when looking ahead, on as
+            // many SMs as the next block LU and the near tiles leave free; the
+            // next panels wait for it.
+            if (P.btrail_tc[t].tiles > 0) {
+                const int nt = P.btrail_tc[t].tiles;
+                int grid = std::min(nt, h->nsm);
+                cudaStream_t st = h->stream;
+                if (ahead) {
+                    const int reserve = std::max(P.btrail_tc0[t].tiles, t + 1 < P.blu.size() ? P.blu[t + 1].tiles : 0);
+                    grid = std::max(std::min(nt, h->nsm - reserve), std::min(nt, h->nsm / 2));
+                    CU(h, cudaEventRecord(h->evP, h->stream));   // with a split: the near tiles done
+                    CU(h, cudaStreamWaitEvent(h->side, h->evP, 0));
+                    st = h->side;
+                }
+                trail(P.btrail_tc[t], 2, grid, st);
+                if (ahead) {
+                    CU(h, cudaEventRecord(h->evB, h->side));
+                    pending = true;
+                }
+            }
+            // The near tiles on the launch stream.
+            if (P.btrail_tc0[t].tiles > 0) trail(P.btrail_tc0[t], 1, std::min(P.btrail_tc0[t].tiles, h->nsm), h->stream);
         }
         if (pending) {   // the level's Schur complement needs every trailing update
             CU(h, cudaStreamWaitEvent(h->stream, h->evB, 0));
@@ -1517,6 +1555,14 @@ static int factor_launches(spk_handle* h, int fs_nrhs = 0) {
         if (P.schur.tiles > 0) {
             LaunchScope ls(h, SPK_K_SCHUR, P.schur.flops, P.schur.words * sizeof(T));
             spk::k_schur<T><<<P.schur.tiles, 256, 0, h->stream>>>(fac, S, launch_of(PL, P.schur));
+        }
+        if constexpr (std::is_same<T, double>::value) {
+            if (P.schur_tc.tiles > 0) {
+                LaunchScope ls(h, SPK_K_TC_SCHUR, P.schur_tc.flops, P.schur_tc.words * sizeof(T));
+                const int nt = P.schur_tc.tiles;
+                spk::k_oz_update<spk::TC_SCHUR><<<std::min(nt, h->nsm), spk::TC_THREADS, spk::OZ_SMEM, h->stream>>>(
+                    fac, storage<T>(h).pack, S, launch_of(PL, P.schur_tc), 0, nt, 0, h->d_info + 1);
+            }
         }
         if constexpr (std::is_same<T, float>::value) {
             auto schur_tc = [&](const LaunchRec& rec, int part, int grid, cudaStream_t st) {
@@ -2937,7 +2983,7 @@ void spk_destroy(spk_handle* h) {
     if (h->own) cudaStreamSynchronize(h->own);
     for (Plan& P : h->plan) free_plan(P);
     void* ptrs[] = {h->d_xs, h->d_rows, h->d_runid, h->d_run_tgt, h->d_run_start, h->d_run_rel,
-                    h->d_rel, h->d_ipiv, h->d_bmap, h->d_info, h->d_slot, h->d_aval, h->d_acsr,
+                    h->d_rel, h->d_ipiv, h->d_bmap, h->d_rexp, h->d_info, h->d_slot, h->d_aval, h->d_acsr,
                     h->d_rowptr, h->d_col, h->d_src, h->d_ccolptr, h->d_crow, h->d_ccol, h->d_rperm, h->d_rinvp, h->d_wb,
                     h->d_wy, h->d_wx, h->d_rhs, h->d_x, h->d_r, h->d_sums, h->gm_V, h->gm_Z, h->gm_w, h->gm_c};
     for (void* p : ptrs)

@@ -2079,6 +2079,137 @@ __host__ __device__ __forceinline__ int panel_tile(int part, int tile, int nL, i
     return tile < nL - aL ? aL + tile : nL + aU + (tile - (nL - aL));
 }
 
+// FP64 panels.  A double multiply-add takes a warp 64 cycles and an SM 19 per
+// warp, so the panels are bound by how many there are and how many SMs share
+// them: a line (row of X, column of Y) is held by eight lanes, lane q entries
+// q, q + 8, .. (cyclic, so that step k touches only the entries after it: 288
+// instead of 1024 multiply-adds per 64-step sweep), and a CTA of four warps
+// takes 16 lines (64 before), four times as many CTAs for the few fronts near
+// the root.  rows: X := X inv(U_B) with the rows of U_B staged over their
+// diagonal, so that only the last step scales; cols: Y := inv(L_B) P_B Y.
+// 48^3 convection-diffusion: 18.0 -> 9.4 ms for all panels (FP64-bound: 5.6 ms
+// at the full rate).
+constexpr int PD_LINES = 16, PD_LANES = 8;
+template <int W>
+__device__ __forceinline__ void sweep_f64(double (&x)[W / PD_LANES], const double* sT, int bw) {
+    constexpr int CQ = W / PD_LANES;
+    const int lane = threadIdx.x & 31, q = lane & (PD_LANES - 1), base = lane & ~(PD_LANES - 1);
+#pragma unroll
+    for (int k = 0; k < W - 1; ++k)
+        if (k < bw - 1) {
+            const double xk = __shfl_sync(0xffffffffu, x[k / PD_LANES], base | (k % PD_LANES));
+            const double* t = sT + k * (W + 1) + q;
+#pragma unroll
+            for (int jj = (k + 1) / PD_LANES; jj < CQ; ++jj) x[jj] -= xk * t[jj * PD_LANES];   // zero up to the diagonal
+        }
+}
+
+// The largest exponent field of every U row over the lines of a CTA into
+// rexp, from which the slices of the tensor-core updates take their scaling
+// along the block.
+template <int CQ>
+__device__ __forceinline__ void oz_row_max(const double (&y)[CQ], bool ok, int bw, int* smx, int* rexp) {
+    const int lane = threadIdx.x & 31, q = lane & (PD_LANES - 1);
+    if ((int)threadIdx.x < PD_LANES * CQ) smx[threadIdx.x] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < CQ; ++i) {
+        int e = ok ? (__double2hiint(y[i]) >> 20) & 0x7ff : 0;
+        e = max(e, __shfl_xor_sync(0xffffffffu, e, 8));
+        e = max(e, __shfl_xor_sync(0xffffffffu, e, 16));
+        if (lane < PD_LANES && e > 0) atomicMax(&smx[i * PD_LANES + q], e);
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < bw && smx[threadIdx.x] > 0) atomicMax(&rexp[threadIdx.x], smx[threadIdx.x]);
+}
+
+template <int W>
+__global__ void __launch_bounds__(128) k_block_panel_f64(double* fac, const int* ipiv, Sched S, Launch L, int step, int* rexp) {
+    constexpr int CQ = W / PD_LANES, LD = W + 1;   // staged row k at k * LD
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double* sT = reinterpret_cast<double*>(smem_raw);
+    __shared__ double sd[W], rd[W];   // U(k, k) and its reciprocal
+    __shared__ int q0[W + 1], gmap[W], pa[W], smx[W];
+    int fid, tile;
+    locate(L, blockIdx.x, fid, tile);
+    const DFront F = S.fronts[fid];
+    const int blk = F.block0 + step;
+    const int c0 = S.blk_c0[blk], c1 = S.blk_c1[blk], bw = c1 - c0;
+    const int p0 = S.blk_p0[blk], np = S.blk_np[blk];
+    const int tid = threadIdx.x, line = tid / PD_LANES, q = tid & (PD_LANES - 1);
+    const int nL = cdiv(F.ld - c1, PD_LINES), nUa = cdiv(F.nf - c1, PD_LINES);
+    const double* blkp = fac + F.loff + (ll)c0 * F.ld + c0;
+    double x[CQ];
+    if (tile < nL) {
+        const int r = c1 + tile * PD_LINES + line;
+        const bool ok = r < F.ld;
+        double* xp = fac + F.loff + (ll)c0 * F.ld + r;   // row r, block column j at xp[j * ld]
+#pragma unroll
+        for (int jj = 0; jj < CQ; ++jj) {   // in flight while the triangle is staged
+            const int j = jj * PD_LANES + q;
+            x[jj] = (ok && j < bw) ? xp[(ll)j * F.ld] : 0.0;
+        }
+        if (tid < bw) {
+            const double d = blkp[(ll)tid * F.ld + tid];
+            sd[tid] = d;
+            rd[tid] = 1.0 / d;
+        }
+        __syncthreads();
+        for (int e = tid; e < W * W; e += 128) {
+            const int k = e % W, j = e / W;   // contiguous in k
+            sT[k * LD + j] = j > k && j < bw ? blkp[(ll)j * F.ld + k] * rd[k] : 0.0;
+        }
+        __syncthreads();
+        sweep_f64<W>(x, sT, bw);
+#pragma unroll
+        for (int jj = 0; jj < CQ; ++jj) {
+            const int j = jj * PD_LANES + q;
+            if (j < bw) x[jj] *= rd[j];
+            if (ok && j < bw) xp[(ll)j * F.ld] = x[jj];
+        }
+        if (S.sym) {   // symmetric form: the U side, U(c0 + j, r) = U(j, j) L(r, c0 + j)
+#pragma unroll
+            for (int jj = 0; jj < CQ; ++jj) {
+                const int j = jj * PD_LANES + q;
+                if (j < bw) x[jj] *= sd[j];
+                if (ok && j < bw) {
+                    if (r < F.nf) fac[F.loff + (ll)r * F.ld + c0 + j] = x[jj];
+                    else fac[F.uoff + (ll)(c0 + j) * F.m + (r - F.nf)] = x[jj];
+                }
+            }
+            if (S.blk_upack[blk] >= 0) oz_row_max<CQ>(x, ok, bw, smx, rexp + F.f + c0);
+        }
+    } else {
+        for (int k = tid; k <= np; k += 128) q0[k] = S.xsuper[p0 + k] - F.f - c0;
+        __syncthreads();
+        block_gather_map(ipiv + F.f + c0, q0, np, gmap, pa);
+        __syncthreads();
+        const bool inner = tile < nL + nUa;
+        const int col = inner ? c1 + (tile - nL) * PD_LINES + line : (tile - nL - nUa) * PD_LINES + line;
+        const bool ok = inner ? col < F.nf : col < F.m;
+        // block row k of this column at cp[k * stride]
+        double* cp = inner ? fac + F.loff + (ll)col * F.ld + c0 : fac + F.uoff + (ll)c0 * F.m + col;
+        const ll stride = inner ? 1 : (ll)F.m;
+#pragma unroll
+        for (int jj = 0; jj < CQ; ++jj) {   // in flight while the triangle is staged
+            const int k = jj * PD_LANES + q;
+            x[jj] = (ok && k < bw) ? cp[(ll)gmap[k] * stride] : 0.0;
+        }
+        for (int e = tid; e < W * W; e += 128) {   // rows left of a piece in its pivoted order, as stage_lower
+            const int i = e % W, k = e / W;
+            sT[k * LD + i] = i > k && i < bw ? blkp[(ll)k * F.ld + (k < pa[i] ? gmap[i] : i)] : 0.0;
+        }
+        __syncthreads();
+        sweep_f64<W>(x, sT, bw);
+#pragma unroll
+        for (int jj = 0; jj < CQ; ++jj) {
+            const int k = jj * PD_LANES + q;
+            if (ok && k < bw) cp[(ll)k * stride] = x[jj];
+        }
+        if (S.blk_upack[blk] >= 0) oz_row_max<CQ>(x, ok, bw, smx, rexp + F.f + c0);
+    }
+}
+
 template <typename T, int W>
 __global__ void __launch_bounds__(256) k_block_panel(T* fac, const int* ipiv, const int* bmap, Sched S, Launch L,
                                                       int step, unsigned char* pack, int bf16, int part) {
@@ -3199,6 +3330,450 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc_update(float* fac, const u
     __syncthreads();
     umma::fence_after();
     if (warp == 1) umma::tmem_dealloc(tmem, G::TMEM_COLS);
+}
+
+// ---------------------------------------------------------------------------
+// FP64 rank updates on the tensor cores by exact integer slices (the error-
+// free transformation of Ozaki, Ogita, Oishi and Rump, "Error-free
+// transformations of matrix multiplication by using fast routines of matrix
+// multiplication and its applications", Numerical Algorithms 59, 2012).
+//   The FP64 units of this GPU do 1.7 multiply-adds per cycle and SM, the
+// BF16 tensor pipe 4096.  Every line of a block's panels (a row of L, a
+// column of U; 64 entries at most) is written as OZ_D = 8 signed base-256
+// digits of a 62-bit fixed-point number relative to the line's largest entry:
+// entries down to 2^-9 of it are held exactly, digits are exact BF16 values
+// and a product of two slices over 64 columns is an exact FP32 integer
+// (below 2^20, and below 2^23 for the up to eight pairs of one weight).  The
+// 36 pairs of weight 0 .. 7 are summed per weight in tensor memory, joined as
+// 64-bit integers in the epilogue and added to the FP64 target with one
+// rounding per 64 columns.  The dropped pairs are below 2^-61 of the product
+// of the two largest entries, so the error is that of a handful of FP64
+// roundings where the multiply-add loop makes 64 (4096 x 4096 entries of
+// 64-term sums of uniform [-1, 1] values against 128-bit sums: largest error
+// 8.7e-16, of the loop 6.2e-15).
+//   Rows and columns may differ in size by any power of two (each line has
+// its exponent); along the block's columns L is scaled by 2^t and U by 2^-t
+// with t the exponent of the U row's largest entry, so that badly row-,
+// column- or symmetrically scaled matrices lose nothing.  A line that holds
+// an infinity or a NaN, and a product whose scale leaves the exponent range,
+// take a plain FP64 sum over the stored factor instead.
+//   Tiles of 128 x 32: eight weights of 32 columns are 256 TMEM columns,
+// double-buffered.  What bounds it: an MMA of 128 rows takes 95 cycles up to 64
+// columns, so a 128 x 32 x 64 product is 144 x 95 = 13,700 cycles, beside
+// the epilogue's FP64 work (two conversions and two multiply-adds per entry, 9,000
+// cycles) and its loads; 15,000 cycles measured, 11 TFLOP/s on a 4096 x 4096 x 64
+// update where the multiply-add tiles give 1.05.  48^3 convection-diffusion,
+// rank updates: 131 -> 23 ms.
+// ---------------------------------------------------------------------------
+constexpr int OZ_D = 8, OZ_N = 32;                       // digits, tile columns
+constexpr int OZ_SLICE = umma::PCHUNK16;                 // one slice of a 128-line tile and 16 columns, 4 KB
+constexpr int OZ_CHUNK = OZ_D * OZ_SLICE;                // 32 KB
+constexpr int OZ_SUB = OZ_SLICE / 4;                     // 32 of its lines, 1 KB
+constexpr int OZ_STAGE = OZ_CHUNK + OZ_D * OZ_SUB;       // A chunk, B chunk: 40 KB
+constexpr int OZ_NST = 5;
+constexpr int OZ_EXPS = (umma::TM + OZ_N) * 4;           // exponents of a tile's rows and columns for one block
+constexpr int OZ_ERING = 8;                              // more than the blocks the copies can run ahead
+constexpr int OZ_SMEM = OZ_NST * OZ_STAGE + OZ_ERING * OZ_EXPS + 2048;
+constexpr int OZ_BAD = 1 << 28;                          // exponent of a line with a NaN or an infinity
+
+// Bytes of one side of a block's pack: T tiles of 128 lines, nch chunks of 16
+// columns, then the lines' exponents.
+__host__ __device__ __forceinline__ ll oz_side_bytes(int T, int nch) { return (ll)T * ((ll)nch * OZ_CHUNK + 512); }
+__device__ __forceinline__ int* oz_exps(unsigned char* side, int T, int nch) {
+    return reinterpret_cast<int*>(side + (ll)T * nch * OZ_CHUNK);
+}
+
+// Tiles of 128 rows x 32 columns, row by row.  TRAIL: (n1 + n2) x c1 on the
+// front columns, then n1 x c2 on U12; the symmetric form the tiles with an
+// entry on or below the diagonal of the front columns.  SCHUR: n2 x c2.
+__host__ __device__ __forceinline__ int oz_lower(int n, int c) {   // rows rt hold min(4 (rt + 1), c) tiles
+    const int full = c / 4 < n ? c / 4 : n;
+    return 2 * full * (full + 1) + (n - full) * c;
+}
+__host__ __device__ __forceinline__ int oz_trail_tiles(int n1, int n2, int c1, int c2, bool sym) {
+    return sym ? oz_lower(n1 + n2, c1) : (n1 + n2) * c1 + n1 * c2;
+}
+__host__ __device__ __forceinline__ int oz_schur_tiles(int n2, int c2, bool sym) { return sym ? oz_lower(n2, c2) : n2 * c2; }
+// The trailing tiles that hold the next block's diagonal block (its 64 columns).
+__host__ __device__ __forceinline__ int oz_near(int c1) { return c1 < 2 ? c1 : 2; }
+__host__ __device__ __forceinline__ void oz_lower_tile(int t, int c, int& rt, int& ct) {
+    rt = 0;
+    for (;;) {
+        const int k = 4 * (rt + 1) < c ? 4 * (rt + 1) : c;
+        if (t < k) break;
+        t -= k;
+        ++rt;
+    }
+    ct = t;
+}
+
+// The slices of a block's L and U panels: a CTA per side and 128-line tile,
+// two threads per line (32 columns each).
+__global__ void __launch_bounds__(256) k_oz_pack(const double* fac, const int* rexp, unsigned char* pack, Sched S, Launch L,
+                                                 int step) {
+    __shared__ int sE[2][128];
+    int fid, tile;
+    locate(L, blockIdx.x, fid, tile);
+    const DFront F = S.fronts[fid];
+    const int blk = F.block0 + step;
+    const int c0 = S.blk_c0[blk], c1 = S.blk_c1[blk], bw = c1 - c0, nch = cdiv(bw, umma::KCH);
+    const int n1 = cdiv(F.nf - c1, umma::TM), T = n1 + cdiv(F.m, umma::TM);
+    const bool isU = tile >= T;
+    const int t = isU ? tile - T : tile, line = threadIdx.x & 127, half = threadIdx.x >> 7;
+    const int idx = t < n1 ? c1 + t * umma::TM + line : F.nf + (t - n1) * umma::TM + line;
+    const bool ok = idx < (t < n1 ? F.nf : F.ld);
+    // entry k of the line at p[k * ps]
+    const double* p = !isU ? fac + F.loff + (ll)c0 * F.ld + idx
+                           : idx < F.nf ? fac + F.loff + (ll)idx * F.ld + c0 : fac + F.uoff + (ll)c0 * F.m + (idx - F.nf);
+    const ll ps = !isU ? F.ld : idx < F.nf ? 1 : F.m;
+    const int k0 = half * 32;
+    long long x[32];
+#pragma unroll
+    for (int k = 0; k < 32; ++k) x[k] = ok && k0 + k < bw ? __double_as_longlong(p[(k0 + k) * ps]) : 0ll;
+    int E = -(1 << 20);
+#pragma unroll
+    for (int k = 0; k < 32; ++k) {
+        const int ex = (int)((x[k] >> 52) & 0x7ff);
+        const int tk = k0 + k < bw ? rexp[F.f + c0 + k0 + k] : 0, sh = tk ? (isU ? 1023 - tk : tk - 1023) : 0;
+        if (ex == 0x7ff) E = OZ_BAD;
+        else if ((x[k] << 1) != 0) E = max(E, (ex ? ex : 1) - 1022 + sh);   // |x| 2^sh < 2^E
+    }
+    sE[half][line] = E;
+    __syncthreads();
+    E = max(sE[0][line], sE[1][line]);
+    if (E == -(1 << 20)) E = 0;
+    unsigned char* side = pack + (isU ? S.blk_upack[blk] : S.blk_lpack[blk]);
+    if (half == 0) oz_exps(side, T, nch)[t * umma::TM + line] = E;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {   // eight columns: one 16-byte unit per slice
+        const int kg = k0 + 8 * g;
+        if (kg >= nch * umma::KCH) break;
+        long long q[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const long long b = x[8 * g + e];
+            const int tk = kg + e < bw ? rexp[F.f + c0 + kg + e] : 0, sh = tk ? (isU ? 1023 - tk : tk - 1023) : 0;
+            const int ex = (int)((b >> 52) & 0x7ff);
+            const long long m = (b & 0xfffffffffffffll) | (ex ? 1ll << 52 : 0ll);
+            const int s = (ex ? ex : 1) - 1075 + sh + 62 - E;   // |x| 2^(sh + 62 - E) = m 2^s, s <= 9
+            long long v = 0;
+            if (E != OZ_BAD && s >= 0) v = m << s;
+            else if (E != OZ_BAD && s > -54) v = (m + (1ll << (-s - 1))) >> -s;
+            q[e] = b < 0 ? -v : v;
+        }
+        // L: slices of 128 lines; U: of 32 lines, so that a tile's eight slices are contiguous
+        unsigned char* dst = side + ((ll)t * nch + kg / umma::KCH) * OZ_CHUNK +
+                             (isU ? (line / OZ_N) * (OZ_D * OZ_SUB) : 0) +
+                             umma::packed_offset16(isU ? line % OZ_N : line, kg % umma::KCH);
+        const int ds = isU ? OZ_SUB : OZ_SLICE;
+#pragma unroll
+        for (int d = OZ_D - 1; d >= 0; --d) {
+            unsigned w[4];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const int c = (int)(signed char)(q[e] & 0xff);
+                q[e] = (q[e] - c) >> 8;
+                const unsigned h = __float_as_uint((float)c) >> 16;   // exact in BF16
+                w[e / 2] = (e & 1) ? w[e / 2] | h << 16 : h;
+            }
+            *reinterpret_cast<uint4*>(dst + d * ds) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+    }
+}
+
+struct OzTile {
+    DFront F;
+    int p0 = 0, p1 = 0;  // tiles of the launch in this front: a CTA's next tile is mostly in the same one
+    int t0;              // its first local tile
+    int rt, ct;          // 128-row tile, 32-column tile (of its region)
+    int n1, n2, c1, c2;  // TRAIL: row tiles of [c1, nf) and [nf, ld), column tiles of [c1, nf) and U12
+    int b0, nb;          // blocks
+    int fc1;             // TRAIL: end column of the block
+};
+// part: TRAIL 1 the near tiles, 2 the others.
+template <int MODE>
+__device__ __forceinline__ void oz_decode(OzTile& T, const Sched& S, const Launch& L, int step, int tile, int part) {
+    if (tile < T.p0 || tile >= T.p1) {
+        int lo = 0, hi = L.count - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (L.prefix[mid] <= tile) lo = mid; else hi = mid - 1;
+        }
+        T.F = S.fronts[L.front_ids[lo]];
+        T.p0 = L.prefix[lo];
+        T.p1 = L.prefix[lo + 1];
+        T.n2 = cdiv(T.F.m, umma::TM);
+        T.c2 = cdiv(T.F.m, OZ_N);
+        T.t0 = 0;
+        if (MODE == TC_TRAIL) {
+            T.fc1 = S.blk_c1[T.F.block0 + step];
+            T.n1 = cdiv(T.F.nf - T.fc1, umma::TM);
+            T.c1 = cdiv(T.F.nf - T.fc1, OZ_N);
+            T.b0 = T.F.block0 + step;
+            T.nb = 1;
+            if (part == 2) T.t0 = oz_near(T.c1);
+        } else {
+            T.n1 = T.c1 = T.fc1 = 0;
+            T.b0 = T.F.block0;
+            T.nb = T.F.nblocks;
+        }
+    }
+    const int t = tile - T.p0 + T.t0;
+    if (MODE == TC_TRAIL) {
+        const int nL = (T.n1 + T.n2) * T.c1;
+        if (S.sym) oz_lower_tile(t, T.c1, T.rt, T.ct);
+        else if (t < nL) {
+            T.rt = t / T.c1;
+            T.ct = t % T.c1;
+        } else {
+            T.rt = (t - nL) / T.c2;
+            T.ct = T.c1 + (t - nL) % T.c2;
+        }
+    } else if (S.sym) {
+        oz_lower_tile(t, T.c2, T.rt, T.ct);
+    } else {
+        T.rt = t / T.c2;
+        T.ct = t % T.c2;
+    }
+}
+// Pack tiles of block b for the tile: row tile ra, column tile rb and its quarter sub.
+template <int MODE>
+__device__ __forceinline__ void oz_lines(const Sched& S, const OzTile& T, int b, int& ra, int& rb, int& sub, int& nt) {
+    const int n1 = MODE == TC_TRAIL ? T.n1 : cdiv(T.F.nf - S.blk_c1[b], umma::TM);
+    nt = n1 + T.n2;
+    if (MODE == TC_TRAIL) {
+        ra = T.rt;
+        rb = T.ct < T.c1 ? T.ct / 4 : n1 + (T.ct - T.c1) / 4;
+        sub = T.ct < T.c1 ? T.ct % 4 : (T.ct - T.c1) % 4;
+    } else {
+        ra = n1 + T.rt;
+        rb = n1 + T.ct / 4;
+        sub = T.ct % 4;
+    }
+}
+
+// Sum over block b of L(row, k) U(k, col), plain FP64 (front-local row; col
+// of the front, or nf + the U12 column).
+__device__ __noinline__ double oz_plain(const double* fac, const Sched& S, const DFront& F, int b, int row, int col) {
+    const int c0 = S.blk_c0[b], c1 = S.blk_c1[b];
+    double s = 0.0;
+    for (int k = c0; k < c1; ++k)
+        s += fac[F.loff + (ll)k * F.ld + row] *
+             (col < F.nf ? fac[F.loff + (ll)col * F.ld + k] : fac[F.uoff + (ll)k * F.m + col - F.nf]);
+    return s;
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(TC_THREADS, 1) k_oz_update(double* fac, unsigned char* pack, Sched S, Launch L, int step,
+                                                             int ntiles, int part, int* err) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ ScatterRow tab[umma::TM + OZ_N];   // SCHUR: tile rows, then tile columns
+    __shared__ int dead;
+    unsigned char* stage = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    unsigned char* exps = stage + OZ_NST * OZ_STAGE;
+    uint64_t* full = reinterpret_cast<uint64_t*>(exps + OZ_ERING * OZ_EXPS);
+    uint64_t *empty = full + OZ_NST, *tfull = empty + OZ_NST, *tempty = tfull + 2, *efull = tempty + 2;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(efull + OZ_ERING);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < OZ_NST; ++s) {
+            umma::mbar_init(&full[s], 1);
+            umma::mbar_init(&empty[s], 1);
+        }
+        for (int b = 0; b < OZ_ERING; ++b) umma::mbar_init(&efull[b], 1);
+        for (int b = 0; b < 2; ++b) {
+            umma::mbar_init(&tfull[b], 1);
+            umma::mbar_init(&tempty[b], 32 * TC_EPI);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        dead = 0;
+    }
+    if (warp == 1) umma::tmem_alloc(tmem_slot, 512);
+    umma::fence_before();
+    __syncthreads();
+    umma::fence_after();
+    const uint32_t tmem = *tmem_slot;
+    volatile int* vdead = &dead;
+
+    if (warp == 0) {
+        if (lane == 0) {   // bulk copies
+            int s = 0, u = 0;
+            uint32_t ph = 0;
+            OzTile T;
+            for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+                oz_decode<MODE>(T, S, L, step, tile, part);
+                for (int b = T.b0; b < T.b0 + T.nb; ++b) {
+                    int ra, rb, sub, nt;
+                    oz_lines<MODE>(S, T, b, ra, rb, sub, nt);
+                    const int nch = cdiv(S.blk_c1[b] - S.blk_c0[b], umma::KCH);
+                    unsigned char *sa = pack + S.blk_lpack[b], *sb = pack + S.blk_upack[b];
+                    const unsigned char* pa = sa + (ll)ra * nch * OZ_CHUNK;
+                    const unsigned char* pb = sb + (ll)rb * nch * OZ_CHUNK + sub * (OZ_D * OZ_SUB);
+                    for (int c = 0; c < nch; ++c) {
+                        umma::wait_bounded(&empty[s], ph ^ 1, vdead, err);
+                        if (c == 0) {
+                            // the exponents: a free stage means that at most OZ_NST chunks, and the two
+                            // blocks whose accumulators are in use, are ahead of the epilogue
+                            const uint32_t e = umma::saddr(exps + (u % OZ_ERING) * OZ_EXPS);
+                            umma::arrive_expect_tx(&efull[u % OZ_ERING], OZ_EXPS);
+                            umma::bulk_g2s(e, oz_exps(sa, nt, nch) + ra * umma::TM, umma::TM * 4, &efull[u % OZ_ERING]);
+                            umma::bulk_g2s(e + umma::TM * 4, oz_exps(sb, nt, nch) + rb * umma::TM + sub * OZ_N, OZ_N * 4,
+                                           &efull[u % OZ_ERING]);
+                            ++u;
+                        }
+                        umma::arrive_expect_tx(&full[s], OZ_STAGE);
+                        const uint32_t dst = umma::saddr(stage + s * OZ_STAGE);
+                        umma::bulk_g2s(dst, pa + (ll)c * OZ_CHUNK, OZ_CHUNK, &full[s]);
+                        umma::bulk_g2s(dst + OZ_CHUNK, pb + (ll)c * OZ_CHUNK, OZ_D * OZ_SUB, &full[s]);
+                        if (++s == OZ_NST) { s = 0; ph ^= 1; }
+                    }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {   // MMAs
+            constexpr uint32_t IDESC = umma::idesc_bf16(umma::TM, OZ_N);
+            int s = 0, acc = 0;
+            uint32_t ph = 0, aph = 0;
+            OzTile T;
+            for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+                oz_decode<MODE>(T, S, L, step, tile, part);
+                for (int b = T.b0; b < T.b0 + T.nb; ++b) {
+                    const int nch = cdiv(S.blk_c1[b] - S.blk_c0[b], umma::KCH);
+                    umma::wait_bounded(&tempty[acc], aph ^ 1, vdead, err);
+                    umma::fence_after();
+                    for (int c = 0; c < nch; ++c) {
+                        umma::wait_bounded(&full[s], ph, vdead, err);
+                        umma::fence_after();
+                        const uint32_t a0 = umma::saddr(stage + s * OZ_STAGE), b0 = a0 + OZ_CHUNK;
+                        const uint64_t da = umma::desc_kmajor(a0, 128, umma::SBO16), db = umma::desc_kmajor(b0, 128, umma::SBO16);
+                        const uint32_t d0 = tmem + acc * (OZ_D * OZ_N);
+                        // weight w: digit pairs i + j = w (descriptors hold addresses in 16-byte units)
+#pragma unroll
+                        for (int w = 0; w < OZ_D; ++w)
+#pragma unroll
+                            for (int i = 0; i <= w; ++i)
+                                umma::mma_bf16(d0 + w * OZ_N, da + i * (OZ_SLICE >> 4), db + (w - i) * (OZ_SUB >> 4), IDESC,
+                                               c > 0 || i > 0 ? 1u : 0u);
+                        umma::commit(&empty[s]);
+                        if (++s == OZ_NST) { s = 0; ph ^= 1; }
+                    }
+                    umma::commit(&tfull[acc]);
+                    if (++acc == 2) { acc = 0; aph ^= 1; }
+                }
+            }
+        }
+    } else if (warp >= 4) {   // epilogue: thread = one TMEM lane (tile row), 8 of the tile's columns
+        const int q4 = warp & 3, i = 32 * q4 + lane, cg = (warp - 4) >> 2, et = threadIdx.x - 128;
+        int acc = 0, u = 0;
+        uint32_t aph = 0;
+        OzTile T;
+        for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+            oz_decode<MODE>(T, S, L, step, tile, part);
+            const DFront& F = T.F;
+            if (MODE == TC_SCHUR) {
+                asm volatile("bar.sync 1, %0;" ::"n"(32 * TC_EPI) : "memory");   // previous tile's scatter done
+                if (et < umma::TM) tab[et] = scatter_row<double>(S, F, T.rt * umma::TM + et);
+                else if (et < umma::TM + OZ_N) tab[et] = scatter_row<double>(S, F, T.ct * OZ_N + et - umma::TM);
+                asm volatile("bar.sync 1, %0;" ::"n"(32 * TC_EPI) : "memory");
+            }
+            // front-local row and columns of the product (columns past nf: U12)
+            int row, rend, col0, cend;
+            if (MODE == TC_TRAIL) {
+                const int c1 = T.fc1;
+                row = T.rt < T.n1 ? c1 + T.rt * umma::TM + i : F.nf + (T.rt - T.n1) * umma::TM + i;
+                rend = T.rt < T.n1 ? F.nf : F.ld;
+                col0 = T.ct < T.c1 ? c1 + T.ct * OZ_N : F.nf + (T.ct - T.c1) * OZ_N;
+                cend = T.ct < T.c1 ? F.nf : F.ld;
+            } else {
+                row = F.nf + T.rt * umma::TM + i;
+                col0 = F.nf + T.ct * OZ_N;
+                rend = cend = F.ld;
+            }
+            col0 += cg * 8;
+            const bool rok = row < rend;
+            // TRAIL: the targets' old values while the products are formed (and all loads before any store: distinct
+            // entries the compiler cannot tell apart)
+            const bool cL = MODE == TC_TRAIL && col0 < F.nf;
+            double* dst = cL ? fac + F.loff + (ll)col0 * F.ld + row : fac + F.uoff + (ll)row * F.m + (col0 - F.nf);
+            const ll sj = cL ? (ll)F.ld : 1;
+            double sum[8];   // SCHUR: the product; TRAIL: the target minus the product
+#pragma unroll
+            for (int j = 0; j < 8; ++j) sum[j] = MODE == TC_TRAIL && rok && col0 + j < cend ? dst[j * sj] : 0.0;
+            constexpr long long SIGN = MODE == TC_TRAIL ? (long long)(1ull << 63) : 0ll;
+            for (int b = T.b0; b < T.b0 + T.nb; ++b) {
+                const int* ev = reinterpret_cast<const int*>(exps + (u % OZ_ERING) * OZ_EXPS);
+                umma::wait_bounded(&efull[u % OZ_ERING], (u / OZ_ERING) & 1, vdead, err);
+                ++u;
+                const int ei = ev[i];
+                const int* fj = ev + umma::TM + cg * 8;
+                umma::wait_bounded(&tfull[acc], aph, vdead, err);
+                umma::fence_after();
+                const uint32_t taddr = tmem + acc * (OZ_D * OZ_N) + cg * 8 + ((uint32_t)(32 * q4) << 16);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float v[OZ_D][4];
+                    umma::tmem_ld8x4<OZ_N>(taddr + 4 * h, v);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        int n[OZ_D];
+#pragma unroll
+                        for (int w = 0; w < OZ_D; ++w) n[w] = __float2int_rn(v[w][j]);
+                        // weights 0..4 in units of 2^-44, 5..7 in units of 2^-68
+                        const long long hi = ((long long)(n[0] * 256 + n[1]) << 24) + ((long long)n[2] << 16) + (n[3] * 256 + n[4]);
+                        const long long lo = ((long long)n[5] << 16) + (n[6] * 256 + n[7]);
+                        const int f = fj[4 * h + j], E = ei + f - 44;
+                        double& s = sum[4 * h + j];
+                        if (E - 24 > -1022 && E < 960) {
+                            s = fma((double)lo, __longlong_as_double((long long)(E - 24 + 1023) << 52 | SIGN), s);
+                            s = fma((double)hi, __longlong_as_double((long long)(E + 1023) << 52 | SIGN), s);
+                        } else if (row < rend && col0 + 4 * h + j < cend) {
+                            const double v = oz_plain(fac, S, F, b, row, col0 + 4 * h + j);
+                            s += MODE == TC_TRAIL ? -v : v;
+                        }
+                    }
+                    __syncwarp();   // the next load is warp-wide
+                }
+                umma::fence_before();
+                umma::arrive(&tempty[acc]);
+                if (++acc == 2) { acc = 0; aph ^= 1; }
+            }
+            if (MODE == TC_TRAIL) {
+                if (rok)
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (col0 + j < cend) dst[j * sj] = sum[j];
+            } else if (rok) {
+                const int r = row - F.nf, c0 = col0 - F.nf;
+                const ScatterRow& R = tab[i];
+                int pos[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int c = c0 + j;
+                    pos[j] = -1;
+                    if (c < F.m && (r >= c || !S.sym)) pos[j] = r >= c ? S.rel[tab[umma::TM + cg * 8 + j].rel0 + r] : S.rel[R.rel0 + c];
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int c = c0 + j;
+                    if (c >= F.m || pos[j] < 0) continue;
+                    if (r >= c) {   // L entry of the front of R_F[c]
+                        const ScatterRow& Cc = tab[umma::TM + cg * 8 + j];
+                        if (Cc.pos >= 0) atomicAdd(&fac[Cc.loff + (ll)Cc.pos * Cc.ld + pos[j]], -sum[j]);
+                    } else if (R.pos >= 0) {   // entry of the front of R_F[r]
+                        const int pc = pos[j];
+                        const ll addr = pc < R.nf ? R.loff + (ll)pc * R.ld + R.pos : R.uoff + (ll)R.pos * R.m + (pc - R.nf);
+                        atomicAdd(&fac[addr], -sum[j]);
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    }
+    umma::fence_before();
+    __syncthreads();
+    umma::fence_after();
+    if (warp == 1) umma::tmem_dealloc(tmem, 512);
 }
 
 // Warp reduce-scatter: N (a power of 2, at most 32) values per lane, summed

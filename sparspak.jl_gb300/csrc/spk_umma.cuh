@@ -115,6 +115,32 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// Warp-wide: four consecutive FP32 columns of this warp's 32 TMEM lanes at
+// each of eight column offsets STEP apart (loads and their wait in one block).
+template <int STEP>
+__device__ __forceinline__ void tmem_ld8x4(uint32_t taddr, float (&v)[8][4]) {
+    uint32_t r[32];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%32];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%4, %5, %6, %7}, [%33];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%8, %9, %10, %11}, [%34];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%12, %13, %14, %15}, [%35];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%16, %17, %18, %19}, [%36];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%20, %21, %22, %23}, [%37];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%24, %25, %26, %27}, [%38];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x4.b32 {%28, %29, %30, %31}, [%39];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7]),
+          "=&r"(r[8]), "=&r"(r[9]), "=&r"(r[10]), "=&r"(r[11]), "=&r"(r[12]), "=&r"(r[13]), "=&r"(r[14]), "=&r"(r[15]),
+          "=&r"(r[16]), "=&r"(r[17]), "=&r"(r[18]), "=&r"(r[19]), "=&r"(r[20]), "=&r"(r[21]), "=&r"(r[22]), "=&r"(r[23]),
+          "=&r"(r[24]), "=&r"(r[25]), "=&r"(r[26]), "=&r"(r[27]), "=&r"(r[28]), "=&r"(r[29]), "=&r"(r[30]), "=&r"(r[31])
+        : "r"(taddr), "r"(taddr + STEP), "r"(taddr + 2 * STEP), "r"(taddr + 3 * STEP), "r"(taddr + 4 * STEP),
+          "r"(taddr + 5 * STEP), "r"(taddr + 6 * STEP), "r"(taddr + 7 * STEP)
+        : "memory");
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i / 4][i % 4] = __uint_as_float(r[i]);
+}
+
 // ---------------------------------------------------------------------------
 // Packed operands.  The panel kernel writes the L and U panels of a block a
 // second time as TF32 hi / lo parts already in the canonical layout: for a
