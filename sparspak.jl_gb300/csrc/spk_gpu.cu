@@ -1187,6 +1187,7 @@ static int ensure_plan(spk_handle* h) {
         (rc = prepare_front_solve<T, 1, true>(h)) || (rc = prepare_front_solve<T, 4, true>(h)))
         return rc;
     if (std::is_same<T, double>::value) {
+        CU(h, cudaFuncSetAttribute(spk::k_block_lu_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, spk::Lu64Smem::bytes));
         CU(h, cudaFuncSetAttribute(spk::k_oz_update<spk::TC_TRAIL>, cudaFuncAttributeMaxDynamicSharedMemorySize, spk::OZ_SMEM));
         CU(h, cudaFuncSetAttribute(spk::k_oz_update<spk::TC_SCHUR>, cudaFuncAttributeMaxDynamicSharedMemorySize, spk::OZ_SMEM));
     }
@@ -1457,8 +1458,8 @@ static int factor_launches(spk_handle* h, int fs_nrhs = 0) {
                     spk::k_block_lu_f32<<<P.blu[t].tiles, spk::LU_THREADS, spk::LuSmem::bytes, h->stream>>>(
                         fac, h->d_ipiv, h->d_info, h->d_bmap, S, launch_of(PL, P.blu[t]), (int)t);
                 else
-                    spk::k_block_lu<T><<<P.blu[t].tiles, spk::LuThreads<T>::value, 0, h->stream>>>(
-                        fac, h->d_ipiv, h->d_info, h->d_bmap, S, launch_of(PL, P.blu[t]), (int)t);
+                    spk::k_block_lu_f64<<<P.blu[t].tiles, spk::LU64_THREADS, spk::Lu64Smem::bytes, h->stream>>>(
+                        fac, h->d_ipiv, h->d_info, S, launch_of(PL, P.blu[t]), (int)t);
             }
             if (pending) {   // the panels read what the previous step's trailing update wrote
                 CU(h, cudaStreamWaitEvent(h->stream, h->evB, 0));

@@ -118,7 +118,7 @@ constexpr int MAXW = 64;
 // ---------------------------------------------------------------------------
 // Blocks.  The pieces of a front are processed in *blocks* of consecutive
 // pieces (at most BlockMax<T> columns).  A block step is: the block LU
-// (k_block_lu / k_block_lu_small) with exactly the reference's in-piece
+// (k_block_lu_f32, k_block_lu_f64, k_block_lu_small) with exactly the reference's in-piece
 // pivoting, then the block's two panels (k_block_panel), then the trailing
 // update of the front (k_block_trail).  After the factorisation
 // k_block_inv forms, per block, the two operators the triangular solves
@@ -380,7 +380,7 @@ __device__ __forceinline__ bool warp_block_lu(T (&r)[W], int bw, int nrow, const
 }
 
 // Blocks of at most 32 columns: one warp per block, four blocks per CTA (the
-// launch holds one block per front).  Same outputs as k_block_lu.
+// launch holds one block per front).
 template <typename T>
 __global__ void __launch_bounds__(128) k_block_lu_small(T* fac, int* ipiv, int* info, Sched S, Launch L, int step) {
     __shared__ int sq[4][33];
@@ -423,25 +423,6 @@ __global__ void __launch_bounds__(128) k_block_lu_small(T* fac, int* ipiv, int* 
     }
 }
 
-// First row holding the largest key (`idx` the row of this lane's key):
-// the reference's first strict maximum.
-__device__ __forceinline__ int warp_first_max_row(unsigned long long key, int idx) {
-    const unsigned FULL = 0xffffffffu;
-    const unsigned hi = (unsigned)(key >> 32), lo = (unsigned)key;
-    const unsigned mh = __reduce_max_sync(FULL, hi);
-    const unsigned ml = __reduce_max_sync(FULL, hi == mh ? lo : 0u);
-    return (int)__reduce_min_sync(FULL, (hi == mh && lo == ml) ? (unsigned)idx : 0xffffffffu);
-}
-template <typename T> struct PivotKey;
-template <> struct PivotKey<float> {
-    using type = unsigned;
-    __device__ static type of(float x, bool cand, bool diag) { return pivot_key32(x, cand, diag); }
-};
-template <> struct PivotKey<double> {
-    using type = unsigned long long;
-    __device__ static type of(double x, bool cand, bool diag) { return pivot_key(x, cand, diag); }
-};
-
 // Row sources of a block's interchanges: applying, piece by piece, the
 // swaps k <-> a + ipiv[k] of the piece [a, b) to a vector v gives
 // v'[R] = v[gmap[R]]; pa[R] = first row of R's piece.  One thread per piece.
@@ -461,265 +442,6 @@ __device__ __forceinline__ void block_gather_map(const int* ipiv_blk, const int*
     }
 }
 
-
-// Block LU in FP64 by a whole CTA (blocks of 33..BlockMax columns; one CTA
-// per front; FP32: k_block_lu_f32).  Warp w holds the column group [4w, 4w+4) of the block, lane l the
-// rows [RPT l, RPT l + RPT) (RPT = BlockMax / 32), in registers.  The block
-// is factored one column group at a time:
-//   A. the group's owner warp factors its four columns in order, on its own
-//      (shuffles only): for column k in piece [a, b), the pivot is the first
-//      strict maximum of |A(i,k)| over the piece's rows i in [k, b)
-//      (ggetrf!; a NaN never wins except on the diagonal); a nonzero pivot
-//      off the diagonal swaps rows k and kp over the group's columns >= a
-//      (ggetrf! inside the piece; columns left of the piece never move); the
-//      rows after k are scaled by 1 / pivot (ggetrf! scaling, the L-panel
-//      trsm 'r','u','n','n' for the block's later rows; no scaling after a
-//      zero pivot) and the group's later columns get the rank-1 update.  The
-//      multipliers and pivots go to shared memory;
-//   B. every later warp applies, column by column in the same order, the
-//      swap (_luswap! of the U rows) and the rank-1 update (the U-panel trsm
-//      'r','l','t','u' and the block-local Schur update) to its columns, with
-//      row k taken from the owning lane by shuffles: the same operations in
-//      the same order as a column-by-column elimination; earlier warps apply
-//      the swaps to their columns of the same piece.
-// The owner of the next group does its part B first and then its part A, so
-// the next panel overlaps the other warps' updates; one barrier per group.
-// ipiv receives the local pivot row within the piece; a zero pivot records
-// the piece in info.
-template <typename T> struct LuThreads { static constexpr int value = (BlockMax<T>::value / 4) * 32; };
-
-template <typename T, int RPT>
-__device__ __forceinline__ T lu_pick(const T (&a)[RPT][4], int ii, int jj) {
-    T v = a[0][jj];
-#pragma unroll
-    for (int q = 1; q < RPT; ++q) v = (ii == q) ? a[q][jj] : v;
-    return v;
-}
-
-
-// Part A for the group of warp `g` (called by that warp only).  cpa / cpb:
-// first and end column of each column's piece.
-template <typename T, int RPT>
-__device__ __forceinline__ void lu_group_factor(T (&a)[RPT][4], int g, int bw, const int* cpa, const int* cpb, T* lb,
-                                                int* skp, T* spv, int* sa0, int* spiv, int* szero, bool sym) {
-    using Key = typename PivotKey<T>::type;
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31, r0 = RPT * lane;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int k = 4 * g + j;
-        if (k >= bw) continue;
-        const int a0 = cpa[k], b = cpb[k];
-        Key best = 0;
-        int brow = 0;
-#pragma unroll
-        for (int ii = 0; ii < RPT; ++ii) {   // rows in ascending order: ties keep the earlier row
-            const int R = r0 + ii;
-            const Key kv = PivotKey<T>::of(a[ii][j], sym ? R == k : (R >= k && R < b), R == k);
-            if (ii == 0 || kv > best) { best = kv; brow = R; }
-        }
-        const int kp = warp_first_max_row(best, brow);
-        const int lk = (4 * g) / RPT + j / RPT, ik = j % RPT, lp = kp / RPT, ip = kp % RPT;   // k = 4g + j
-        const T pv = __shfl_sync(FULL, lu_pick(a, ip, j), lp);
-        const bool scale = pv != T(0);
-        if (scale && kp != k) {   // swap rows k and kp over the group's columns >= a0
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj) {
-                const T vk = __shfl_sync(FULL, a[ik][jj], lk);
-                const T vp = __shfl_sync(FULL, lu_pick(a, ip, jj), lp);
-                if (4 * g + jj >= a0) {
-#pragma unroll
-                    for (int ii = 0; ii < RPT; ++ii) {
-                        if (lane == lk && ii == ik) a[ii][jj] = vp;
-                        if (lane == lp && ii == ip) a[ii][jj] = vk;
-                    }
-                }
-            }
-        }
-        const T rinv = scale ? lu_recip(pv) : T(1);
-#pragma unroll
-        for (int ii = 0; ii < RPT; ++ii) {
-            const int R = r0 + ii;
-            if (R > k) {
-                if (scale) a[ii][j] *= rinv;
-                lb[j * (32 * RPT) + R] = a[ii][j];
-            }
-        }
-#pragma unroll
-        for (int jj = j + 1; jj < 4; ++jj) {   // rank-1 update of the group's later columns
-            const T u = __shfl_sync(FULL, a[ik][jj], lk);
-#pragma unroll
-            for (int ii = 0; ii < RPT; ++ii)
-                if (r0 + ii > k) a[ii][jj] -= a[ii][j] * u;
-        }
-        if (lane == 0) {
-            skp[j] = kp;
-            spv[j] = pv;
-            sa0[j] = a0;
-            spiv[k] = kp - a0;
-            if (!scale && k < *szero) *szero = k;
-        }
-    }
-}
-
-// Part B of group `g` for a later warp.
-template <typename T, int RPT>
-__device__ __forceinline__ void lu_group_update(T (&a)[RPT][4], int g, int bw, const T* lb, const int* skp, const T* spv) {
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31, r0 = RPT * lane;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int k = 4 * g + j;
-        if (k >= bw) continue;
-        const int kp = skp[j];
-        const T pv = spv[j];
-        const int lk = (4 * g) / RPT + j / RPT, ik = j % RPT;   // k = 4g + j
-        if (pv != T(0) && kp != k) {   // all columns here are after k, hence >= a0
-            const int lp = kp / RPT, ip = kp % RPT;
-#pragma unroll
-            for (int jj = 0; jj < 4; ++jj) {
-                const T vk = __shfl_sync(FULL, a[ik][jj], lk);
-                const T vp = __shfl_sync(FULL, lu_pick(a, ip, jj), lp);
-#pragma unroll
-                for (int ii = 0; ii < RPT; ++ii) {
-                    if (lane == lk && ii == ik) a[ii][jj] = vp;
-                    if (lane == lp && ii == ip) a[ii][jj] = vk;
-                }
-            }
-        }
-        T l[RPT];
-#pragma unroll
-        for (int ii = 0; ii < RPT; ++ii) l[ii] = lb[j * (32 * RPT) + r0 + ii];
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-            const T u = __shfl_sync(FULL, a[ik][jj], lk);
-#pragma unroll
-            for (int ii = 0; ii < RPT; ++ii)
-                if (r0 + ii > k) a[ii][jj] -= l[ii] * u;
-        }
-    }
-}
-
-// The swaps of group `g` for an earlier warp: its columns of the same piece
-// (>= the piece's first column) hold L entries that move with the rows.
-template <typename T, int RPT>
-__device__ __forceinline__ void lu_group_swap_left(T (&a)[RPT][4], int g, int bw, const int* skp, const T* spv,
-                                                   const int* sa0) {
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int k = 4 * g + j;
-        if (k >= bw) continue;
-        const int kp = skp[j], a0 = sa0[j];
-        if (spv[j] == T(0) || kp == k || 4 * w + 3 < a0) continue;   // uniform in the warp
-        const int lk = (4 * g) / RPT + j / RPT, ik = j % RPT, lp = kp / RPT, ip = kp % RPT;   // k = 4g + j
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-            const T vk = __shfl_sync(FULL, a[ik][jj], lk);
-            const T vp = __shfl_sync(FULL, lu_pick(a, ip, jj), lp);
-            if (4 * w + jj >= a0) {
-#pragma unroll
-                for (int ii = 0; ii < RPT; ++ii) {
-                    if (lane == lk && ii == ik) a[ii][jj] = vp;
-                    if (lane == lp && ii == ip) a[ii][jj] = vk;
-                }
-            }
-        }
-    }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(LuThreads<T>::value, 1) k_block_lu(T* fac, int* ipiv, int* info, int* bmap, Sched S,
-                                                                      Launch L, int step) {
-    constexpr int BM = BlockMax<T>::value, RPT = BM / 32;
-    __shared__ __align__(16) T lbuf[2][4 * BM];   // the group's multipliers by column and row (by group parity)
-    __shared__ T s_pv[2][4];
-    __shared__ int s_kp[2][4], s_a0[2][4];
-    __shared__ int q0[BM + 1];
-    __shared__ int spiv[BM], sgmap[BM], cpa[BM], cpb[BM];
-    __shared__ int szero;
-    int fid, tile;
-    locate(L, blockIdx.x, fid, tile);
-    const DFront F = S.fronts[fid];
-    const int blk = F.block0 + step;
-    const int c0 = S.blk_c0[blk], c1 = S.blk_c1[blk], bw = c1 - c0;
-    const int p0 = S.blk_p0[blk], np = S.blk_np[blk];
-    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-    const int r0 = RPT * lane, cl0 = 4 * w;
-    for (int k = tid; k <= np; k += blockDim.x) q0[k] = S.xsuper[p0 + k] - F.f - c0;
-    if (tid == 0) szero = INT_MAX;
-    __syncthreads();
-    for (int pc = tid; pc < np; pc += blockDim.x)
-        for (int k = q0[pc]; k < q0[pc + 1]; ++k) {
-            cpa[k] = q0[pc];
-            cpb[k] = q0[pc + 1];
-        }
-    T* blkp = fac + F.loff + (ll)c0 * F.ld + c0;   // block (i, j) at blkp[j * ld + i]
-    T a[RPT][4];
-#pragma unroll
-    for (int jj = 0; jj < 4; ++jj)
-#pragma unroll
-        for (int ii = 0; ii < RPT; ++ii) {
-            const int R = r0 + ii, C = cl0 + jj;
-            // symmetric form: the upper triangle mirrors the lower one
-            a[ii][jj] = (R < bw && C < bw) ? ((S.sym && R < C) ? blkp[(ll)R * F.ld + C] : blkp[(ll)C * F.ld + R]) : T(0);
-        }
-    __syncthreads();
-    const int ng = cdiv(bw, 4);
-    const bool sym = S.sym != 0;
-    if (w == 0) lu_group_factor<T, RPT>(a, 0, bw, cpa, cpb, lbuf[0], s_kp[0], s_pv[0], s_a0[0], spiv, &szero, sym);
-    __syncthreads();
-#pragma unroll 1
-    for (int g = 0; g < ng; ++g) {
-        const int par = g & 1;
-        if (w < g) lu_group_swap_left<T, RPT>(a, g, bw, s_kp[par], s_pv[par], s_a0[par]);
-        if (w > g && w < ng) {
-            lu_group_update<T, RPT>(a, g, bw, lbuf[par], s_kp[par], s_pv[par]);
-            if (w == g + 1)   // the next panel while the other warps update
-                lu_group_factor<T, RPT>(a, g + 1, bw, cpa, cpb, lbuf[par ^ 1], s_kp[par ^ 1], s_pv[par ^ 1],
-                                        s_a0[par ^ 1], spiv, &szero, sym);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int jj = 0; jj < 4; ++jj)
-#pragma unroll
-        for (int ii = 0; ii < RPT; ++ii) {
-            const int R = r0 + ii, C = cl0 + jj;
-            if (R < bw && C < bw) blkp[(ll)C * F.ld + R] = a[ii][jj];
-        }
-    for (int c = tid; c < bw; c += blockDim.x) ipiv[F.f + c0 + c] = spiv[c];
-    // Row sources of the block's interchanges (block_gather_map), a warp per
-    // piece of at most 32 columns: lane i tracks gmap[a + i] through the
-    // piece's swaps.  spiv and q0 were published by the loop's last barrier.
-    for (int pc = w; pc < np; pc += blockDim.x / 32) {
-        const int a = q0[pc], b = q0[pc + 1];
-        if (b - a <= 32) {
-            int g = a + lane;
-            for (int k = a; k < b; ++k) {
-                const int kp = a + spiv[k];
-                const int vk = __shfl_sync(0xffffffffu, g, k - a), vp = __shfl_sync(0xffffffffu, g, kp - a);
-                g = lane == k - a ? vp : (lane == kp - a ? vk : g);
-            }
-            if (lane < b - a) bmap[F.f + c0 + a + lane] = g | (a << 8);
-        } else if (lane == 0) {
-            for (int i = a; i < b; ++i) sgmap[i] = i;
-            for (int k = a; k < b; ++k) {
-                const int kp = a + spiv[k];
-                const int t = sgmap[k];
-                sgmap[k] = sgmap[kp];
-                sgmap[kp] = t;
-            }
-            for (int i = a; i < b; ++i) bmap[F.f + c0 + i] = sgmap[i] | (a << 8);
-        }
-    }
-    if (tid == 0 && szero != INT_MAX) {
-        int p = 0;
-        while (q0[p + 1] <= szero) ++p;
-        atomicMin(info, p0 + p + 1);   // first singular piece of the block
-    }
-}
 
 // ---------------------------------------------------------------------------
 // FP32 block LU by a whole CTA (blocks of 33..128 columns; one CTA per
@@ -744,8 +466,8 @@ __global__ void __launch_bounds__(LuThreads<T>::value, 1) k_block_lu(T* fac, int
 // column only publishes its multipliers and goes on, and the warps of the
 // later columns follow two columns behind.  One block of 120 columns alone
 // on the GPU: 29 us when every pivot is on the diagonal, 37 us with searches
-// (60 us in the column-group form k_block_lu, whose owner warp also moved rows
-// and updated 128 of them per column).
+// (60 us in the form before it, whose owner warp of each four columns also moved
+// rows and updated 128 of them per column).
 // ---------------------------------------------------------------------------
 constexpr int LU_THREADS = 512, LU_G = 32, LU_W = 8;   // group, columns per warp of a sweep
 constexpr int LU_LSW = LU_G + 4;   // entries per staged row of a group: 16-byte rows, 4 words apart in the bank cycle
@@ -1299,8 +1021,8 @@ __global__ void __launch_bounds__(LU_THREADS, 1) k_block_lu_f32(float* fac, int*
 //       a warp per four columns with its lanes on the rows.
 // Only the w rows of the piece are on the sequential path of (1); the rows
 // below are solved in parallel afterwards, which is where this form gains
-// over k_block_lu (whose owner warp sweeps all rows of the block for every
-// column).  Same outputs as k_block_lu: the factored block, ipiv, the row
+// over forms whose owner warp sweeps all rows of the block for every column.
+// Outputs: the factored block, ipiv, the row
 // sources of the interchanges (bmap) and the first singular piece.
 constexpr int PC_THREADS = 512;
 template <typename T> struct PcLu {
@@ -1836,7 +1558,7 @@ __device__ __forceinline__ int block_scale_exp(const float* blkp, int ld, int bw
 // entries [8c, 8c + 8) of the tile's lines 4h .. 4h + 3.  Same tiles,
 // operations and outputs as the generic form in k_block_panel; the row
 // sources of the block's interchanges (gmap | pa << 8 per block column) come
-// from k_block_lu through bmap.  The 64 lines of the tile pass through a
+// from k_block_lu_f32 through bmap.  The 64 lines of the tile pass through a
 // shared-memory copy sX (line li, entry j at li * PT_LD + j) so that the
 // global loads, stores and packed writes are coalesced: a warp moves 8 rows
 // x 4 columns of a column-major array (32-byte runs), and the packed writes
@@ -1987,7 +1709,7 @@ __device__ __forceinline__ void block_panel128(float* fac, const int* bmap, cons
             else if (offu >= 0) pack_tile(pack + offu, sX, nl, nch, whereL);
         }
     } else {
-        if (tid < bw) {   // the block's row sources, from k_block_lu
+        if (tid < bw) {   // the block's row sources, from k_block_lu_f32
             const int v = bmap[F.f + c0 + tid];
             gmap[tid] = v & 255;
             pa[tid] = v >> 8;
@@ -2207,6 +1929,288 @@ __global__ void __launch_bounds__(128) k_block_panel_f64(double* fac, const int*
             if (ok && k < bw) cp[(ll)k * stride] = x[jj];
         }
         if (S.blk_upack[blk] >= 0) oz_row_max<CQ>(x, ok, bw, smx, rexp + F.f + c0);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// FP64 block LU by a whole CTA (blocks of 33..64 columns; one CTA per front),
+// in the groups of k_block_lu_f32.  What bounds it is the number of double
+// multiply-adds (64 cycles each for a warp, 19 for an SM): every step touches
+// only rows and columns that are left, spread over the SM's four quarters:
+// a group's rows and columns in four warps of eight columns each (a lane per
+// row; the reciprocals of all candidates, 350 cycles, beside the search), its
+// L21 rows and U12 columns eight lanes per line as in the panels, the
+// rank-w update over all warps.  The form before it updated every row of the
+// block in every step: all block LUs of the 48^3 convection-diffusion system
+// 15.8 -> 13.3 ms, of the 256 x 256 diffusion system 2.0 -> 1.8 ms.
+// ---------------------------------------------------------------------------
+constexpr int LU64_THREADS = 256;
+struct Lu64Smem {   // offsets in doubles
+    static constexpr int BM = 64, LD = BM + 1, LT = LU_G + 1;
+    static constexpr int a = 0;                       // A(i, j) at a + j * LD + i
+    static constexpr int ex = a + BM * LD + 1;        // multipliers of the group's column k by row: ex + k * BM + row
+    static constexpr int t = ex + LU_G * BM;          // the group's triangles: U over its diagonal, row k at t + k * LT
+    static constexpr int l = t + LU_G * LT;           // L11, column k at l + k * LT
+    static constexpr int bytes = (l + LU_G * LT) * 8;
+};
+
+// Part 1 of a group, by warps q = 0 .. cdiv(w, 8) - 1: rows [0, nrow) (up to
+// 32 RPL) and columns [0, w) at A(i, j) = A[j * LD + i], in place (rows in
+// their final positions: entry (i, j) of original row r at position (j >=
+// left[r] ? at[r] : r), left[r] the first column (of the group) of r's piece).
+// piv: row | position << 8 of each column's pivot; at: positions; rd: pivot
+// reciprocals (1 for a zero pivot).
+template <int RPL>
+__device__ __forceinline__ void lu64_sweep(double* A, int nrow, int w, int cend, const int* left, double* ex, double* rd,
+                                           int* piv, int* at, int* zero, bool sym, int q) {
+    constexpr int LD = Lu64Smem::LD, BM = Lu64Smem::BM;
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, nq = cdiv(w, LU_W);
+    double P[RPL][LU_W];
+    int pos[RPL];
+    bool act[RPL];
+#pragma unroll
+    for (int s = 0; s < RPL; ++s) {
+        const int r = lane + 32 * s;
+        pos[s] = r;
+        act[s] = r < nrow;
+#pragma unroll
+        for (int j = 0; j < LU_W; ++j) P[s][j] = r < nrow && q * LU_W + j < w ? A[(q * LU_W + j) * LD + r] : 0.0;
+    }
+    auto place = [&](int k, int kr, int pp) {
+#pragma unroll
+        for (int s = 0; s < RPL; ++s) {
+            if (pos[s] == k) pos[s] = pp;
+            if (lane + 32 * s == kr) {
+                pos[s] = k;
+                act[s] = false;
+            }
+        }
+    };
+#pragma unroll 1
+    for (int o = 0; o < q; ++o)   // follow the warps of the earlier columns
+#pragma unroll 1
+        for (int t = 0; t < LU_W; ++t) {
+            const int k = o * LU_W + t;
+            asm volatile("bar.sync %0, %1;" ::"r"(4 + t), "r"(32 * (nq - o)) : "memory");
+            double l[RPL];
+#pragma unroll
+            for (int s = 0; s < RPL; ++s) l[s] = ex[k * BM + lane + 32 * s];
+            const int pv = piv[k], kr = pv & 255;
+            place(k, kr, pv >> 8);
+#pragma unroll
+            for (int j = 0; j < LU_W; ++j) {
+                const double u = __shfl_sync(FULL, RPL == 2 && kr >= 32 ? P[RPL - 1][j] : P[0][j], kr & 31);
+#pragma unroll
+                for (int s = 0; s < RPL; ++s)
+                    if (act[s]) P[s][j] -= l[s] * u;
+            }
+        }
+#pragma unroll
+    for (int t = 0; t < LU_W; ++t) {
+        const int k = q * LU_W + t;
+        if (k >= w) break;
+        const int ce = __shfl_sync(FULL, cend, k);
+        double rc[RPL];
+        unsigned long long key[RPL], best = 0ull;
+#pragma unroll
+        for (int s = 0; s < RPL; ++s) {
+            const bool diag = pos[s] == k, cand = act[s] && (sym ? diag : pos[s] < ce);
+            rc[s] = rcp_rn(cand ? P[s][t] : 1.0);
+            key[s] = pivot_key(P[s][t], cand, diag);
+            best = key[s] > best ? key[s] : best;
+        }
+        const unsigned mh = __reduce_max_sync(FULL, (unsigned)(best >> 32));
+        const unsigned ml = __reduce_max_sync(FULL, (unsigned)(best >> 32) == mh ? (unsigned)best : 0u);
+        const unsigned long long mx = ((unsigned long long)mh << 32) | ml;
+        unsigned p = 0xffffffffu;   // the first position that holds it
+#pragma unroll
+        for (int s = 0; s < RPL; ++s)
+            if (key[s] == mx && (unsigned)pos[s] < p) p = (unsigned)pos[s];
+        const unsigned pp = __reduce_min_sync(FULL, p);
+        int kr = 0;
+#pragma unroll
+        for (int s = 0; s < RPL; ++s) {
+            const unsigned b = __ballot_sync(FULL, act[s] && (unsigned)pos[s] == pp);
+            if (b) kr = 31 - __clz(b) + 32 * s;
+        }
+        const bool hi = RPL == 2 && kr >= 32;
+        const double pv = __shfl_sync(FULL, hi ? P[RPL - 1][t] : P[0][t], kr & 31);
+        double inv = __shfl_sync(FULL, hi ? rc[RPL - 1] : rc[0], kr & 31);
+        if (pv == 0.0) {   // no scaling
+            inv = 1.0;
+            if (lane == 0) atomicMin(zero, k);
+        }
+        place(k, kr, (int)pp);
+        double l[RPL];
+#pragma unroll
+        for (int s = 0; s < RPL; ++s) {
+            l[s] = P[s][t] * inv;
+            ex[k * BM + lane + 32 * s] = l[s];
+            if (act[s]) P[s][t] = l[s];
+        }
+        if (lane == 0) {
+            piv[k] = kr | (int)pp << 8;
+            rd[k] = inv;
+        }
+        if (q + 1 < nq) asm volatile("bar.arrive %0, %1;" ::"r"(4 + t), "r"(32 * (nq - q)) : "memory");
+#pragma unroll
+        for (int j = t + 1; j < LU_W; ++j) {
+            const double u = __shfl_sync(FULL, hi ? P[RPL - 1][j] : P[0][j], kr & 31);
+#pragma unroll
+            for (int s = 0; s < RPL; ++s)
+                if (act[s]) P[s][j] -= l[s] * u;
+        }
+    }
+    if (q == nq - 1)
+#pragma unroll
+        for (int s = 0; s < RPL; ++s)
+            if (lane + 32 * s < nrow) at[lane + 32 * s] = pos[s];
+    asm volatile("bar.sync 12, %0;" ::"r"(32 * nq) : "memory");   // (and every warp has read its columns)
+#pragma unroll
+    for (int s = 0; s < RPL; ++s) {
+        const int r = lane + 32 * s;
+        if (r < nrow)
+#pragma unroll
+            for (int j = 0; j < LU_W; ++j)
+                if (q * LU_W + j < w) A[(q * LU_W + j) * LD + (q * LU_W + j >= left[r] ? at[r] : r)] = P[s][j];
+    }
+}
+
+__global__ void __launch_bounds__(LU64_THREADS) k_block_lu_f64(double* fac, int* ipiv, int* info, Sched S, Launch L, int step) {
+    using SM = Lu64Smem;
+    constexpr int BM = SM::BM, LD = SM::LD, LT = SM::LT, NW = LU64_THREADS / 32;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double* sm = reinterpret_cast<double*>(smem_raw);
+    double *A = sm + SM::a, *ex = sm + SM::ex, *sT = sm + SM::t, *sL = sm + SM::l;
+    __shared__ double srd[LU_G];
+    __shared__ int cpa[BM], cpb[BM], spiv[BM];            // piece of each column, local pivot rows
+    __shared__ int spv[LU_G], sat[BM], slsrc[BM], sleft[BM], szero, zpiece;
+    int fid, tile;
+    locate(L, blockIdx.x, fid, tile);
+    const DFront F = S.fronts[fid];
+    const int blk = F.block0 + step;
+    const int c0 = S.blk_c0[blk], c1 = S.blk_c1[blk], bw = c1 - c0;
+    const int p0 = S.blk_p0[blk], np = S.blk_np[blk];
+    const int tid = threadIdx.x, wp = tid >> 5, lane = tid & 31;
+    const bool sym = S.sym != 0;
+    double* blkp = fac + F.loff + (ll)c0 * F.ld + c0;   // block (i, j) at blkp[j * ld + i]
+#pragma unroll
+    for (int x = 0; x < BM / NW; ++x)
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            const int C = wp + x * NW, R = lane + 32 * s;
+            if (C < bw && R < bw && (!sym || R >= C)) {
+                const double v = blkp[(ll)C * F.ld + R];
+                A[C * LD + R] = v;
+                if (sym) A[R * LD + C] = v;   // symmetric form: the upper triangle mirrors the lower one
+            }
+        }
+    for (int pc = tid; pc < np; pc += LU64_THREADS) {
+        const int a = S.xsuper[p0 + pc] - F.f - c0, b = S.xsuper[p0 + pc + 1] - F.f - c0;
+        for (int k = a; k < b; ++k) {
+            cpa[k] = a;
+            cpb[k] = b;
+        }
+    }
+    if (tid == 0) zpiece = INT_MAX;
+    __syncthreads();
+    for (int a = 0; a < bw;) {
+        // group [a, b): whole pieces of up to 32 columns, or a slice of a wider one; rows to e
+        int b = a;
+        while (b < bw && cpb[b] - a <= LU_G) b = cpb[b];
+        int e = b;
+        if (b == a) {
+            e = cpb[a];
+            b = a + LU_G;
+        }
+        const int w = b - a, nrow = e - a, nr = bw - b;
+        if (tid < nrow) sleft[tid] = max(cpa[a + tid] - a, 0);
+        if (tid == 0) szero = LU_G;
+        __syncthreads();
+        if (wp < cdiv(w, LU_W)) {
+            const int cend = lane < w ? cpb[a + lane] - a : 0;
+            if (nrow <= 32) lu64_sweep<1>(A + a * LD + a, nrow, w, cend, sleft, ex, srd, spv, sat, &szero, sym, wp);
+            else lu64_sweep<2>(A + a * LD + a, nrow, w, cend, sleft, ex, srd, spv, sat, &szero, sym, wp);
+        }
+        __syncthreads();
+        if (tid < nrow) slsrc[sat[tid]] = tid;
+        if (tid < w) spiv[a + tid] = a + (spv[tid] >> 8) - cpa[a + tid];
+        if (tid == 0 && szero < LU_G) zpiece = min(zpiece, a + szero);
+        __syncthreads();
+        // the interchanges over the columns right of the group, and over those of
+        // the first piece left of it when that is a slice (its rows only)
+        const int nleft = a - cpa[a];
+        for (int c = wp; c < nleft + nr; c += NW) {
+            double* col = A + (c < nleft ? cpa[a] + c : b + c - nleft) * LD + a;
+            const int lim = c < nleft ? cpb[a] - a : nrow;
+            const double v0 = lane < lim ? col[slsrc[lane]] : 0.0, v1 = lane + 32 < lim ? col[slsrc[lane + 32]] : 0.0;
+            __syncwarp();
+            if (lane < lim) col[lane] = v0;
+            if (lane + 32 < lim) col[lane + 32] = v1;
+        }
+        if (nr > 0) {
+            // U11 over its diagonal by rows, L11 by columns (as the rows eliminated: original rows' multipliers)
+            for (int t = tid; t < w * LU_G; t += LU64_THREADS) {
+                const int k = t / LU_G, j = t % LU_G;
+                sT[k * LT + j] = j > k && j < w ? A[(a + j) * LD + a + k] * srd[k] : 0.0;
+                sL[k * LT + j] = j > k && j < w ? ex[k * BM + slsrc[j]] : 0.0;
+            }
+            __syncthreads();
+            // L21 rows below e (warps 0 .. 3) and U12 columns (4 .. 7), eight lanes per line
+            const bool isU = wp >= 4;
+            const int q = lane & (PD_LANES - 1);
+            for (int x = (wp & 3) * 4 + lane / PD_LANES; x < cdiv(nr, 16) * 16; x += 16) {
+                const bool ok = x < nr && (isU || b + x >= e);
+                double* line = isU ? A + (b + min(x, nr - 1)) * LD + a : A + a * LD + b + min(x, nr - 1);
+                const int ls = isU ? 1 : LD;
+                double y[LU_G / PD_LANES];
+#pragma unroll
+                for (int jj = 0; jj < LU_G / PD_LANES; ++jj) {
+                    const int j = jj * PD_LANES + q;
+                    y[jj] = ok && j < w ? line[j * ls] : 0.0;
+                }
+                sweep_f64<LU_G>(y, isU ? sL : sT, w);
+#pragma unroll
+                for (int jj = 0; jj < LU_G / PD_LANES; ++jj) {
+                    const int j = jj * PD_LANES + q;
+                    if (ok && j < w) line[j * ls] = isU ? y[jj] : y[jj] * srd[j];
+                }
+            }
+            // a sliced piece's own later rows: their multipliers came out of the sweep in place
+            __syncthreads();
+            // A22 -= L21 U12: a lane per row, eight columns per warp and pass
+            for (int cq = wp; cq < cdiv(nr, 4); cq += NW)
+                for (int r = b + lane; r < b + cdiv(nr, 32) * 32; r += 32) {
+                    const bool ok = r < bw;
+                    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+                    for (int k = 0; k < w; ++k) {
+                        const double lv = ok ? A[(a + k) * LD + r] : 0.0;
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) acc[j] += lv * A[min(b + 4 * cq + j, bw - 1) * LD + a + k];
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (ok && b + 4 * cq + j < bw) A[(b + 4 * cq + j) * LD + r] -= acc[j];
+                }
+            __syncthreads();
+        }
+        a = b;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int x = 0; x < BM / NW; ++x)
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            const int C = wp + x * NW, R = lane + 32 * s;
+            if (C < bw && R < bw) blkp[(ll)C * F.ld + R] = A[C * LD + R];
+        }
+    if (tid < bw) ipiv[F.f + c0 + tid] = spiv[tid];
+    if (tid == 0 && zpiece != INT_MAX) {
+        int p = 0;
+        while (S.xsuper[p0 + p + 1] - F.f - c0 <= zpiece) ++p;
+        atomicMin(info, p0 + p + 1);   // first singular piece of the block
     }
 }
 

@@ -82,3 +82,28 @@ def test_spd_blocks(n):
         f = int(s.slvr.xsuper[s.slvr.snode[j] - 1]) - 1
         L[f:, j] = s.slvr.lnz[s.slvr.xlnz[j] - 1: s.slvr.xlnz[j + 1] - 1]
     assert rel(np.tril(L), C) <= 5e-5
+
+
+@pytest.mark.parametrize("n", [33, 63, 64, 65, 128, 150])
+@pytest.mark.parametrize("kind", ["dominant", "pivoting", "ties"])
+@pytest.mark.parametrize("maxblocksize", [30, 7, 48])
+def test_dense_blocks_fp64(kind, n, maxblocksize):
+    """FP64: eight times what a change of A by n u moves the oracle's factors by
+    (the growth of the elimination is below 8 of it: pivots limited to a piece
+    of at most 48 rows of matrices with a diagonal of sqrt(n) / 2)."""
+    A = sp.csc_matrix(dense(kind, n))
+    s = S.SparseSolver(A, maxblocksize=maxblocksize)
+    S.findorder_(s)
+    S.symbolicfactor_(s)
+    P = A.copy()
+    P.data *= 1.0 + n * 2.0 ** -53 * np.random.default_rng(1).uniform(-1.0, 1.0, P.nnz)
+    if kind == "ties":   # the perturbed copy keeps them
+        P[:, 0] = A[:, 0]
+    o, q = (oracle.OracleLU(s.slvr) for _ in range(2))
+    for orc, M in ((o, A), (q, sp.csc_matrix(P))):
+        orc.inmatrix_csc(*S.sparse_solver._matrix_arrays(M))
+        orc.factor()
+    S.inmatrix_(s)
+    S.factor_(s)
+    assert np.array_equal(s.slvr.ipiv, o.ipiv) and np.array_equal(q.ipiv, o.ipiv)
+    assert np.max(np.abs(s.slvr.lnz - o.lnz)) <= 8.0 * np.max(np.abs(q.lnz - o.lnz))
