@@ -333,8 +333,11 @@ int spk_measure_peaks(double* fp32_tflops, double* fp64_tflops, double* dmma_tfl
  *                        reference's operation order (ggetrf!, trsm, gemm
  *                        per supernode), hence FP64 factors closer to its
  *                        rounding, but a slower chain on GB300 (the piece's
- *                        column steps are as long as the block form's);
- *                        0 (default): every wide block in column groups.
+ *                        column steps are as long as the block form's).
+ *                        In FP64 the panels and the rank updates keep that
+ *                        order too (CUDA cores, no integer slices).
+ *                        0 (default): every wide block in groups of at most
+ *                        32 columns.
  *  SPK_OPT_SOLVE_CLUSTER_MINB  fronts of at least this many blocks (2..128,
  *                        default 4) are solved by one 16-CTA cluster each
  *                        (all block steps in one launch); smaller ones by a

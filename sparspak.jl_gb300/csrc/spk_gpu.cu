@@ -93,7 +93,8 @@ struct LevelPlan {
 constexpr int TC_SCHUR_M = 96, TC_TRAIL_ROWS = 128;
 // FP64 fronts whose rank updates go to the tensor cores as integer slices
 // (k_oz_update): at least OZ_MIN rows below the front, or below its first
-// block when it has several.
+// block when it has several; none in the reference's operation order
+// (SPK_OPT_LU_PIECES).
 constexpr int OZ_MIN = 128;
 // Polls of a bounded device wait (the leaf queue's dependency waits) before
 // it gives up and records a timeout.
@@ -644,7 +645,9 @@ static void add_launch(Plan* h, LaunchRec& rec, const std::vector<int>& ids, con
 
 // Lines per panel tile: the 128-wide FP32 form (a launch with a block wider
 // than 64 columns) takes spk::PT_LINES, the others 64.
-static int panel_lines(bool fp32, bool wide) { return !fp32 ? spk::PD_LINES : wide ? spk::PT_LINES : 64; }
+static int panel_lines(bool fp32, bool wide, bool pieces) {
+    return !fp32 ? (pieces ? 64 : spk::PD_LINES) : wide ? spk::PT_LINES : 64;
+}
 
 // Group each front's pieces into blocks of at most `bmax` columns and lay
 // out the launches of every level.
@@ -686,7 +689,7 @@ static void build_plan(const spk_handle* h, Plan& P, int bmax, bool tc, bool sym
             const HFront& F = h->fronts[i];
             const int b0 = P.block0[i], nb = P.nblocks[i];
             const bool packed = tc ? F.m >= h->tc_schur_m || (nb > 1 && F.nf + F.m - P.blk_c1[b0] >= h->tc_trail_rows)
-                                   : F.m >= OZ_MIN || (nb > 1 && F.nf + F.m - P.blk_c1[b0] >= OZ_MIN);
+                                   : !h->lu_pieces && (F.m >= OZ_MIN || (nb > 1 && F.nf + F.m - P.blk_c1[b0] >= OZ_MIN));
             if (!packed) continue;
             const int n2 = cdiv(F.m, spk::umma::TM);
             for (int b = b0; b < b0 + nb; ++b) {
@@ -887,7 +890,7 @@ static void build_plan(const spk_handle* h, Plan& P, int bmax, bool tc, bool sym
                 tl[k] = leafF[k] ? 0 : 1;
                 fl[k] = 2.0 * bw * bw * bw;
                 wl[k] = 2.0 * bw * bw + 2.0 * bw;   // the block read and written once, its pivots and row sources
-                const int lpt = panel_lines(tc, wide[t]);
+                const int lpt = panel_lines(tc, wide[t], h->lu_pieces);
                 // the SPD form launches the L-panel tiles only (they also write the U side)
                 tp[k] = leafF[k] ? 0 : cdiv(ld - c1, lpt) + (sym ? 0 : cdiv(F.nf - c1, lpt) + cdiv(F.m, lpt));
                 const double rowsL = ld - c1, colsU = (double)(F.nf - c1) + F.m;
@@ -938,7 +941,7 @@ static void build_plan(const spk_handle* h, Plan& P, int bmax, bool tc, bool sym
                     fn[k] = wn[k] = ffar[k] = wfar[k] = 0.0;
                     if (tp[k] <= 0) continue;
                     const HFront& F = h->fronts[ids[k]];
-                    const int c1 = P.blk_c1[P.block0[ids[k]] + t], lpt = panel_lines(tc, wide[t]);
+                    const int c1 = P.blk_c1[P.block0[ids[k]] + t], lpt = panel_lines(tc, wide[t], h->lu_pieces);
                     tn[k] = std::min(2, cdiv(F.nf + F.m - c1, lpt)) + (sym ? 0 : std::min(2, cdiv(F.nf - c1, lpt)));
                     tfar[k] = tp[k] - tn[k];
                     const double a = (double)tn[k] / tp[k];
@@ -1158,9 +1161,8 @@ static int ensure_plan(spk_handle* h) {
     S.blk_upack = P.d_blk_upack;
     S.sym = P.sym ? 1 : 0;
     constexpr int BM = spk::BlockMax<T>::value;
-    if constexpr (std::is_same<T, float>::value)
-        CU(h, cudaFuncSetAttribute(spk::k_block_panel<T, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)panel_smem<T, BM>()));
+    CU(h, cudaFuncSetAttribute(spk::k_block_panel<T, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)panel_smem<T, BM>()));
     CU(h, cudaFuncSetAttribute(spk::k_block_lu_pc<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)spk::PcLu<T>::smem));
     CU(h, cudaFuncSetAttribute(spk::k_block_inv<T, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1477,11 +1479,14 @@ static int factor_launches(spk_handle* h, int fs_nrhs = 0) {
                 if (rec.tiles <= 0) return;
                 LaunchScope ls(h, SPK_K_PANEL, rec.flops, rec.words * sizeof(T));
                 const spk::Launch la = launch_of(PL, rec);
-                if constexpr (std::is_same<T, double>::value) {
-                    if (bw <= 32)
-                        spk::k_block_panel_f64<32><<<rec.tiles, 128, panel64_smem<32>(), st>>>(fac, h->d_ipiv, S, la, (int)t, h->d_rexp);
-                    else
-                        spk::k_block_panel_f64<64><<<rec.tiles, 128, panel64_smem<64>(), st>>>(fac, h->d_ipiv, S, la, (int)t, h->d_rexp);
+                constexpr bool f64 = std::is_same<T, double>::value;
+                if (f64 && !h->lu_pieces) {   // eight lanes per line; the piece form keeps the reference's order
+                    if constexpr (f64) {
+                        if (bw <= 32)
+                            spk::k_block_panel_f64<32><<<rec.tiles, 128, panel64_smem<32>(), st>>>(fac, h->d_ipiv, S, la, (int)t, h->d_rexp);
+                        else
+                            spk::k_block_panel_f64<64><<<rec.tiles, 128, panel64_smem<64>(), st>>>(fac, h->d_ipiv, S, la, (int)t, h->d_rexp);
+                    }
                 } else if (bw <= 32)
                     spk::k_block_panel<T, 32><<<rec.tiles, 256, sweep_smem<T, 32>(1), st>>>(
                         fac, h->d_ipiv, h->d_bmap, S, la, (int)t, storage<T>(h).pack, bf16, part);
@@ -2359,8 +2364,10 @@ int spk_set_option(spk_handle* h, int option, int64_t value) {
         return SPK_OK;
     case SPK_OPT_LU_PIECES:
         if (value != 0 && value != 1) break;
-        h->lu_pieces = (int)value;
-        drop_factor_graphs(h);
+        if (h->lu_pieces != (int)value) {   // FP64: another panel form, no slices
+            h->lu_pieces = (int)value;
+            reset_plans_keep_factors(h);
+        }
         return SPK_OK;
     case SPK_OPT_PANEL_SPLIT:
         if (value != 0 && value != 1) break;
