@@ -3362,12 +3362,17 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc_update(float* fac, const u
 // an infinity or a NaN, and a product whose scale leaves the exponent range,
 // take a plain FP64 sum over the stored factor instead.
 //   Tiles of 128 x 32: eight weights of 32 columns are 256 TMEM columns,
-// double-buffered.  What bounds it: an MMA of 128 rows takes 95 cycles up to 64
-// columns, so a 128 x 32 x 64 product is 144 x 95 = 13,700 cycles, beside
-// the epilogue's FP64 work (two conversions and two multiply-adds per entry, 9,000
-// cycles) and its loads; 15,000 cycles measured, 11 TFLOP/s on a 4096 x 4096 x 64
-// update where the multiply-add tiles give 1.05.  48^3 convection-diffusion,
-// rank updates: 131 -> 23 ms.
+// double-buffered.  Digit i of L meets digits 0 .. 7 - i of U in one MMA of
+// 32 (8 - i) columns, whose products are weights i .. 7: eight MMAs per 16
+// columns where one per pair was 36, of 95 cycles each up to 64 columns.  The
+// weights are joined and rounded by integer instructions (oz_join).  What
+// bounds it now is latency, no pipe is above a third: a tile's chain of copies
+// (160 KB), accumulator loads, joins and target accesses, 13,900 cycles per
+// 128 x 32 x 64 product; 12 TFLOP/s on a 4096 x 4096 x 64 update where the
+// multiply-add tiles give 1.05.  48^3 convection-diffusion, rank updates:
+// 131 -> 20.3 ms (23.5 with an MMA per pair and FP64 joins).  Two groups of
+// epilogue warps on alternate tiles, and eight warps with twice the registers,
+// took 21.1 and 22.4 ms.
 // ---------------------------------------------------------------------------
 constexpr int OZ_D = 8, OZ_N = 32;                       // digits, tile columns
 constexpr int OZ_SLICE = umma::PCHUNK16;                 // one slice of a 128-line tile and 16 columns, 4 KB
@@ -3556,6 +3561,38 @@ __device__ __forceinline__ void oz_lines(const Sched& S, const OzTile& T, int b,
     }
 }
 
+// The product from its weights (0 .. 4 joined in units of 2^E, 5 .. 7 of
+// 2^(E - 24); 76 bits at most), rounded once to nearest; SIGN flips it.  By
+// integer instructions: a conversion or an addition in FP64 costs a quarter of
+// the SM 64 cycles and more, and the form with both takes four of them.
+__device__ __forceinline__ double oz_join(const int (&n)[OZ_D], int E, long long SIGN) {
+    // |weight w| <= 2^20 (w + 1)
+    const long long hi = ((long long)(n[0] * 256 + n[1]) << 24) + ((long long)n[2] << 16) + (n[3] * 256 + n[4]);
+    const long long lo = ((long long)n[5] << 16) + (n[6] * 256 + n[7]);
+    // 96 bits, units of 2^(E - 10) and 2^(E - 42): below 2^63 of the former
+    const long long top = (hi << 10) + (lo >> 14);
+    const unsigned frac = (unsigned)lo << 18;
+    const long long neg = top >> 63;
+    const unsigned long long a = (unsigned long long)(top ^ neg) + (neg && frac == 0);
+    const unsigned fr = (frac ^ (unsigned)neg) - (unsigned)neg;
+    const int z = __clzll((long long)a);
+    if (z > 43) {   // small after cancellation, or zero
+        const double v = fma((double)lo, __longlong_as_double((long long)(E - 24 + 1023) << 52),
+                             (double)hi * __longlong_as_double((long long)(E + 1023) << 52));
+        return SIGN ? -v : v;
+    }
+    unsigned w2 = (unsigned)(a >> 32), w1 = (unsigned)a, w0 = fr;
+    if (z >= 32) {
+        w2 = w1;
+        w1 = w0;
+        w0 = 0;
+    }
+    w2 = __funnelshift_l(w1, w2, z);   // the leading 64 bits; ties away from zero
+    w1 = __funnelshift_l(w0, w1, z);
+    const unsigned long long m = (((unsigned long long)w2 << 32 | w1) >> 11) + ((w1 >> 10) & 1u);
+    return __longlong_as_double((((long long)(E + 1075 - z) << 52) + (long long)m) ^ (neg & (long long)(1ull << 63)) ^ SIGN);
+}
+
 // Sum over block b of L(row, k) U(k, col), plain FP64 (front-local row; col
 // of the front, or nf + the U12 column).
 __device__ __noinline__ double oz_plain(const double* fac, const Sched& S, const DFront& F, int b, int row, int col) {
@@ -3636,7 +3673,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_update(double* fac, unsign
         }
     } else if (warp == 1) {
         if (lane == 0) {   // MMAs
-            constexpr uint32_t IDESC = umma::idesc_bf16(umma::TM, OZ_N);
             int s = 0, acc = 0;
             uint32_t ph = 0, aph = 0;
             OzTile T;
@@ -3652,13 +3688,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_update(double* fac, unsign
                         const uint32_t a0 = umma::saddr(stage + s * OZ_STAGE), b0 = a0 + OZ_CHUNK;
                         const uint64_t da = umma::desc_kmajor(a0, 128, umma::SBO16), db = umma::desc_kmajor(b0, 128, umma::SBO16);
                         const uint32_t d0 = tmem + acc * (OZ_D * OZ_N);
-                        // weight w: digit pairs i + j = w (descriptors hold addresses in 16-byte units)
+                        // digit i of L with digits 0 .. 7 - i of U, whose lines follow one another: weights
+                        // i .. 7 (descriptors hold addresses in 16-byte units)
 #pragma unroll
-                        for (int w = 0; w < OZ_D; ++w)
-#pragma unroll
-                            for (int i = 0; i <= w; ++i)
-                                umma::mma_bf16(d0 + w * OZ_N, da + i * (OZ_SLICE >> 4), db + (w - i) * (OZ_SUB >> 4), IDESC,
-                                               c > 0 || i > 0 ? 1u : 0u);
+                        for (int i = 0; i < OZ_D; ++i)
+                            umma::mma_bf16(d0 + i * OZ_N, da + i * (OZ_SLICE >> 4), db,
+                                           umma::idesc_bf16(umma::TM, (OZ_D - i) * OZ_N), c > 0 || i > 0 ? 1u : 0u);
                         umma::commit(&empty[s]);
                         if (++s == OZ_NST) { s = 0; ph ^= 1; }
                     }
@@ -3723,14 +3758,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_update(double* fac, unsign
                         int n[OZ_D];
 #pragma unroll
                         for (int w = 0; w < OZ_D; ++w) n[w] = __float2int_rn(v[w][j]);
-                        // weights 0..4 in units of 2^-44, 5..7 in units of 2^-68
-                        const long long hi = ((long long)(n[0] * 256 + n[1]) << 24) + ((long long)n[2] << 16) + (n[3] * 256 + n[4]);
-                        const long long lo = ((long long)n[5] << 16) + (n[6] * 256 + n[7]);
                         const int f = fj[4 * h + j], E = ei + f - 44;
                         double& s = sum[4 * h + j];
                         if (E - 24 > -1022 && E < 960) {
-                            s = fma((double)lo, __longlong_as_double((long long)(E - 24 + 1023) << 52 | SIGN), s);
-                            s = fma((double)hi, __longlong_as_double((long long)(E + 1023) << 52 | SIGN), s);
+                            s += oz_join(n, E, SIGN);
                         } else if (row < rend && col0 + 4 * h + j < cend) {
                             const double v = oz_plain(fac, S, F, b, row, col0 + 4 * h + j);
                             s += MODE == TC_TRAIL ? -v : v;
