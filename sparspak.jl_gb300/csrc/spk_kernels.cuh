@@ -3942,6 +3942,13 @@ __global__ void __launch_bounds__(TS) k_fwd(const T* fac, const T* inv2, T* b, T
     }
 }
 
+// First right-hand side of this CTA's groups of RG (grid y).  A single
+// right-hand side has no groups: its one pass starts without a barrier, which
+// would hold back the factor loads (backward solves of a 48^3 step 3.1 ms, with
+// a barrier 3.6).
+template <int RG>
+__device__ __forceinline__ unsigned group0() { return RG == 1 ? 0u : blockIdx.y * RG; }
+
 // Products y[F.f + k] -= dot(line k, x[R_F]) over the lines of a front's
 // off-diagonal part (U12 rows for the backward solve, L21 columns for the
 // transposed one; line k at base + k * stride, F.m values, contiguous).  A
@@ -3961,9 +3968,9 @@ __device__ __forceinline__ void front_line_dots(const T* base, ll stride, T* y, 
     const int ncc = cdiv(F.m, U12_COLS);
     const int i0 = (tile / ncc) * U12_ROWS + wid, c0 = (tile % ncc) * U12_COLS;
     const int nc = min(U12_COLS, F.m - c0);
-    for (int r0 = blockIdx.y * RG; r0 < nrhs; r0 += gridDim.y * RG) {
+    for (int r0 = group0<RG>(); r0 < nrhs; r0 += gridDim.y * RG) {
         const int nr = min(RG, nrhs - r0);
-        __syncthreads();
+        if (RG > 1 || r0 > 0) __syncthreads();
         for (int c = threadIdx.x; c < nc; c += 256) {
             const int g = rows[c0 + c];
 #pragma unroll
@@ -4303,7 +4310,7 @@ __global__ void __cluster_dims__(NC, 1, 1) __launch_bounds__(FC_THREADS, 1)
             }
         }
     };
-    for (int r0 = blockIdx.y * RG; r0 < nrhs; r0 += gridDim.y * RG) {
+    for (int r0 = group0<RG>(); r0 < nrhs; r0 += gridDim.y * RG) {
         const int nr = min(RG, nrhs - r0);
         prefetch(rank);
         for (int st = rank, o = 0; st < nb; st += FC, ++o) {   // the owned blocks' right-hand sides
@@ -4575,9 +4582,9 @@ __global__ void __launch_bounds__(256) k_fwd_l21(const T* fac, T* b, const T* y,
     const ll sk = TRANS ? F.m : F.ld;
     const T* a = fac + (TRANS ? F.uoff : F.loff + F.nf) + k0 * sk + (ok ? i : 0);
     griddep_wait();
-    for (int r0 = blockIdx.y * RG; r0 < nrhs; r0 += gridDim.y * RG) {
+    for (int r0 = group0<RG>(); r0 < nrhs; r0 += gridDim.y * RG) {
         const int nr = min(RG, nrhs - r0);
-        __syncthreads();
+        if (RG > 1 || r0 > 0) __syncthreads();
         for (int e = threadIdx.x; e < L21_COLS * RG; e += blockDim.x) {
             const int k = e % L21_COLS, r = e / L21_COLS;
             sy[e] = (k < nk && r < nr) ? y[(ll)(r0 + r) * n + F.f + k0 + k] : T(0);
@@ -4617,9 +4624,9 @@ __global__ void __launch_bounds__(256) k_front_gemv(const T* fac, T* out, const 
     const int nk = min(L21_COLS, c1 - k0), i = i0 + threadIdx.x;
     const bool ok = i < r1;
     const T* a = fac + loff + (ll)k0 * ld + (ok ? i : 0);
-    for (int q0 = blockIdx.y * RG; q0 < nrhs; q0 += gridDim.y * RG) {
+    for (int q0 = group0<RG>(); q0 < nrhs; q0 += gridDim.y * RG) {
         const int nr = min(RG, nrhs - q0);
-        __syncthreads();
+        if (RG > 1 || q0 > 0) __syncthreads();
         for (int e = threadIdx.x; e < L21_COLS * RG; e += blockDim.x) {
             const int k = e % L21_COLS, r = e / L21_COLS;
             sv[e] = (k < nk && r < nr) ? in[(ll)(q0 + r) * n + f + k0 + k] : T(0);
@@ -4650,7 +4657,7 @@ template <typename T, int RG>
 __global__ void __launch_bounds__(256) k_front_gemv_t(const T* fac, T* out, const T* in, int n, int nrhs, ll loff, int ld, int f,
                                                       int r0, int r1, int c0, int c1) {
     const int lane = threadIdx.x & 31, i0 = r0 + (int)blockIdx.x * GT_ROWS + (int)(threadIdx.x >> 5) * 4;
-    for (int q0 = blockIdx.y * RG; q0 < nrhs; q0 += gridDim.y * RG) {
+    for (int q0 = group0<RG>(); q0 < nrhs; q0 += gridDim.y * RG) {
         T acc[4 * RG];
 #pragma unroll
         for (int e = 0; e < 4 * RG; ++e) acc[e] = T(0);
