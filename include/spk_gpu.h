@@ -45,7 +45,10 @@ extern "C" {
 #define SPK_HOST 0
 #define SPK_DEVICE 1
 
-#define SPK_FP64 0         /* factor, solve and residual in double                */
+#define SPK_FP64 0         /* factor, solve and residual in double; the large
+                              rank updates as exact integer slices on the
+                              tensor cores where memory for them (twice the
+                              factor's) is free, else double multiply-adds      */
 #define SPK_FP32 1         /* factor and solve in float; residual and correction
                               in double (mixed form for spk_refine); the large
                               rank updates as 3xTF32 tensor-core products        */

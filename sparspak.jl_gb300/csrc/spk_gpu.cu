@@ -190,7 +190,7 @@ struct spk_handle {
         *d_rel = nullptr;
     ll* d_run_rel = nullptr;
     int* d_ipiv = nullptr;
-    int* d_bmap = nullptr;     // row sources of each block's interchanges (k_block_lu -> panels)
+    int* d_bmap = nullptr;     // row sources of each block's interchanges (k_block_lu_f32 -> panels)
     int* d_rexp = nullptr;     // FP64: exponent field of each U row's largest panel entry (panels -> k_oz_pack)
     int* d_info = nullptr;
 
@@ -247,6 +247,7 @@ struct spk_handle {
     int stall_test = -1;                   // SPK_OPT_STALL_TEST
     int tc_schur_m = TC_SCHUR_M, tc_trail_rows = TC_TRAIL_ROWS;
     int tc_wide = 1;                       // SPK_OPT_TC_WIDE: Schur tiles of 128 x 256
+    bool no_slices = false;                // FP64: the slices' pack did not fit
     int lu_pieces = 0;                     // SPK_OPT_LU_PIECES: block LU by pieces (slower on GB300, see header)
     int fc_minb = spk::FC_MINB;            // SPK_OPT_SOLVE_CLUSTER_MINB: blocks of a front for the cluster solve
     int panel_split = 1;                   // SPK_OPT_PANEL_SPLIT: near / far panel tiles on two streams
@@ -689,7 +690,7 @@ static void build_plan(const spk_handle* h, Plan& P, int bmax, bool tc, bool sym
             const HFront& F = h->fronts[i];
             const int b0 = P.block0[i], nb = P.nblocks[i];
             const bool packed = tc ? F.m >= h->tc_schur_m || (nb > 1 && F.nf + F.m - P.blk_c1[b0] >= h->tc_trail_rows)
-                                   : !h->lu_pieces && (F.m >= OZ_MIN || (nb > 1 && F.nf + F.m - P.blk_c1[b0] >= OZ_MIN));
+                                   : !h->lu_pieces && !h->no_slices && (F.m >= OZ_MIN || (nb > 1 && F.nf + F.m - P.blk_c1[b0] >= OZ_MIN));
             if (!packed) continue;
             const int n2 = cdiv(F.m, spk::umma::TM);
             for (int b = b0; b < b0 + nb; ++b) {
@@ -1237,7 +1238,25 @@ static int ensure_storage(spk_handle* h) {
     if (!S.inv2) CU(h, cudaMalloc((void**)&S.inv2, sizeof(T) * std::max<ll>(h->plan[plan_index<T>(h)].inv2_size, 1)));
     // BF16 packs take a quarter of the TF32 hi + lo bytes (same tiles and chunks)
     const ll pack_bytes = h->plan[plan_index<T>(h)].pack_size / (std::is_same<T, float>::value && h->fmode ? 4 : 1);
-    if (!S.pack && pack_bytes > 0) CU(h, cudaMalloc((void**)&S.pack, (size_t)pack_bytes));
+    if (!S.pack && pack_bytes > 0) {
+        // The FP64 slices (twice the factor) are taken only where as much memory
+        // as the factor itself stays free: the CUDA-core updates need none.
+        cudaError_t e = cudaSuccess;
+        if (std::is_same<T, double>::value) {
+            size_t avail = 0, all = 0;
+            CU(h, cudaMemGetInfo(&avail, &all));
+            if ((size_t)pack_bytes + sizeof(T) * (size_t)h->fsize > avail) e = cudaErrorMemoryAllocation;
+        }
+        if (e == cudaSuccess) e = cudaMalloc((void**)&S.pack, (size_t)pack_bytes);
+        if (e == cudaErrorMemoryAllocation && std::is_same<T, double>::value) {
+            cudaGetLastError();
+            S.pack = nullptr;
+            h->no_slices = true;
+            free_plan(h->plan[plan_index<T>(h)]);
+            return ensure_plan<T>(h);
+        }
+        CU(h, e);
+    }
     return SPK_OK;
 }
 
