@@ -76,13 +76,14 @@ SPK_HOST, SPK_DEVICE = 0, 1
 KERNEL_CLASSES = ["assemble", "getrf", "panel", "trail", "schur", "fwd", "bwd", "permute", "residual", "blockinv",
                   "tc_trail", "tc_schur"]
 KERNEL_NAMES = {"assemble": "k_scatter_values",
-                "getrf": "k_block_lu_pc+k_block_lu+k_block_lu_small+k_leaf_factor+k_leaf_queue",
-                "panel": "k_block_panel",
+                "getrf": "k_block_lu_pc+k_block_lu_f32+k_block_lu_f64+k_block_lu_small+k_leaf_factor+k_leaf_queue",
+                "panel": "k_block_panel+k_block_panel_f64+k_oz_pack",
                 "trail": "k_block_trail", "schur": "k_schur",
                 "fwd": "k_fwd+k_front_solve<fwd>+k_fwd_l21+k_solve_leaf<fwd>",
                 "bwd": "k_bwd_u12+k_bwd+k_front_solve<bwd>+k_solve_leaf<bwd>", "permute": "k_permute+k_unpermute",
                 "residual": "k_residual", "blockinv": "k_block_inv",
-                "tc_trail": "k_tc_update<TC_TRAIL>", "tc_schur": "k_tc_update<TC_SCHUR>"}
+                "tc_trail": "k_tc_update<TC_TRAIL>+k_oz_update<TC_TRAIL>",
+                "tc_schur": "k_tc_update<TC_SCHUR>+k_oz_update<TC_SCHUR>"}
 # How each class's FP32 form computes: tensor cores (tcgen05, 3xTF32) or CUDA cores.
 KERNEL_UNITS = {"tc_trail": "tcgen05 kind::tf32, 3xTF32 per term", "tc_schur": "tcgen05 kind::tf32, 3xTF32 per term",
                 "trail": "FP32/FP64 FMA (fronts without a pack)", "schur": "FP32/FP64 FMA (fronts without a pack)",
