@@ -1364,6 +1364,7 @@ static int factor_launches(spk_handle* h, int fs_nrhs = 0) {
     T* fac = storage<T>(h).d;
     const Plan& PL = h->plan[plan_index<T>(h)];
     const spk::Sched& S = PL.sched;
+    if (PL.pack_size > 0 && !storage<T>(h).pack) return set_err(h, SPK_ESTRUCT, "the plan's packed panels are not allocated");
     // Look ahead (not while timing kernels one by one): see spk_handle::side.
     const bool ahead = h->prof_mask == 0;
     const int bf16 = std::is_same<T, float>::value ? h->fmode : 0;
@@ -1634,7 +1635,7 @@ static int factor_launches(spk_handle* h, int fs_nrhs = 0) {
 template <typename T>
 static int run_factor(spk_handle* h) {
     static const int init[3] = {INT_MAX, 0, 0};
-    int rc = ensure_plan<T>(h);   // rebuilt after an option dropped it
+    int rc = ensure_storage<T>(h);   // an option may have dropped the plan, and the new one may need a pack
     if (rc) return rc;
     CU(h, cudaMemcpyAsync(h->d_info, init, sizeof(init), cudaMemcpyHostToDevice, h->stream));
     return via_graph(h, h->g_factor[graph_index<T>(h)], [&] { return factor_launches<T>(h); });
@@ -2784,7 +2785,7 @@ int spk_refine_ex(spk_handle* h, const double* b, double* x, int64_t nrhs, int64
 template <typename T>
 static int factor_refine_first(spk_handle* h, int nrhs, double* dx, i64 ldx, int64_t* first_singular) {
     static const int init[3] = {INT_MAX, 0, 0};
-    int rc = ensure_plan<T>(h);
+    int rc = ensure_storage<T>(h);
     if (rc) return rc;
     CU(h, cudaMemcpyAsync(h->d_info, init, sizeof(init), cudaMemcpyHostToDevice, h->stream));
     const int gi = graph_index<T>(h);

@@ -1,0 +1,59 @@
+"""Memory of the FP64 slices (packed panels of the tensor-core rank updates):
+allocated whenever the plan in use has them, in whatever order the options,
+the values and the factorisation come.
+
+Tolerance: 1e-10 against the oracle's solution and 1e-12 for the residual, as
+the other solution tests on these grids.
+"""
+import numpy as np
+import pytest
+
+import oracle
+import sparspak as S
+from sparspak.sparse_solver import _ensure_engine, _inmatrix_, _matrix_arrays
+
+pytestmark = pytest.mark.gpu
+
+SIDE = 14   # a grid whose upper fronts take the slices
+
+
+def system():
+    A = S.gallery.convection_diffusion(k=SIDE)
+    s = S.SparseSolver(A)
+    S.findorder_(s, S.nd_grid(SIDE, SIDE, SIDE))
+    S.symbolicfactor_(s)
+    b = S.gallery.random_rhs(A.shape[0], 2, seed=1)
+    return s, A, b
+
+
+def check(s, A, b, x):
+    o = oracle.OracleLU(s.slvr)
+    o.inmatrix_csc(*_matrix_arrays(A))
+    assert o.factor() == 0
+    xo = o.solve(b)
+    assert np.max(np.abs(x - xo)) <= 1e-10 * np.max(np.abs(xo))
+    assert np.max(np.linalg.norm(b - A @ x, axis=0) / np.linalg.norm(b, axis=0)) <= 1e-12
+
+
+def slices(eng):
+    p = eng.profile_read()
+    return p["tc_trail"]["launches"] + p["tc_schur"]["launches"] > 0
+
+
+@pytest.mark.parametrize("fused", [False, True])
+def test_option_switched_back_between_load_and_factor(fused):
+    # the values' first assembly is under a plan without slices, their factorisation under one with them
+    s, A, b = system()
+    eng = _ensure_engine(s.slvr)
+    eng.set_option("lu_pieces", 1)
+    _inmatrix_(s.slvr, A)
+    eng.set_option("lu_pieces", 0)
+    eng.profile_reset()
+    x = np.zeros_like(b, order="F")
+    if fused:
+        eng.factor_refine(b, x, "fp64")
+    else:
+        eng.factor("fp64")
+        x = eng.solve(np.array(b, order="F"), "fp64")
+    assert slices(eng)
+    check(s, A, b, x)
