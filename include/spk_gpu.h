@@ -373,6 +373,14 @@ int spk_measure_peaks(double* fp32_tflops, double* fp64_tflops, double* dmma_tfl
  *                        the L rows below a chunk, backward the U rows
  *                        above it); 0: one cluster launch.  Keeps the
  *                        factors.
+ *  SPK_OPT_SLICE_LIMIT   bytes that the integer slices of an FP64 form's rank
+ *                        updates may take (-1, the default: what is free, as
+ *                        long as the factor's size stays free beside them; 0:
+ *                        none, the rank updates on the CUDA cores).  Where
+ *                        they do not fit when a factorisation is prepared it
+ *                        goes without, and the next one asks again; the
+ *                        launches of the classes SPK_K_TC_TRAIL and
+ *                        SPK_K_TC_SCHUR tell which it was.  Keeps the factors.
  */
 #define SPK_OPT_LEAF_QUEUE 0
 #define SPK_OPT_WAIT_BUDGET 1
@@ -386,6 +394,7 @@ int spk_measure_peaks(double* fp32_tflops, double* fp64_tflops, double* dmma_tfl
 #define SPK_OPT_SCHUR_SPLIT 9
 #define SPK_OPT_SCHUR_FAR_SMS 10
 #define SPK_OPT_SOLVE_CHUNK 11
+#define SPK_OPT_SLICE_LIMIT 12
 int spk_set_option(spk_handle* h, int option, int64_t value);
 int spk_get_option(spk_handle* h, int option, int64_t* value);
 

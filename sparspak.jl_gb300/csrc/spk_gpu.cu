@@ -158,7 +158,9 @@ template <typename T>
 struct Storage {
     T* d = nullptr;
     T* inv2 = nullptr;      // whole-block forward / backward operators
-    unsigned char* pack = nullptr;   // packed panels of the tensor-core fronts (FP32)
+    unsigned char* pack = nullptr;   // packed panels of the tensor-core fronts (FP64: integer slices)
+    ll slice_bytes = 0;     // FP64: what the slices take; no_slices: refused when last asked for
+    bool no_slices = false;
     bool loaded = false;    // values assembled since the last factor
     bool factored = false;
 };
@@ -247,7 +249,7 @@ struct spk_handle {
     int stall_test = -1;                   // SPK_OPT_STALL_TEST
     int tc_schur_m = TC_SCHUR_M, tc_trail_rows = TC_TRAIL_ROWS;
     int tc_wide = 1;                       // SPK_OPT_TC_WIDE: Schur tiles of 128 x 256
-    bool no_slices = false;                // FP64: the slices' pack did not fit
+    long long slice_limit = -1;            // SPK_OPT_SLICE_LIMIT: bytes of an FP64 form's slices at most
     int lu_pieces = 0;                     // SPK_OPT_LU_PIECES: block LU by pieces (slower on GB300, see header)
     int fc_minb = spk::FC_MINB;            // SPK_OPT_SOLVE_CLUSTER_MINB: blocks of a front for the cluster solve
     int panel_split = 1;                   // SPK_OPT_PANEL_SPLIT: near / far panel tiles on two streams
@@ -690,7 +692,7 @@ static void build_plan(const spk_handle* h, Plan& P, int bmax, bool tc, bool sym
             const HFront& F = h->fronts[i];
             const int b0 = P.block0[i], nb = P.nblocks[i];
             const bool packed = tc ? F.m >= h->tc_schur_m || (nb > 1 && F.nf + F.m - P.blk_c1[b0] >= h->tc_trail_rows)
-                                   : !h->lu_pieces && !h->no_slices && (F.m >= OZ_MIN || (nb > 1 && F.nf + F.m - P.blk_c1[b0] >= OZ_MIN));
+                                   : !h->lu_pieces && !h->s64[sym].no_slices && (F.m >= OZ_MIN || (nb > 1 && F.nf + F.m - P.blk_c1[b0] >= OZ_MIN));
             if (!packed) continue;
             const int n2 = cdiv(F.m, spk::umma::TM);
             for (int b = b0; b < b0 + nb; ++b) {
@@ -1092,10 +1094,20 @@ static int prepare_front_solve(spk_handle* h) {
     return SPK_OK;
 }
 
+static void free_plan(Plan& P) {
+    void* ptrs[] = {P.d_fronts,     P.d_blk_c0,      P.d_blk_c1,   P.d_blk_p0,     P.d_blk_np,    P.d_blk_inv2,
+                    P.d_blk_lpack,  P.d_blk_upack,   P.d_blk_front, P.d_inv_ids,   P.d_sched_ids, P.d_sched_prefix,
+                    P.d_q_order,    P.d_q_parent,    P.d_q_deps0,  P.d_q_deps,     P.d_q_next};
+    for (void* q : ptrs)
+        if (q) cudaFree(q);
+    P = Plan();
+}
+
 template <typename T>
 static int ensure_plan(spk_handle* h) {
     Plan& P = h->plan[plan_index<T>(h)];
     if (P.built) return SPK_OK;
+    free_plan(P);   // of an attempt that ran out of memory
     try {
         build_plan(h, P, spk::BlockMax<T>::value, std::is_same<T, float>::value, h->sym != 0);
     } catch (const std::bad_alloc&) {
@@ -1213,15 +1225,6 @@ static int ensure_plan(spk_handle* h) {
     return SPK_OK;
 }
 
-static void free_plan(Plan& P) {
-    void* ptrs[] = {P.d_fronts,     P.d_blk_c0,      P.d_blk_c1,   P.d_blk_p0,     P.d_blk_np,    P.d_blk_inv2,
-                    P.d_blk_lpack,  P.d_blk_upack,   P.d_blk_front, P.d_inv_ids,   P.d_sched_ids, P.d_sched_prefix,
-                    P.d_q_order,    P.d_q_parent,    P.d_q_deps0,  P.d_q_deps,     P.d_q_next};
-    for (void* q : ptrs)
-        if (q) cudaFree(q);
-    P = Plan();
-}
-
 template <typename T>
 static Storage<T>& storage(spk_handle* h);
 template <>
@@ -1229,30 +1232,46 @@ Storage<double>& storage<double>(spk_handle* h) { return h->s64[h->sym]; }
 template <>
 Storage<float>& storage<float>(spk_handle* h) { return h->fmode ? h->s16[h->sym] : h->s32[h->sym]; }
 
+// Drop a plan with every captured graph (they hold its device arrays).
+static void drop_plan(spk_handle* h, Plan& P) {
+    drop_factor_graphs(h);
+    drop_solve_graphs(h);
+    free_plan(P);
+}
+
+// The FP64 slices (about twice the factor) are taken only where as much memory
+// as the factor itself stays free, and within SPK_OPT_SLICE_LIMIT: the
+// CUDA-core updates need none.
+static bool slices_fit(spk_handle* h, ll bytes) {
+    if (h->slice_limit >= 0 && bytes > h->slice_limit) return false;
+    size_t avail = 0, all = 0;
+    if (cudaMemGetInfo(&avail, &all) != cudaSuccess) return false;
+    return (size_t)bytes + sizeof(double) * (size_t)h->fsize <= avail;
+}
+
 template <typename T>
 static int ensure_storage(spk_handle* h) {
+    Plan& P = h->plan[plan_index<T>(h)];
+    Storage<T>& S = storage<T>(h);
+    constexpr bool f64 = std::is_same<T, double>::value;
+    if (f64 && S.no_slices && slices_fit(h, S.slice_bytes)) {   // there is room for them again
+        S.no_slices = false;
+        drop_plan(h, P);
+    }
     int rc = ensure_plan<T>(h);
     if (rc) return rc;
-    Storage<T>& S = storage<T>(h);
     if (!S.d) CU(h, cudaMalloc((void**)&S.d, sizeof(T) * std::max<i64>(h->fsize, 1)));
-    if (!S.inv2) CU(h, cudaMalloc((void**)&S.inv2, sizeof(T) * std::max<ll>(h->plan[plan_index<T>(h)].inv2_size, 1)));
+    if (!S.inv2) CU(h, cudaMalloc((void**)&S.inv2, sizeof(T) * std::max<ll>(P.inv2_size, 1)));
     // BF16 packs take a quarter of the TF32 hi + lo bytes (same tiles and chunks)
-    const ll pack_bytes = h->plan[plan_index<T>(h)].pack_size / (std::is_same<T, float>::value && h->fmode ? 4 : 1);
+    const ll pack_bytes = P.pack_size / (std::is_same<T, float>::value && h->fmode ? 4 : 1);
     if (!S.pack && pack_bytes > 0) {
-        // The FP64 slices (twice the factor) are taken only where as much memory
-        // as the factor itself stays free: the CUDA-core updates need none.
-        cudaError_t e = cudaSuccess;
-        if (std::is_same<T, double>::value) {
-            size_t avail = 0, all = 0;
-            CU(h, cudaMemGetInfo(&avail, &all));
-            if ((size_t)pack_bytes + sizeof(T) * (size_t)h->fsize > avail) e = cudaErrorMemoryAllocation;
-        }
-        if (e == cudaSuccess) e = cudaMalloc((void**)&S.pack, (size_t)pack_bytes);
-        if (e == cudaErrorMemoryAllocation && std::is_same<T, double>::value) {
+        cudaError_t e = f64 && !slices_fit(h, pack_bytes) ? cudaErrorMemoryAllocation : cudaMalloc((void**)&S.pack, (size_t)pack_bytes);
+        if (f64 && e == cudaErrorMemoryAllocation) {   // a plan without slices
             cudaGetLastError();
             S.pack = nullptr;
-            h->no_slices = true;
-            free_plan(h->plan[plan_index<T>(h)]);
+            S.slice_bytes = pack_bytes;
+            S.no_slices = true;
+            drop_plan(h, P);
             return ensure_plan<T>(h);
         }
         CU(h, e);
@@ -2403,6 +2422,19 @@ int spk_set_option(spk_handle* h, int option, int64_t value) {
             reset_plans_keep_factors(h);
         }
         return SPK_OK;
+    case SPK_OPT_SLICE_LIMIT:
+        if (value < -1) break;
+        if (h->slice_limit != (long long)value) {
+            h->slice_limit = value;
+            for (int y = 0; y < 2; ++y) {   // the next factorisation asks for them afresh
+                Storage<double>& S = h->s64[y];
+                if (S.pack) cudaFree(S.pack);
+                S.pack = nullptr;
+                S.no_slices = false;
+                drop_plan(h, h->plan[2 * y]);
+            }
+        }
+        return SPK_OK;
     case SPK_OPT_PANEL_SPLIT:
         if (value != 0 && value != 1) break;
         h->panel_split = (int)value;
@@ -2460,6 +2492,7 @@ int spk_get_option(spk_handle* h, int option, int64_t* value) {
     case SPK_OPT_SCHUR_SPLIT: *value = h->schur_split; return SPK_OK;
     case SPK_OPT_SCHUR_FAR_SMS: *value = h->schur_far_sms; return SPK_OK;
     case SPK_OPT_SOLVE_CHUNK: *value = h->solve_chunk; return SPK_OK;
+    case SPK_OPT_SLICE_LIMIT: *value = h->slice_limit; return SPK_OK;
     default: return set_err(h, SPK_EARG, "spk_get_option: unknown option");
     }
 }

@@ -1,6 +1,6 @@
 """Memory of the FP64 slices (packed panels of the tensor-core rank updates):
 allocated whenever the plan in use has them, in whatever order the options,
-the values and the factorisation come.
+the values and the factorisation come, and refused without a trace.
 
 Tolerance: 1e-10 against the oracle's solution and 1e-12 for the residual, as
 the other solution tests on these grids.
@@ -57,3 +57,35 @@ def test_option_switched_back_between_load_and_factor(fused):
         x = eng.solve(np.array(b, order="F"), "fp64")
     assert slices(eng)
     check(s, A, b, x)
+
+
+def test_refused_slices():
+    # a factorisation without them, one with them again, and solves captured under either plan
+    s, A, b = system()
+    eng = _ensure_engine(s.slvr)
+    for limit in (-1, 0, 4096, -1):
+        eng.set_option("slice_limit", limit)
+        assert eng.get_option("slice_limit") == limit
+        _inmatrix_(s.slvr, A)
+        eng.profile_reset()
+        eng.factor("fp64")
+        assert slices(eng) == (limit < 0)
+        for _ in range(2):   # captured, then replayed
+            check(s, A, b, eng.solve(np.array(b, order="F"), "fp64"))
+
+
+def test_solve_captured_before_a_refusal():
+    # factored without slices by the option, solved (captured) under a plan that has them, then loaded again where
+    # they are refused: the replayed solve must not belong to the plan that was dropped
+    s, A, b = system()
+    eng = _ensure_engine(s.slvr)
+    eng.set_option("slice_limit", 0)
+    eng.set_option("lu_pieces", 1)
+    _inmatrix_(s.slvr, A)
+    eng.factor("fp64")
+    eng.set_option("lu_pieces", 0)
+    check(s, A, b, eng.solve(np.array(b, order="F"), "fp64"))
+    _inmatrix_(s.slvr, A)   # the slices are refused here
+    eng.factor("fp64")
+    assert not slices(eng)
+    check(s, A, b, eng.solve(np.array(b, order="F"), "fp64"))
