@@ -47,8 +47,8 @@ extern "C" {
 
 #define SPK_FP64 0         /* factor, solve and residual in double; the large
                               rank updates as exact integer slices on the
-                              tensor cores where memory for them (twice the
-                              factor's) is free, else double multiply-adds      */
+                              tensor cores where memory for one level's of
+                              them is free, else double multiply-adds           */
 #define SPK_FP32 1         /* factor and solve in float; residual and correction
                               in double (mixed form for spk_refine); the large
                               rank updates as 3xTF32 tensor-core products        */
@@ -376,11 +376,13 @@ int spk_measure_peaks(double* fp32_tflops, double* fp64_tflops, double* dmma_tfl
  *  SPK_OPT_SLICE_LIMIT   bytes that the integer slices of an FP64 form's rank
  *                        updates may take (-1, the default: what is free, as
  *                        long as the factor's size stays free beside them; 0:
- *                        none, the rank updates on the CUDA cores).  Where
- *                        they do not fit when a factorisation is prepared it
- *                        goes without, and the next one asks again; the
- *                        launches of the classes SPK_K_TC_TRAIL and
- *                        SPK_K_TC_SCHUR tell which it was.  Keeps the factors.
+ *                        none, the rank updates on the CUDA cores).  They are
+ *                        given back when another allocation of the handle
+ *                        finds no memory.  Where they do not fit when a
+ *                        factorisation is prepared it goes without, and the
+ *                        next one asks again; the launches of the classes
+ *                        SPK_K_TC_TRAIL and SPK_K_TC_SCHUR tell which it was.
+ *                        Keeps the factors.
  */
 #define SPK_OPT_LEAF_QUEUE 0
 #define SPK_OPT_WAIT_BUDGET 1

@@ -687,7 +687,10 @@ static void build_plan(const spk_handle* h, Plan& P, int bmax, bool tc, bool sym
     P.blk_lpack.assign(P.blk_c0.size(), -1);
     P.blk_upack.assign(P.blk_c0.size(), -1);
     {
+        // FP32 packs live side by side (far Schur tiles read a level's packs beside the next level's
+        // factorisation); FP64 levels follow one another, and all use the same memory
         const ll chunk = spk::umma::PCHUNK;
+        std::vector<ll> used(tc ? 1 : h->nlevels, 0);
         for (int i = 0; i < nfr; ++i) {
             const HFront& F = h->fronts[i];
             const int b0 = P.block0[i], nb = P.nblocks[i];
@@ -699,9 +702,11 @@ static void build_plan(const spk_handle* h, Plan& P, int bmax, bool tc, bool sym
                 const int n1 = cdiv(F.nf - P.blk_c1[b], spk::umma::TM);
                 const int nch = cdiv(P.blk_c1[b] - P.blk_c0[b], spk::umma::KCH);
                 const ll bytes = tc ? (ll)(n1 + n2) * nch * chunk : spk::oz_side_bytes(n1 + n2, nch);
-                P.blk_lpack[b] = P.pack_size;
-                P.blk_upack[b] = P.pack_size + bytes;
-                P.pack_size += 2 * bytes;
+                ll& at = used[tc ? 0 : F.level];
+                P.blk_lpack[b] = at;
+                P.blk_upack[b] = at + bytes;
+                at += 2 * bytes;
+                P.pack_size = std::max(P.pack_size, at);
             }
         }
     }
@@ -1239,7 +1244,7 @@ static void drop_plan(spk_handle* h, Plan& P) {
     free_plan(P);
 }
 
-// The FP64 slices (about twice the factor) are taken only where as much memory
+// The FP64 slices (one level's at a time) are taken only where as much memory
 // as the factor itself stays free, and within SPK_OPT_SLICE_LIMIT: the
 // CUDA-core updates need none.
 static bool slices_fit(spk_handle* h, ll bytes) {
@@ -1249,8 +1254,35 @@ static bool slices_fit(spk_handle* h, ll bytes) {
     return (size_t)bytes + sizeof(double) * (size_t)h->fsize <= avail;
 }
 
+// Give the FP64 slices back; the plans that had them are rebuilt without.
+static bool release_slices(spk_handle* h) {
+    bool any = false;
+    for (int y = 0; y < 2; ++y) {
+        Storage<double>& S = h->s64[y];
+        if (!S.pack) continue;
+        cudaFree(S.pack);
+        S.pack = nullptr;
+        S.no_slices = any = true;
+        drop_plan(h, h->plan[2 * y]);
+    }
+    return any;
+}
+
+// Run `alloc` (which can be run again after it failed); where the device has
+// no memory for it, the FP64 slices make room and it is run once more.
+template <typename Alloc>
+static int with_memory(spk_handle* h, Alloc alloc) {
+    int rc = alloc();
+    if (rc == SPK_ENOMEM && release_slices(h)) {
+        cudaGetLastError();
+        rc = alloc();
+    }
+    if (rc == SPK_ENOMEM) cudaGetLastError();
+    return rc;
+}
+
 template <typename T>
-static int ensure_storage(spk_handle* h) {
+static int try_storage(spk_handle* h) {
     Plan& P = h->plan[plan_index<T>(h)];
     Storage<T>& S = storage<T>(h);
     constexpr bool f64 = std::is_same<T, double>::value;
@@ -1264,12 +1296,12 @@ static int ensure_storage(spk_handle* h) {
     if (!S.inv2) CU(h, cudaMalloc((void**)&S.inv2, sizeof(T) * std::max<ll>(P.inv2_size, 1)));
     // BF16 packs take a quarter of the TF32 hi + lo bytes (same tiles and chunks)
     const ll pack_bytes = P.pack_size / (std::is_same<T, float>::value && h->fmode ? 4 : 1);
+    if (f64 && pack_bytes > 0) S.slice_bytes = pack_bytes;
     if (!S.pack && pack_bytes > 0) {
         cudaError_t e = f64 && !slices_fit(h, pack_bytes) ? cudaErrorMemoryAllocation : cudaMalloc((void**)&S.pack, (size_t)pack_bytes);
         if (f64 && e == cudaErrorMemoryAllocation) {   // a plan without slices
             cudaGetLastError();
             S.pack = nullptr;
-            S.slice_bytes = pack_bytes;
             S.no_slices = true;
             drop_plan(h, P);
             return ensure_plan<T>(h);
@@ -1278,10 +1310,10 @@ static int ensure_storage(spk_handle* h) {
     }
     return SPK_OK;
 }
+template <typename T>
+static int ensure_storage(spk_handle* h) { return with_memory(h, [&] { return try_storage<T>(h); }); }
 
-static int ensure_rhs(spk_handle* h, i64 nrhs) {
-    if (nrhs <= h->rhs_cap) return SPK_OK;
-    drop_solve_graphs(h);
+static int try_rhs(spk_handle* h, i64 nrhs) {
     cudaFree(h->d_wb); cudaFree(h->d_wy); cudaFree(h->d_wx);
     cudaFree(h->d_rhs); cudaFree(h->d_x); cudaFree(h->d_r); cudaFree(h->d_sums);
     h->d_wb = h->d_wy = h->d_wx = nullptr;
@@ -1299,6 +1331,11 @@ static int ensure_rhs(spk_handle* h, i64 nrhs) {
     CU(h, cudaMalloc((void**)&h->d_sums, sizeof(double) * 2 * (size_t)nrhs));
     h->rhs_cap = nrhs;
     return SPK_OK;
+}
+static int ensure_rhs(spk_handle* h, i64 nrhs) {
+    if (nrhs <= h->rhs_cap) return SPK_OK;
+    drop_solve_graphs(h);
+    return with_memory(h, [&] { return try_rhs(h, nrhs); });
 }
 
 // ---------------------------------------------------------------------------
@@ -1936,8 +1973,11 @@ static int residual_device(spk_handle* h, const double* b, i64 ldb, const double
 // ---------------------------------------------------------------------------
 constexpr int GM_M = 30;
 
-static int ensure_gmres(spk_handle* h) {
-    if (h->gm_V) return SPK_OK;
+static int try_gmres(spk_handle* h) {
+    for (double** p : {&h->gm_V, &h->gm_Z, &h->gm_w, &h->gm_c}) {   // of an attempt that ran out of memory
+        cudaFree(*p);
+        *p = nullptr;
+    }
     const size_t blk = sizeof(double) * (size_t)h->n * spk::GM_MAXRHS;
     CU(h, cudaMalloc((void**)&h->gm_V, blk * (GM_M + 1)));
     CU(h, cudaMalloc((void**)&h->gm_Z, blk * GM_M));
@@ -1945,6 +1985,7 @@ static int ensure_gmres(spk_handle* h) {
     CU(h, cudaMalloc((void**)&h->gm_c, sizeof(double) * (2 * (GM_M + 1) + 1) * spk::GM_MAXRHS));
     return SPK_OK;
 }
+static int ensure_gmres(spk_handle* h) { return h->gm_c ? SPK_OK : with_memory(h, [&] { return try_gmres(h); }); }
 
 // Columns [0, nrhs) of b / x (nrhs <= GM_MAXRHS).  `budget` preconditioned
 // solves at most; *used receives the number made, *cycles the restarts.
@@ -2920,7 +2961,11 @@ int spk_grad_pattern(spk_handle* h, const double* lambda, const double* x, int64
                                 cudaMemcpyHostToDevice, h->stream));
         CU(h, cudaMemcpy2DAsync(h->d_x, sizeof(double) * n, x, sizeof(double) * ld, sizeof(double) * n, nrhs,
                                 cudaMemcpyHostToDevice, h->stream));
-        CU(h, cudaMallocAsync((void**)&tmp, sizeof(double) * (size_t)h->nnz, h->stream));
+        if ((rc = with_memory(h, [&]() -> int {
+                CU(h, cudaMallocAsync((void**)&tmp, sizeof(double) * (size_t)h->nnz, h->stream));
+                return SPK_OK;
+            })))
+            return rc;
         dl = h->d_rhs;
         dxp = h->d_x;
         dg = tmp;

@@ -89,3 +89,53 @@ def test_solve_captured_before_a_refusal():
     eng.factor("fp64")
     assert not slices(eng)
     check(s, A, b, eng.solve(np.array(b, order="F"), "fp64"))
+
+
+def test_slices_make_room():
+    # an allocation that finds no memory gets that of the slices first; here not even that is enough, the call fails
+    # with a status, and the factor and the next factorisations are sound
+    import ctypes
+
+    from sparspak import _native as N
+
+    s, A, b = system()
+    eng = _ensure_engine(s.slvr)
+    _inmatrix_(s.slvr, A)
+    eng.profile_reset()
+    eng.factor("fp64")
+    assert slices(eng)
+    rc = N.gpu().spk_solve(eng._h, ctypes.c_void_p(1), 1 << 40, A.shape[0], N.SPK_HOST, N.SPK_FP64)   # the right-hand sides are not read
+    assert rc == N.SPK_ENOMEM
+    check(s, A, b, eng.solve(np.array(b, order="F"), "fp64"))
+    for fused in (False, True):
+        _inmatrix_(s.slvr, A)
+        x = np.zeros_like(b, order="F")
+        eng.profile_reset()
+        if fused:
+            eng.factor_refine(b, x, "fp64")
+        else:
+            eng.factor("fp64")
+            x = eng.solve(np.array(b, order="F"), "fp64")
+        assert slices(eng)   # there is room again
+        check(s, A, b, x)
+
+
+def test_pack_of_one_level_serves_all():
+    # levels use the same memory for their slices: a system with tensor-core fronts on several levels, every factor
+    # entry against the oracle's
+    k = 20
+    A = S.gallery.convection_diffusion(k=k)
+    s = S.SparseSolver(A)
+    S.findorder_(s, S.nd_grid(k, k, k))
+    S.symbolicfactor_(s)
+    _inmatrix_(s.slvr, A)
+    eng = s.slvr.engine
+    eng.profile_reset()
+    S.sparse_solver._factor_(s.slvr)
+    assert eng.profile_read()["tc_schur"]["launches"] >= 2
+    o = oracle.OracleLU(s.slvr)
+    o.inmatrix_csc(*_matrix_arrays(A))
+    assert o.factor() == 0
+    assert np.array_equal(s.slvr.ipiv, o.ipiv)
+    for a, r in ((s.slvr.lnz, o.lnz), (s.slvr.unz, o.unz[: s.slvr.unz.size])):
+        assert np.max(np.abs(a - r)) <= 1e-12 * np.max(np.abs(r))
