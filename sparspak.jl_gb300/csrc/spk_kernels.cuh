@@ -1826,9 +1826,10 @@ __device__ __forceinline__ void sweep_f64(double (&x)[W / PD_LANES], const doubl
         }
 }
 
-// The largest exponent field of every U row over the lines of a CTA into
-// rexp, from which the slices of the tensor-core updates take their scaling
-// along the block.
+// The largest exponent field of the finite entries of every U row over the
+// lines of a CTA into rexp, from which the slices of the tensor-core updates
+// take their scaling along the block.  (An infinity's would leave nothing of
+// the columns beside it.)
 template <int CQ>
 __device__ __forceinline__ void oz_row_max(const double (&y)[CQ], bool ok, int bw, int* smx, int* rexp) {
     const int lane = threadIdx.x & 31, q = lane & (PD_LANES - 1);
@@ -1837,6 +1838,7 @@ __device__ __forceinline__ void oz_row_max(const double (&y)[CQ], bool ok, int b
 #pragma unroll
     for (int i = 0; i < CQ; ++i) {
         int e = ok ? (__double2hiint(y[i]) >> 20) & 0x7ff : 0;
+        e = e == 0x7ff ? 0 : e;
         e = max(e, __shfl_xor_sync(0xffffffffu, e, 8));
         e = max(e, __shfl_xor_sync(0xffffffffu, e, 16));
         if (lane < PD_LANES && e > 0) atomicMax(&smx[i * PD_LANES + q], e);
