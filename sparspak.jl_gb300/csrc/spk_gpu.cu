@@ -193,7 +193,7 @@ struct spk_handle {
     ll* d_run_rel = nullptr;
     int* d_ipiv = nullptr;
     int* d_bmap = nullptr;     // row sources of each block's interchanges (k_block_lu_f32 -> panels)
-    int* d_rexp = nullptr;     // FP64: exponent field of each U row's largest panel entry (panels -> k_oz_pack)
+    int* d_rexp = nullptr;     // FP64: exponent fields of each U row's and L column's largest panel entry (panels -> k_oz_pack)
     int* d_info = nullptr;
 
     // pattern and values
@@ -1044,7 +1044,7 @@ static int upload_structure(spk_handle* h) {
     if ((rc = upload(h, &h->d_rel, h->rel))) return rc;
     CU(h, cudaMalloc((void**)&h->d_ipiv, sizeof(int) * std::max<i64>(h->n, 1)));
     CU(h, cudaMalloc((void**)&h->d_bmap, sizeof(int) * std::max<i64>(h->n, 1)));
-    CU(h, cudaMalloc((void**)&h->d_rexp, sizeof(int) * std::max<i64>(h->n, 1)));
+    CU(h, cudaMalloc((void**)&h->d_rexp, 2 * sizeof(int) * std::max<i64>(h->n, 1)));
     // first singular piece, tensor-core wait timeout, leaf-queue wait timeout
     CU(h, cudaMalloc((void**)&h->d_info, 3 * sizeof(int)));
     return SPK_OK;
@@ -1454,7 +1454,7 @@ static int factor_launches(spk_handle* h, int fs_nrhs = 0) {
                                                                                   PL.d_blk_front, ent);
         }
     };
-    if (std::is_same<T, double>::value) CU(h, cudaMemsetAsync(h->d_rexp, 0, sizeof(int) * (size_t)h->n, h->stream));
+    if (std::is_same<T, double>::value) CU(h, cudaMemsetAsync(h->d_rexp, 0, 2 * sizeof(int) * (size_t)h->n, h->stream));
     const bool queue = h->leaf_queue != 0 && PL.nq > 0;
     if (queue) {   // the bottom subtrees first, in one persistent launch
         CU(h, cudaMemcpyAsync(PL.d_q_deps, PL.d_q_deps0, sizeof(int) * h->fronts.size(), cudaMemcpyDeviceToDevice,
@@ -1589,7 +1589,7 @@ static int factor_launches(spk_handle* h, int fs_nrhs = 0) {
             if constexpr (std::is_same<T, double>::value) {
                 if (P.oz_pack[t].tiles > 0) {
                     LaunchScope ls(h, SPK_K_PANEL, 0.0, 3.0 * P.oz_pack[t].words * sizeof(T));
-                    spk::k_oz_pack<<<P.oz_pack[t].tiles, 256, 0, h->stream>>>(fac, h->d_rexp, storage<T>(h).pack, S,
+                    spk::k_oz_pack<<<P.oz_pack[t].tiles, 8 * spk::OZ_PLINES, 0, h->stream>>>(fac, h->d_rexp, storage<T>(h).pack, S,
                                                                             launch_of(PL, P.oz_pack[t]), (int)t);
                 }
             }

@@ -1826,10 +1826,10 @@ __device__ __forceinline__ void sweep_f64(double (&x)[W / PD_LANES], const doubl
         }
 }
 
-// The largest exponent field of the finite entries of every U row over the
-// lines of a CTA into rexp, from which the slices of the tensor-core updates
-// take their scaling along the block.  (An infinity's would leave nothing of
-// the columns beside it.)
+// The largest exponent field of the finite entries of every U row (L column)
+// over the lines of a CTA into every second entry of rexp, from which the
+// slices of the tensor-core updates take their scaling along the block.  (An
+// infinity's would leave nothing of the columns beside it.)
 template <int CQ>
 __device__ __forceinline__ void oz_row_max(const double (&y)[CQ], bool ok, int bw, int* smx, int* rexp) {
     const int lane = threadIdx.x & 31, q = lane & (PD_LANES - 1);
@@ -1844,7 +1844,7 @@ __device__ __forceinline__ void oz_row_max(const double (&y)[CQ], bool ok, int b
         if (lane < PD_LANES && e > 0) atomicMax(&smx[i * PD_LANES + q], e);
     }
     __syncthreads();
-    if ((int)threadIdx.x < bw && smx[threadIdx.x] > 0) atomicMax(&rexp[threadIdx.x], smx[threadIdx.x]);
+    if ((int)threadIdx.x < bw && smx[threadIdx.x] > 0) atomicMax(&rexp[2 * threadIdx.x], smx[threadIdx.x]);
 }
 
 template <int W>
@@ -1891,6 +1891,7 @@ __global__ void __launch_bounds__(128) k_block_panel_f64(double* fac, const int*
             if (j < bw) x[jj] *= rd[j];
             if (ok && j < bw) xp[(ll)j * F.ld] = x[jj];
         }
+        if (S.blk_upack[blk] >= 0) oz_row_max<CQ>(x, ok, bw, smx, rexp + 2 * (F.f + c0) + 1);
         if (S.sym) {   // symmetric form: the U side, U(c0 + j, r) = U(j, j) L(r, c0 + j)
 #pragma unroll
             for (int jj = 0; jj < CQ; ++jj) {
@@ -1901,7 +1902,7 @@ __global__ void __launch_bounds__(128) k_block_panel_f64(double* fac, const int*
                     else fac[F.uoff + (ll)(c0 + j) * F.m + (r - F.nf)] = x[jj];
                 }
             }
-            if (S.blk_upack[blk] >= 0) oz_row_max<CQ>(x, ok, bw, smx, rexp + F.f + c0);
+            if (S.blk_upack[blk] >= 0) oz_row_max<CQ>(x, ok, bw, smx, rexp + 2 * (F.f + c0));
         }
     } else {
         for (int k = tid; k <= np; k += 128) q0[k] = S.xsuper[p0 + k] - F.f - c0;
@@ -1930,7 +1931,7 @@ __global__ void __launch_bounds__(128) k_block_panel_f64(double* fac, const int*
             const int k = jj * PD_LANES + q;
             if (ok && k < bw) cp[(ll)k * stride] = x[jj];
         }
-        if (S.blk_upack[blk] >= 0) oz_row_max<CQ>(x, ok, bw, smx, rexp + F.f + c0);
+        if (S.blk_upack[blk] >= 0) oz_row_max<CQ>(x, ok, bw, smx, rexp + 2 * (F.f + c0));
     }
 }
 
@@ -3357,12 +3358,35 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc_update(float* fac, const u
 // roundings where the multiply-add loop makes 64 (4096 x 4096 entries of
 // 64-term sums of uniform [-1, 1] values against 128-bit sums: largest error
 // 8.7e-16, of the loop 6.2e-15).
-//   Rows and columns may differ in size by any power of two (each line has
-// its exponent); along the block's columns L is scaled by 2^t and U by 2^-t
-// with t the exponent of the U row's largest entry, so that badly row-,
-// column- or symmetrically scaled matrices lose nothing.  A line that holds
-// an infinity or a NaN, and a product whose scale leaves the exponent range,
-// take a plain FP64 sum over the stored factor instead.
+//   Rows and columns may differ in size by any power of two: each line has its
+// exponent, and along the block column k of L is scaled by 2^t, row k of U by
+// 2^-t, t half of what separates the exponents of the largest entries of the
+// two.  That alone is not enough.  With M_i and N_j the largest scaled entries of
+// a row of L and a column of U the error of entry (i, j) is about 2^-59 M_i N_j;
+// where the entries of a line lie far apart (a column of A that is large, and
+// zero in some rows of the block), the entry can be far smaller.  So
+//   - index i (row i of L, column i of U) is marked where M_i N_i is more than
+//     2^OZ_SPREAD times its largest product L(i, k) U(k, i).  Between indices
+//     without a mark the error is below the rounding errors that the
+//     multiply-add loop makes on the two diagonal entries, and no scaling of A's
+//     rows or columns changes that (M_i N_i and the products change alike);
+//   - an entry of a marked index that came out, and left its target, below
+//     2^-OZ_TIGHT M_i N_j is formed again as a plain FP64 sum over the stored
+//     factor, other entries below 2^-OZ_LOOSE.
+// Errors of 64-term sums of 256 x 256 entries in units of 2^-53 (|target| +
+// sum |L||U|), of the multiply-add loop, the slices with this rule and without
+// it: uniform entries 3.7, 0.9, 0.9; one U column 2^40 larger in half of its
+// rows 4.1, 4.1, 11,000; one L column 8.0, 4.6, 5,600.  Tighter than 2^-8 gains
+// nothing over the loop, 2^-10 leaves 20.  Fronts of Laplacians, convection-
+// diffusion and 2-D diffusion have no marked index (M_i N_i is at most 2^3 of
+// the largest product; 2^8 with t from the U rows alone); 2^-8 for them too
+// would form 1% of their entries again, nearly all in tiles beside the diagonal
+// whose indices are far apart in a separator (48^3 convection-diffusion: 50.5 ms
+// for the factorisation instead of 35.4; none at all 34.0).  With one column of
+// that system scaled by 2^40 it takes 42 ms, with its rows scaled by random
+// powers of two up to 2^30 159 ms (multiply-add loop: 164, 165).
+//   Entries of a line that holds an infinity or a NaN, and those whose scale
+// leaves the exponent range, are formed again too.
 //   Tiles of 128 x 32: eight weights of 32 columns are 256 TMEM columns,
 // double-buffered.  Digit i of L meets digits 0 .. 7 - i of U in one MMA of
 // 32 (8 - i) columns, whose products are weights i .. 7: eight MMAs per 16
@@ -3386,6 +3410,10 @@ constexpr int OZ_EXPS = (umma::TM + OZ_N) * 4;           // exponents of a tile'
 constexpr int OZ_ERING = 8;                              // more than the blocks the copies can run ahead
 constexpr int OZ_SMEM = OZ_NST * OZ_STAGE + OZ_ERING * OZ_EXPS + 2048;
 constexpr int OZ_BAD = 1 << 28;                          // exponent of a line with a NaN or an infinity
+constexpr int OZ_ZERO = -(1 << 20);                      // of a line of zeros
+constexpr int OZ_SPREAD = 4;                             // lines marked: bits between M_i N_i and their largest common product
+constexpr int OZ_TIGHT = 8, OZ_LOOSE = 16;               // entries formed again: bits below M_i N_j, of a marked line and of others
+constexpr int OZ_FEW = 256;                              // of a tile's at most by eight lanes each
 
 // Bytes of one side of a block's pack: T tiles of 128 lines, nch chunks of 16
 // columns, then the lines' exponents.
@@ -3418,58 +3446,81 @@ __host__ __device__ __forceinline__ void oz_lower_tile(int t, int c, int& rt, in
     ct = t;
 }
 
-// The slices of a block's L and U panels: a CTA per side and 128-line tile,
-// two threads per line (32 columns each).
-__global__ void __launch_bounds__(256) k_oz_pack(const double* fac, const int* rexp, unsigned char* pack, Sched S, Launch L,
-                                                 int step) {
-    __shared__ int sE[2][128];
+// The slices of a block's L and U panels: a CTA per 64 lines of both sides, four
+// threads per line (16 columns each).  A line's exponent is stored with its mark
+// in the lowest bit.
+constexpr int OZ_PLINES = 64;
+__global__ void __launch_bounds__(8 * OZ_PLINES) k_oz_pack(const double* fac, const int* rexp, unsigned char* pack, Sched S, Launch L,
+                                                           int step) {
+    __shared__ int sE[2][4][OZ_PLINES], sB[4][OZ_PLINES], sS[64];
+    __shared__ short sX[64][OZ_PLINES];   // exponents of the U lines' entries
     int fid, tile;
     locate(L, blockIdx.x, fid, tile);
     const DFront F = S.fronts[fid];
     const int blk = F.block0 + step;
     const int c0 = S.blk_c0[blk], c1 = S.blk_c1[blk], bw = c1 - c0, nch = cdiv(bw, umma::KCH);
     const int n1 = cdiv(F.nf - c1, umma::TM), T = n1 + cdiv(F.m, umma::TM);
-    const bool isU = tile >= T;
-    const int t = isU ? tile - T : tile, line = threadIdx.x & 127, half = threadIdx.x >> 7;
+    const bool isU = threadIdx.x >= 4 * OZ_PLINES;
+    const int x0 = threadIdx.x % OZ_PLINES, part = (threadIdx.x / OZ_PLINES) & 3;
+    const int t = tile / 2, line = (tile & 1) * OZ_PLINES + x0;
     const int idx = t < n1 ? c1 + t * umma::TM + line : F.nf + (t - n1) * umma::TM + line;
     const bool ok = idx < (t < n1 ? F.nf : F.ld);
     // entry k of the line at p[k * ps]
     const double* p = !isU ? fac + F.loff + (ll)c0 * F.ld + idx
                            : idx < F.nf ? fac + F.loff + (ll)idx * F.ld + c0 : fac + F.uoff + (ll)c0 * F.m + (idx - F.nf);
     const ll ps = !isU ? F.ld : idx < F.nf ? 1 : F.m;
-    const int k0 = half * 32;
-    long long x[32];
+    const int k0 = part * 16;
+    long long x[16];
 #pragma unroll
-    for (int k = 0; k < 32; ++k) x[k] = ok && k0 + k < bw ? __double_as_longlong(p[(k0 + k) * ps]) : 0ll;
-    int E = -(1 << 20);
+    for (int k = 0; k < 16; ++k) x[k] = ok && k0 + k < bw ? __double_as_longlong(p[(k0 + k) * ps]) : 0ll;
+    if (threadIdx.x < 64) {   // a column of L (row of U) without a normal entry scales the other out of the way
+        const int k = threadIdx.x, fu = k < bw ? rexp[2 * (F.f + c0 + k)] : 0, fl = k < bw ? rexp[2 * (F.f + c0 + k) + 1] : 0;
+        sS[k] = fu && fl ? (fu - fl) >> 1 : fu ? fu + 2000 : fl ? -(fl + 2000) : 0;
+    }
+    __syncthreads();
+    int E = OZ_ZERO;
 #pragma unroll
-    for (int k = 0; k < 32; ++k) {
-        const int ex = (int)((x[k] >> 52) & 0x7ff);
-        const int tk = k0 + k < bw ? rexp[F.f + c0 + k0 + k] : 0, sh = tk ? (isU ? 1023 - tk : tk - 1023) : 0;
+    for (int k = 0; k < 16; ++k) {
+        const int ex = (int)((x[k] >> 52) & 0x7ff), sh = isU ? -sS[k0 + k] : sS[k0 + k];
         if (ex == 0x7ff) E = OZ_BAD;
         else if ((x[k] << 1) != 0) E = max(E, (ex ? ex : 1) - 1022 + sh);   // |x| 2^sh < 2^E
+        if (isU) sX[k0 + k][x0] = (x[k] << 1) != 0 ? (short)ex : (short)-30000;
     }
-    sE[half][line] = E;
+    sE[isU][part][x0] = E;
     __syncthreads();
-    E = max(sE[0][line], sE[1][line]);
-    if (E == -(1 << 20)) E = 0;
-    unsigned char* side = pack + (isU ? S.blk_upack[blk] : S.blk_lpack[blk]);
-    if (half == 0) oz_exps(side, T, nch)[t * umma::TM + line] = E;
+    E = max(max(sE[isU][0][x0], sE[isU][1][x0]), max(sE[isU][2][x0], sE[isU][3][x0]));
+    if (!isU) {   // the line's largest product L(i, k) U(k, i) is below 2^B
+        int B = OZ_ZERO;
 #pragma unroll
-    for (int g = 0; g < 4; ++g) {   // eight columns: one 16-byte unit per slice
+        for (int k = 0; k < 16; ++k) {
+            const int ex = (x[k] << 1) != 0 ? (int)((x[k] >> 52) & 0x7ff) : -30000;
+            B = max(B, ex + sX[k0 + k][x0] - 2 * 1022);
+        }
+        sB[part][x0] = B;
+    }
+    __syncthreads();
+    unsigned char* side = pack + (isU ? S.blk_upack[blk] : S.blk_lpack[blk]);
+    if (part == 0) {
+        const int O = isU ? 0 : 1;
+        const int other = max(max(sE[O][0][x0], sE[O][1][x0]), max(sE[O][2][x0], sE[O][3][x0]));
+        const int B = max(max(sB[0][x0], sB[1][x0]), max(sB[2][x0], sB[3][x0]));
+        const bool mark = (E != OZ_ZERO || other != OZ_ZERO) && E + other - B > OZ_SPREAD;
+        oz_exps(side, T, nch)[t * umma::TM + line] = 2 * E + (mark ? 1 : 0);
+    }
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {   // eight columns: one 16-byte unit per slice
         const int kg = k0 + 8 * g;
         if (kg >= nch * umma::KCH) break;
         long long q[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             const long long b = x[8 * g + e];
-            const int tk = kg + e < bw ? rexp[F.f + c0 + kg + e] : 0, sh = tk ? (isU ? 1023 - tk : tk - 1023) : 0;
-            const int ex = (int)((b >> 52) & 0x7ff);
+            const int ex = (int)((b >> 52) & 0x7ff), sh = isU ? -sS[kg + e] : sS[kg + e];
             const long long m = (b & 0xfffffffffffffll) | (ex ? 1ll << 52 : 0ll);
             const int s = (ex ? ex : 1) - 1075 + sh + 62 - E;   // |x| 2^(sh + 62 - E) = m 2^s, s <= 9
             long long v = 0;
-            if (E != OZ_BAD && s >= 0) v = m << s;
-            else if (E != OZ_BAD && s > -54) v = (m + (1ll << (-s - 1))) >> -s;
+            if (E != OZ_BAD && E != OZ_ZERO && s >= 0) v = m << s;
+            else if (E != OZ_BAD && E != OZ_ZERO && s > -54) v = (m + (1ll << (-s - 1))) >> -s;
             q[e] = b < 0 ? -v : v;
         }
         // L: slices of 128 lines; U: of 32 lines, so that a tile's eight slices are contiguous
@@ -3566,8 +3617,9 @@ __device__ __forceinline__ void oz_lines(const Sched& S, const OzTile& T, int b,
 // The product from its weights (0 .. 4 joined in units of 2^E, 5 .. 7 of
 // 2^(E - 24); 76 bits at most), rounded once to nearest; SIGN flips it.  By
 // integer instructions: a conversion or an addition in FP64 costs a quarter of
-// the SM 64 cycles and more, and the form with both takes four of them.
-__device__ __forceinline__ double oz_join(const int (&n)[OZ_D], int E, long long SIGN) {
+// the SM 64 cycles and more, and the form with both takes four of them.  z:
+// the product is below 2^(E + 54 - z), not below half of that.
+__device__ __forceinline__ double oz_join(const int (&n)[OZ_D], int E, long long SIGN, int& z) {
     // |weight w| <= 2^20 (w + 1)
     const long long hi = ((long long)(n[0] * 256 + n[1]) << 24) + ((long long)n[2] << 16) + (n[3] * 256 + n[4]);
     const long long lo = ((long long)n[5] << 16) + (n[6] * 256 + n[7]);
@@ -3577,7 +3629,7 @@ __device__ __forceinline__ double oz_join(const int (&n)[OZ_D], int E, long long
     const long long neg = top >> 63;
     const unsigned long long a = (unsigned long long)(top ^ neg) + (neg && frac == 0);
     const unsigned fr = (frac ^ (unsigned)neg) - (unsigned)neg;
-    const int z = __clzll((long long)a);
+    z = __clzll((long long)a);
     if (z > 43) {   // small after cancellation, or zero
         const double v = fma((double)lo, __longlong_as_double((long long)(E - 24 + 1023) << 52),
                              (double)hi * __longlong_as_double((long long)(E + 1023) << 52));
@@ -3595,15 +3647,44 @@ __device__ __forceinline__ double oz_join(const int (&n)[OZ_D], int E, long long
     return __longlong_as_double((((long long)(E + 1075 - z) << 52) + (long long)m) ^ (neg & (long long)(1ull << 63)) ^ SIGN);
 }
 
-// Sum over block b of L(row, k) U(k, col), plain FP64 (front-local row; col
-// of the front, or nf + the U12 column).
-__device__ __noinline__ double oz_plain(const double* fac, const Sched& S, const DFront& F, int b, int row, int col) {
-    const int c0 = S.blk_c0[b], c1 = S.blk_c1[b];
+// Sum of L(row, k) U(k, col) over k = c0, c0 + step, .. below c1 of a front,
+// plain FP64 (front-local row; col of the front, or nf + the U12 column).
+__device__ __forceinline__ double oz_sum(const double* fac, const DFront& F, int row, int col, int c0, int c1, int step) {
+    const bool in = col < F.nf;
+    const double *l = fac + F.loff + row, *u = in ? fac + F.loff + (ll)col * F.ld : fac + F.uoff + (col - F.nf);
+    const ll us = in ? 1 : F.m;
     double s = 0.0;
-    for (int k = c0; k < c1; ++k)
-        s += fac[F.loff + (ll)k * F.ld + row] *
-             (col < F.nf ? fac[F.loff + (ll)col * F.ld + k] : fac[F.uoff + (ll)k * F.m + col - F.nf]);
+#pragma unroll 8
+    for (int k = c0; k < c1; k += step) s += l[(ll)k * F.ld] * u[k * us];
     return s;
+}
+__device__ __forceinline__ bool oz_below(double v, int lim) {   // |v| < 2^lim
+    return ((__double2hiint(v) >> 20) & 0x7ff) - 1023 < lim;
+}
+// SCHUR: offset of entry (r, c)'s target, -1 if it has none.  (Rc, Rr: the
+// scatter rows of c and r.)
+__device__ __forceinline__ ll oz_target(const int* rel, const ScatterRow& Rc, const ScatterRow& Rr, int r, int c) {
+    const ScatterRow& R = r >= c ? Rc : Rr;
+    const int p = rel[R.rel0 + (r >= c ? r : c)];
+    if (p < 0 || R.pos < 0) return -1;
+    if (r >= c) return R.loff + (ll)R.pos * R.ld + p;   // L entry of the front of R_F[c]
+    return p < R.nf ? R.loff + (ll)p * R.ld + R.pos : R.uoff + (ll)R.pos * R.m + (p - R.nf);   // of the front of R_F[r]
+}
+// A warp's entries to form again (place + j with bit j of fix), those of a
+// column together.
+__device__ __noinline__ void oz_push(unsigned short* again, int* n, int place, unsigned fix) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, total = __reduce_add_sync(FULL, __popc(fix));
+    if (total == 0) return;
+    int at = 0;
+    if (lane == 0) at = atomicAdd(n, total);
+    at = __shfl_sync(FULL, at, 0);
+#pragma unroll 1
+    for (int j = 0; j < 8; ++j) {
+        const unsigned m = __ballot_sync(FULL, (fix >> j) & 1u);
+        if ((fix >> j) & 1u) again[at + __popc(m & ((1u << lane) - 1u))] = (unsigned short)(place + j);
+        at += __popc(m);
+    }
 }
 
 template <int MODE>
@@ -3611,6 +3692,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_update(double* fac, unsign
                                                              int ntiles, int part, int* err) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ ScatterRow tab[umma::TM + OZ_N];   // SCHUR: tile rows, then tile columns
+    __shared__ unsigned short again[umma::TM * OZ_N];   // the tile's entries to form again: row * OZ_N + column
+    __shared__ int nagain[3];                           // their number, of this tile, the next and the last but one
     __shared__ int dead;
     unsigned char* stage = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char* exps = stage + OZ_NST * OZ_STAGE;
@@ -3630,6 +3713,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_update(double* fac, unsign
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         dead = 0;
+        nagain[0] = nagain[1] = nagain[2] = 0;
     }
     if (warp == 1) umma::tmem_alloc(tmem_slot, 512);
     umma::fence_before();
@@ -3706,7 +3790,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_update(double* fac, unsign
         }
     } else if (warp >= 4) {   // epilogue: thread = one TMEM lane (tile row), 8 of the tile's columns
         const int q4 = warp & 3, i = 32 * q4 + lane, cg = (warp - 4) >> 2, et = threadIdx.x - 128;
-        int acc = 0, u = 0;
+        int acc = 0, u = 0, turn = 0;   // turn: of nagain
         uint32_t aph = 0;
         OzTile T;
         for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -3742,11 +3826,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_update(double* fac, unsign
 #pragma unroll
             for (int j = 0; j < 8; ++j) sum[j] = MODE == TC_TRAIL && rok && col0 + j < cend ? dst[j * sj] : 0.0;
             constexpr long long SIGN = MODE == TC_TRAIL ? (long long)(1ull << 63) : 0ll;
+            unsigned low = 0;            // columns whose product came out low (or could not be formed) in some block
+            int lim = -(1 << 30);        // and the largest 2^lim that it was below
             for (int b = T.b0; b < T.b0 + T.nb; ++b) {
                 const int* ev = reinterpret_cast<const int*>(exps + (u % OZ_ERING) * OZ_EXPS);
                 umma::wait_bounded(&efull[u % OZ_ERING], (u / OZ_ERING) & 1, vdead, err);
                 ++u;
-                const int ei = ev[i];
+                const int ei = ev[i];   // exponent, and the mark in the lowest bit
                 const int* fj = ev + umma::TM + cg * 8;
                 umma::wait_bounded(&tfull[acc], aph, vdead, err);
                 umma::fence_after();
@@ -3760,13 +3846,19 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_update(double* fac, unsign
                         int n[OZ_D];
 #pragma unroll
                         for (int w = 0; w < OZ_D; ++w) n[w] = __float2int_rn(v[w][j]);
-                        const int f = fj[4 * h + j], E = ei + f - 44;
+                        const int fe = fj[4 * h + j], W = (ei >> 1) + (fe >> 1);   // M_i N_j < 2^W
                         double& s = sum[4 * h + j];
-                        if (E - 24 > -1022 && E < 960) {
-                            s += oz_join(n, E, SIGN);
-                        } else if (row < rend && col0 + 4 * h + j < cend) {
-                            const double v = oz_plain(fac, S, F, b, row, col0 + 4 * h + j);
-                            s += MODE == TC_TRAIL ? -v : v;
+                        if (W - 68 > -1022 && W < 1004) {
+                            int z;
+                            s += oz_join(n, W - 44, SIGN, z);
+                            const int guard = (ei | fe) & 1 ? OZ_TIGHT : OZ_LOOSE;
+                            if (z >= 10 + guard) {
+                                low |= 1u << (4 * h + j);
+                                lim = max(lim, W - guard);
+                            }
+                        } else if (W > OZ_ZERO / 2) {   // (a line of zeros adds nothing)
+                            low |= 1u << (4 * h + j);
+                            lim = 1 << 20;
                         }
                     }
                     __syncwarp();   // the next load is warp-wide
@@ -3775,11 +3867,19 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_update(double* fac, unsign
                 umma::arrive(&tempty[acc]);
                 if (++acc == 2) { acc = 0; aph ^= 1; }
             }
+            if (__any_sync(0xffffffffu, low != 0)) {   // low: becomes the entries left out here and formed again below
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const bool there = rok && col0 + j < cend && (MODE == TC_TRAIL || row >= col0 + j || !S.sym);
+                    if (!there || !oz_below(sum[j], lim)) low &= ~(1u << j);
+                }
+                oz_push(again, &nagain[turn], i * OZ_N + cg * 8, low);
+            }
             if (MODE == TC_TRAIL) {
                 if (rok)
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
-                        if (col0 + j < cend) dst[j * sj] = sum[j];
+                        if (col0 + j < cend && !((low >> j) & 1u)) dst[j * sj] = sum[j];
             } else if (rok) {
                 const int r = row - F.nf, c0 = col0 - F.nf;
                 const ScatterRow& R = tab[i];
@@ -3788,7 +3888,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_update(double* fac, unsign
                 for (int j = 0; j < 8; ++j) {
                     const int c = c0 + j;
                     pos[j] = -1;
-                    if (c < F.m && (r >= c || !S.sym)) pos[j] = r >= c ? S.rel[tab[umma::TM + cg * 8 + j].rel0 + r] : S.rel[R.rel0 + c];
+                    if (c < F.m && (r >= c || !S.sym) && !((low >> j) & 1u)) pos[j] = r >= c ? S.rel[tab[umma::TM + cg * 8 + j].rel0 + r] : S.rel[R.rel0 + c];
                 }
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
@@ -3803,6 +3903,35 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_oz_update(double* fac, unsign
                         atomicAdd(&fac[addr], -sum[j]);
                     }
                 }
+            }
+            // The entries to form again: eight lanes for each, along k, where they are few (their loads are what takes
+            // time), else a lane (the multiply-adds do; neighbours share a column)
+            if (et == 0) nagain[turn == 2 ? 0 : turn + 1] = 0;   // of the last but one tile, read by all before the last one's barrier
+            asm volatile("bar.sync 2, %0;" ::"n"(32 * TC_EPI) : "memory");
+            const int n = nagain[turn];
+            turn = turn == 2 ? 0 : turn + 1;
+            if (n > 0) {
+                const int k0 = S.blk_c0[T.b0], k1 = S.blk_c1[T.b0 + T.nb - 1], row0 = row - i, c0 = col0 - cg * 8;
+                const int along = n <= OZ_FEW ? 8 : 1, q = lane & (along - 1);
+                for (int e0 = (warp - 4) * (32 / along); e0 < n; e0 += TC_EPI * 32 / along) {
+                    const int e = e0 + lane / along;
+                    const bool ok = e < n;
+                    const int at = ok ? again[e] : 0, r = row0 + at / OZ_N, c = c0 + at % OZ_N;
+                    double* d = fac + (c < F.nf ? F.loff + (ll)c * F.ld + r : F.uoff + (ll)r * F.m + (c - F.nf));
+                    const double old = MODE == TC_TRAIL && ok ? *d : 0.0;
+                    double s = ok ? oz_sum(fac, F, r, c, k0 + q, k1, along) : 0.0;
+                    if (along == 8)
+#pragma unroll
+                        for (int off = 4; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+                    if (!ok || q != 0) continue;
+                    if (MODE == TC_TRAIL) {
+                        *d = old - s;
+                    } else {
+                        const ll t = oz_target(S.rel, tab[umma::TM + at % OZ_N], tab[at / OZ_N], r - F.nf, c - F.nf);
+                        if (t >= 0) atomicAdd(&fac[t], -s);
+                    }
+                }
+                asm volatile("bar.sync 2, %0;" ::"n"(32 * TC_EPI) : "memory");   // `again` is free
             }
             __syncwarp();
         }
