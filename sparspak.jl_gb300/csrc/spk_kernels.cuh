@@ -324,9 +324,13 @@ __device__ __forceinline__ bool warp_block_lu(T (&r)[W], int bw, int nrow, const
             const T c = r[k];
             const int ce = __shfl_sync(FULL, p1, k);
             const bool diag = pos == k, cand = act && (sym ? diag : pos < ce);
-            T rc;   // every candidate's reciprocal, beside the search
-            if constexpr (sizeof(T) == 4) rc = rcp_approx(c);
-            else rc = lu_recip(cand ? c : T(1));
+            T rc, rn = T(1);   // every candidate's reciprocal, beside the search; rn for the rows below the block
+            if constexpr (sizeof(T) == 4) {
+                rc = rcp_approx(c);
+                if (nrow > bw) rn = rcp_rn(cand ? c : T(1));
+            } else {
+                rc = rn = lu_recip(cand ? c : T(1));
+            }
             unsigned m;
             if constexpr (sizeof(T) == 4) {
                 const unsigned key = pivot_key32(c, cand, diag);
@@ -356,6 +360,10 @@ __device__ __forceinline__ bool warp_block_lu(T (&r)[W], int bw, int nrow, const
             if (pv == T(0)) {   // no scaling
                 inv = T(1);
                 sing = true;
+            }
+            if (nrow > bw) {   // below the block 1 / U(k, k) correctly rounded, as the panels take it
+                const T r21 = __shfl_sync(FULL, rn, kl);
+                if (lane >= bw) inv = r21;
             }
             if (pos == k) pos = pp;
             if (lane == kl) {
