@@ -1815,18 +1815,22 @@ __host__ __device__ __forceinline__ int panel_tile(int part, int tile, int nL, i
 // q, q + 8, .. (cyclic, so that step k touches only the entries after it: 288
 // instead of 1024 multiply-adds per 64-step sweep), and a CTA of four warps
 // takes 16 lines (64 before), four times as many CTAs for the few fronts near
-// the root.  rows: X := X inv(U_B) with the rows of U_B staged over their
-// diagonal, so that only the last step scales; cols: Y := inv(L_B) P_B Y.
-// 48^3 convection-diffusion: 18.0 -> 9.4 ms for all panels (FP64-bound: 5.6 ms
-// at the full rate).
+// the root.  rows: X := X inv(U_B), entry k scaled by 1 / U(k, k) at its step
+// (rows of U_B over their diagonal would spare that multiplication, but overflow
+// where columns of A differ by more than the exponent range, and round once
+// more); cols: Y := inv(L_B) P_B Y.
+// 48^3 convection-diffusion: 18.0 -> 10.0 ms for all panels (FP64-bound: 5.6 ms
+// at the full rate, without the scaling; 9.8 with the rows over their diagonal).
 constexpr int PD_LINES = 16, PD_LANES = 8;
 template <int W>
-__device__ __forceinline__ void sweep_f64(double (&x)[W / PD_LANES], const double* sT, int bw) {
+__device__ __forceinline__ void sweep_f64(double (&x)[W / PD_LANES], const double* sT, const double* rd, int bw) {   // rd null: cols
     constexpr int CQ = W / PD_LANES;
     const int lane = threadIdx.x & 31, q = lane & (PD_LANES - 1), base = lane & ~(PD_LANES - 1);
 #pragma unroll
-    for (int k = 0; k < W - 1; ++k)
-        if (k < bw - 1) {
+    for (int k = 0; k < W; ++k)
+        if (k < bw) {
+            if (rd && q == k % PD_LANES) x[k / PD_LANES] *= rd[k];
+            if (k == bw - 1) break;
             const double xk = __shfl_sync(0xffffffffu, x[k / PD_LANES], base | (k % PD_LANES));
             const double* t = sT + k * (W + 1) + q;
 #pragma unroll
@@ -1889,14 +1893,13 @@ __global__ void __launch_bounds__(128) k_block_panel_f64(double* fac, const int*
         __syncthreads();
         for (int e = tid; e < W * W; e += 128) {
             const int k = e % W, j = e / W;   // contiguous in k
-            sT[k * LD + j] = j > k && j < bw ? blkp[(ll)j * F.ld + k] * rd[k] : 0.0;
+            sT[k * LD + j] = j > k && j < bw ? blkp[(ll)j * F.ld + k] : 0.0;
         }
         __syncthreads();
-        sweep_f64<W>(x, sT, bw);
+        sweep_f64<W>(x, sT, rd, bw);
 #pragma unroll
         for (int jj = 0; jj < CQ; ++jj) {
             const int j = jj * PD_LANES + q;
-            if (j < bw) x[jj] *= rd[j];
             if (ok && j < bw) xp[(ll)j * F.ld] = x[jj];
         }
         if (S.blk_upack[blk] >= 0) oz_row_max<CQ>(x, ok, bw, smx, rexp + 2 * (F.f + c0) + 1);
@@ -1933,7 +1936,7 @@ __global__ void __launch_bounds__(128) k_block_panel_f64(double* fac, const int*
             sT[k * LD + i] = i > k && i < bw ? blkp[(ll)k * F.ld + (k < pa[i] ? gmap[i] : i)] : 0.0;
         }
         __syncthreads();
-        sweep_f64<W>(x, sT, bw);
+        sweep_f64<W>(x, sT, nullptr, bw);
 #pragma unroll
         for (int jj = 0; jj < CQ; ++jj) {
             const int k = jj * PD_LANES + q;
@@ -1960,7 +1963,7 @@ struct Lu64Smem {   // offsets in doubles
     static constexpr int BM = 64, LD = BM + 1, LT = LU_G + 1;
     static constexpr int a = 0;                       // A(i, j) at a + j * LD + i
     static constexpr int ex = a + BM * LD + 1;        // multipliers of the group's column k by row: ex + k * BM + row
-    static constexpr int t = ex + LU_G * BM;          // the group's triangles: U over its diagonal, row k at t + k * LT
+    static constexpr int t = ex + LU_G * BM;          // the group's triangles: U, row k at t + k * LT
     static constexpr int l = t + LU_G * LT;           // L11, column k at l + k * LT
     static constexpr int bytes = (l + LU_G * LT) * 8;
 };
@@ -2161,10 +2164,10 @@ __global__ void __launch_bounds__(LU64_THREADS) k_block_lu_f64(double* fac, int*
             if (lane + 32 < lim) col[lane + 32] = v1;
         }
         if (nr > 0) {
-            // U11 over its diagonal by rows, L11 by columns (as the rows eliminated: original rows' multipliers)
+            // U11 by rows, L11 by columns (as the rows eliminated: original rows' multipliers)
             for (int t = tid; t < w * LU_G; t += LU64_THREADS) {
                 const int k = t / LU_G, j = t % LU_G;
-                sT[k * LT + j] = j > k && j < w ? A[(a + j) * LD + a + k] * srd[k] : 0.0;
+                sT[k * LT + j] = j > k && j < w ? A[(a + j) * LD + a + k] : 0.0;
                 sL[k * LT + j] = j > k && j < w ? ex[k * BM + slsrc[j]] : 0.0;
             }
             __syncthreads();
@@ -2181,16 +2184,17 @@ __global__ void __launch_bounds__(LU64_THREADS) k_block_lu_f64(double* fac, int*
                     const int j = jj * PD_LANES + q;
                     y[jj] = ok && j < w ? line[j * ls] : 0.0;
                 }
-                sweep_f64<LU_G>(y, isU ? sL : sT, w);
+                if (isU) sweep_f64<LU_G>(y, sL, nullptr, w);
+                else sweep_f64<LU_G>(y, sT, srd, w);
 #pragma unroll
                 for (int jj = 0; jj < LU_G / PD_LANES; ++jj) {
                     const int j = jj * PD_LANES + q;
-                    if (ok && j < w) line[j * ls] = isU ? y[jj] : y[jj] * srd[j];
+                    if (ok && j < w) line[j * ls] = y[jj];
                 }
             }
             // a sliced piece's own later rows: their multipliers came out of the sweep in place
             __syncthreads();
-            // A22 -= L21 U12: a lane per row, eight columns per warp and pass
+            // A22 -= L21 U12: a lane per row, four columns per warp and pass
             for (int cq = wp; cq < cdiv(nr, 4); cq += NW)
                 for (int r = b + lane; r < b + cdiv(nr, 32) * 32; r += 32) {
                     const bool ok = r < bw;
