@@ -228,8 +228,6 @@ __device__ __forceinline__ T pickw(const T (&r)[W], int k) {
         return pickw<W / 2>(h, k);
     }
 }
-template <typename T>
-__device__ __forceinline__ T pick32(const T (&r)[32], int k) { return pickw<32>(r, k); }
 
 // One right-looking LU sweep over the columns [0, ncols) of a register block
 // held one row per lane (rows/columns below 32).  For column k in piece
@@ -497,26 +495,33 @@ __device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
 struct LuSweep {
     float* lu;    // L and U by position: entry (i, j) at lu + i * LU_LSW + j (up to 64 rows)
     float* lt;    // the first w rows transposed: entry (i, j) at lt + j * LU_LSW + i
-    float* ex;    // exchange: multipliers of column k by row (ex + k * 64), or work space of the general form
+    float* ex;    // exchange: multipliers of column k by row (ex + k * 64)
     float* rd;    // per column, the reciprocal of its pivot (1 for a zero pivot: no scaling)
     int* piv;     // per column, row | position << 8 of the pivot (position before the interchange)
     int* lsrc;    // original row now at each position
     int* at;      // position of each original row
     int* bad;     // set when the group has to be repeated by a more general form
+    int* zero;    // least column with a zero pivot (LU_GENERAL), counted from the block's first: the group's is a
+    int a;
 };
 
 // Called by warps q = 0 .. cdiv(w, 8) - 1; A is only read, so that a group can
 // be repeated.  RPL: rows per lane (at most 32 RPL rows).  cend: in lane k,
 // the end of the candidate positions of column k (its piece's end; k + 1 in
 // the symmetric form, where the diagonal row is the only candidate).
-//   SEARCH = false: the diagonal row is taken as every column's pivot and
-//     each candidate is checked against it beside the chain; *bad is set when
-//     one is larger.  Nothing of the chain waits for a search then: a column
-//     is two shuffles and a multiply-add.
-//   SEARCH = true: a reduction and a vote find the pivot.
-// Both set *bad for a column whose pivot is not unique, not finite, or not
-// normal (as its reciprocal).
-template <bool SEARCH, int RPL>
+//   LU_DIAG: the diagonal row is taken as every column's pivot and each
+//     candidate is checked against it beside the chain; *bad is set when one is
+//     larger.  Nothing of the chain waits for a search then: a column is two
+//     shuffles and a multiply-add.
+//   LU_SEARCH: a reduction and a vote find the pivot, the first position among
+//     equal ones.
+//   LU_GENERAL: the same with zero pivots (no scaling), NaN (never wins, except
+//     on the diagonal) and reciprocals outside the normal range, for which the
+//     other two set *bad.
+// A 120-column block with pivots of the one kind throughout: 29, 37 (equal values
+// or not) and 63 us.
+constexpr int LU_DIAG = 0, LU_SEARCH = 1, LU_GENERAL = 2;
+template <int MODE, int RPL>
 __device__ __forceinline__ void lu_sweep(const float* A, int lda, int nrow, int w, int cend, const LuSweep& O, int q) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, nq = cdiv(w, LU_W);
@@ -553,7 +558,7 @@ __device__ __forceinline__ void lu_sweep(const float* A, int lda, int nrow, int 
     auto place = [&](int k, int kl, int ks, int pp) {
 #pragma unroll
         for (int s = 0; s < RPL; ++s) {
-            if (SEARCH && pos[s] == k) pos[s] = pp;
+            if (MODE != LU_DIAG && pos[s] == k) pos[s] = pp;
             if (lane == kl && s == ks) {
                 pos[s] = k;
                 act[s] = false;
@@ -572,11 +577,11 @@ __device__ __forceinline__ void lu_sweep(const float* A, int lda, int nrow, int 
             for (int c = 0; c < 2; ++c) {
 #pragma unroll
                 for (int s = 0; s < RPL; ++s) l[c][s] = O.ex[(k + c) * 64 + lane + 32 * s];
-                if (SEARCH) pv[c] = O.piv[k + c];
+                if (MODE != LU_DIAG) pv[c] = O.piv[k + c];
             }
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                const int kr = SEARCH ? pv[c] & 255 : k + c;
+                const int kr = MODE != LU_DIAG ? pv[c] & 255 : k + c;
                 place(k + c, kr & 31, kr >> 5, pv[c] >> 8);
                 update(0, kr & 31, kr >> 5, l[c]);
             }
@@ -594,11 +599,13 @@ __device__ __forceinline__ void lu_sweep(const float* A, int lda, int nrow, int 
         }
         int kl = k, ks = 0, pp = k;
         float inv;
-        if constexpr (SEARCH) {
+        if constexpr (MODE != LU_DIAG) {
             unsigned key[RPL], best = 0u, m = 0u, dup = 0u;
 #pragma unroll
             for (int s = 0; s < RPL; ++s) {
-                key[s] = act[s] && pos[s] < ce ? __float_as_uint(c[s]) & 0x7fffffffu : 0u;   // NaN above infinity: caught below
+                const bool cand = act[s] && pos[s] < ce;
+                if (MODE == LU_GENERAL) key[s] = pivot_key32(c[s], cand, pos[s] == k);
+                else key[s] = cand ? __float_as_uint(c[s]) & 0x7fffffffu : 0u;   // NaN above infinity: caught below
                 best = max(best, key[s]);
             }
             const unsigned mx = __reduce_max_sync(FULL, best);
@@ -609,9 +616,30 @@ __device__ __forceinline__ void lu_sweep(const float* A, int lda, int nrow, int 
                 if (b) ks = s;
                 m |= b;
             }
-            kl = 31 - __clz(m);   // the only lane, or the group is repeated
-            bad |= dup != 0u || mx - 0x00800000u > 0x7e000000u - 0x00800000u;
-            inv = __shfl_sync(FULL, RPL == 2 && ks ? r[RPL - 1] : r[0], kl);
+            kl = 31 - __clz(m);
+            if (dup && mx) {   // equal values: the first position
+                unsigned p = 0xffffffffu;
+#pragma unroll
+                for (int s = 0; s < RPL; ++s)
+                    if (key[s] == mx) p = min(p, (unsigned)pos[s]);
+                p = __reduce_min_sync(FULL, p);
+#pragma unroll
+                for (int s = 0; s < RPL; ++s) {
+                    const unsigned b = __ballot_sync(FULL, key[s] == mx && (unsigned)pos[s] == p);
+                    if (b) {
+                        ks = s;
+                        kl = 31 - __clz(b);
+                    }
+                }
+            }
+            if constexpr (MODE == LU_GENERAL) {
+                const float pv = __shfl_sync(FULL, RPL == 2 && ks ? c[RPL - 1] : c[0], kl);
+                inv = pv != 0.0f ? lu_recip(pv) : 1.0f;
+                if (pv == 0.0f && lane == 0) atomicMin(O.zero, O.a + k);
+            } else {
+                bad |= mx - 0x00800000u > 0x7e000000u - 0x00800000u;
+                inv = __shfl_sync(FULL, RPL == 2 && ks ? r[RPL - 1] : r[0], kl);
+            }
             pp = __shfl_sync(FULL, RPL == 2 && ks ? pos[RPL - 1] : pos[0], kl);
         } else {
             inv = __shfl_sync(FULL, r[0], k);
@@ -628,7 +656,7 @@ __device__ __forceinline__ void lu_sweep(const float* A, int lda, int nrow, int 
             O.ex[k * 64 + lane + 32 * s] = l[s];
             if (lane == kl && s == ks) {
                 O.piv[k] = (kl + 32 * ks) | pp << 8;
-                O.rd[k] = r[s];
+                O.rd[k] = inv;
             }
         }
         if ((t & 1) && q + 1 < nq) asm volatile("bar.arrive %0, %1;" ::"r"(4 + t / 2), "r"(32 * (nq - q)) : "memory");
@@ -666,69 +694,6 @@ __device__ __forceinline__ void lu_sweep(const float* A, int lda, int nrow, int 
                 for (int j = 0; j < LU_W; ++j)
                     O.lt[(q * LU_W + j) * LU_LSW + i] = (j & 1) ? f2_hi(P[s][j / 2]) : f2_lo(P[s][j / 2]);
         }
-}
-
-// General form, by one warp (up to 64 rows, at slots lane and lane + 32): the
-// same with ties (the first position wins), zero pivots (no scaling), NaN
-// (never wins, except on the diagonal) and reciprocals outside the normal
-// range.  The rows stay in O.ex, column k of row r at ex[k * 64 + r].
-// Returns the first step with a zero pivot, or LU_G.
-__device__ __noinline__ int lu_sweep_general(const float* A, int lda, int nrow, int w, int cend, const LuSweep& O, bool sym) {
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    int pos[2] = {lane, lane + 32}, zero = LU_G;
-    bool act[2] = {lane < nrow, lane + 32 < nrow};
-    for (int j = 0; j < w; ++j)
-        for (int s = 0; s < 2; ++s)
-            if (lane + 32 * s < nrow) O.ex[j * 64 + lane + 32 * s] = A[j * lda + lane + 32 * s];
-    __syncwarp();
-    for (int k = 0; k < w; ++k) {
-        const int ce = __shfl_sync(FULL, cend, k);
-        float c[2];
-        unsigned key[2];
-        for (int s = 0; s < 2; ++s) {
-            c[s] = act[s] ? O.ex[k * 64 + lane + 32 * s] : 0.0f;
-            key[s] = pivot_key32(c[s], act[s] && (sym ? pos[s] == k : pos[s] < ce), pos[s] == k);
-        }
-        const unsigned mx = __reduce_max_sync(FULL, max(key[0], key[1]));
-        unsigned p = 0xffffffffu;   // the first position holding it
-        for (int s = 0; s < 2; ++s)
-            if (key[s] == mx) p = min(p, (unsigned)pos[s]);
-        p = __reduce_min_sync(FULL, p);
-        const unsigned b0 = __ballot_sync(FULL, act[0] && pos[0] == (int)p), b1 = __ballot_sync(FULL, act[1] && pos[1] == (int)p);
-        const int kr = b0 ? __ffs(b0) - 1 : 31 + __ffs(b1);   // the pivot row
-        const float pv = O.ex[k * 64 + kr];
-        const float inv = pv != 0.0f ? lu_recip(pv) : 1.0f;
-        if (pv == 0.0f) zero = min(zero, k);
-        if (lane == 0) {
-            O.piv[k] = kr | (int)p << 8;
-            O.rd[k] = inv;
-        }
-        for (int s = 0; s < 2; ++s) {
-            if (pos[s] == k) pos[s] = (int)p;
-            if (lane + 32 * s == kr) {
-                pos[s] = k;
-                act[s] = false;
-            }
-            if (act[s]) {
-                const float l = c[s] * inv;
-                O.ex[k * 64 + lane + 32 * s] = l;
-                for (int j = k + 1; j < w; ++j) O.ex[j * 64 + lane + 32 * s] -= l * O.ex[j * 64 + kr];
-            }
-        }
-        __syncwarp();
-    }
-    for (int s = 0; s < 2; ++s)
-        if (lane + 32 * s < nrow) {
-            O.at[lane + 32 * s] = pos[s];
-            O.lsrc[pos[s]] = lane + 32 * s;
-            for (int j = 0; j < w; ++j) {
-                const float v = O.ex[j * 64 + lane + 32 * s];
-                O.lu[pos[s] * LU_LSW + j] = v;
-                if (pos[s] < LU_G) O.lt[j * LU_LSW + pos[s]] = v;
-            }
-        }
-    return zero;
 }
 
 struct LuSmem {   // offsets in floats
@@ -858,48 +823,40 @@ __global__ void __launch_bounds__(LU_THREADS, 1) k_block_lu_f32(float* fac, int*
         gs[n] = bw;
         ngrp = n;
     }
-    const LuSweep O{lu, sm + SM::lt, sm + SM::ex, srd, spv, lsrc, sat, &sbad};
+    LuSweep O{lu, sm + SM::lt, sm + SM::ex, srd, spv, lsrc, sat, &sbad, &szero, 0};
     // part 1 of group [a, b), rows to e (warps 0..3)
-    auto sweep = [&](int a, int b, int e, bool search) {
+    auto sweep = [&](int a, int b, int e, int mode) {
         const int w = b - a, nrow = e - a;
+        O.a = a;
         if (wp >= cdiv(w, LU_W)) return;
         const int cend = lane < w ? (sym ? lane + 1 : cpb[a + lane] - a) : 0;
         const float* D = A + a * LD + a;
         if (nrow <= 32) {
-            if (search) lu_sweep<true, 1>(D, LD, nrow, w, cend, O, wp);
-            else lu_sweep<false, 1>(D, LD, nrow, w, cend, O, wp);
+            if (mode == LU_DIAG) lu_sweep<LU_DIAG, 1>(D, LD, nrow, w, cend, O, wp);
+            else if (mode == LU_SEARCH) lu_sweep<LU_SEARCH, 1>(D, LD, nrow, w, cend, O, wp);
+            else lu_sweep<LU_GENERAL, 1>(D, LD, nrow, w, cend, O, wp);
         } else {
-            lu_sweep<true, 2>(D, LD, nrow, w, cend, O, wp);
+            if (mode != LU_GENERAL) lu_sweep<LU_SEARCH, 2>(D, LD, nrow, w, cend, O, wp);
+            else lu_sweep<LU_GENERAL, 2>(D, LD, nrow, w, cend, O, wp);
         }
     };
     __syncthreads();
     const int ng = ngrp;
-    bool search = false;   // once a group needed an interchange, look for the pivots of the next ones
-    if (wp < 4) sweep(gs[0], gs[1], ge[0], search);
+    int mode = LU_DIAG;   // a group that needs a more general form starts the next ones with it
+    if (wp < 4) sweep(gs[0], gs[1], ge[0], mode);
     __syncthreads();
     int done = 0;   // columns [0, done) and their rows are written out
 #pragma unroll 1
     for (int g = 0; g < ng; ++g) {
         const int a = gs[g], b = gs[g + 1], w = b - a, e = ge[g], nrow = e - a;
         const bool moved = e > b || cpa[a] < a;
-        if (sbad) {   // the diagonal was not every column's pivot: search
-            const bool again = !search && !sym && nrow <= 32;
+        for (int again = sbad; again; again = sbad) {   // (the symmetric form has nothing to search)
+            mode = mode == LU_DIAG && !sym && nrow <= 32 ? LU_SEARCH : LU_GENERAL;
             __syncthreads();
-            if (again) {
-                if (tid == 0) sbad = 0;
-                search = true;
-                __syncthreads();
-                if (wp < 4) sweep(a, b, e, true);
-                __syncthreads();
-            }
-            if (!again || sbad) {   // an exceptional pivot
-                if (wp == 0) {
-                    const int z = lu_sweep_general(A + a * LD + a, LD, nrow, w, lane < w ? cpb[a + lane] - a : 0, O, sym);
-                    if (lane == 0 && z < LU_G) szero = min(szero, a + z);
-                }
-                __syncthreads();
-                if (tid == 0) sbad = 0;
-            }
+            if (tid == 0) sbad = 0;
+            __syncthreads();
+            if (wp < 4) sweep(a, b, e, mode);
+            __syncthreads();
         }
         if (moved) {
             // a slice of a wide piece: its interchanges move whole rows, over
@@ -992,7 +949,7 @@ __global__ void __launch_bounds__(LU_THREADS, 1) k_block_lu_f32(float* fac, int*
             asm volatile("bar.sync 1, 256;" ::: "memory");
         }
         if (wp < 4) {
-            sweep(b, b2, e2, search);
+            sweep(b, b2, e2, mode);
         } else {
             for (int c = wp - 4; c < cdiv(nr, 4); c += NW - 4) lu_rank_quad(D, sl, su, w, c < cn ? rn : 0, nr, c, nr);
             if (e == b) {   // whole pieces: their columns, and their rows right of them, are final
