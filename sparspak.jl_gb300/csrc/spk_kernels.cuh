@@ -191,12 +191,13 @@ __device__ __forceinline__ float rcp_approx(float x) {   // normal x whose recip
 
 // Scaling factor 1 / pivot of the FP32 block LU: the hardware reciprocal
 // (within 2 ulp; the FP32 factor is refined in FP64); FP64 keeps the
-// correctly rounded one.  __fdividef covers the pivots whose reciprocal is
-// not normal; everywhere else it costs 140 cycles of a column's chain where
-// the bare instruction takes 20 (measured in a loop of one warp).
+// correctly rounded one, and so do the FP32 pivots whose reciprocal is not
+// normal (__fdividef would give 0 above 2^126).  In a column's chain
+// __fdividef costs 140 cycles where the bare instruction takes 20 (measured in
+// a loop of one warp).
 __device__ __forceinline__ float lu_recip(float x) {
     const float a = fabsf(x);
-    return a >= 1.1754944e-38f && a <= 8.5070592e37f ? rcp_approx(x) : __fdividef(1.0f, x);
+    return a >= 1.1754944e-38f && a <= 8.5070592e37f ? rcp_approx(x) : rcp_rn(x);
 }
 __device__ __forceinline__ double lu_recip(double x) { return rcp_rn(x); }
 

@@ -1,6 +1,7 @@
-"""The FP32 block LU where its pivots tie or are NaN, in every group of a block:
-identical pivots to the oracle's, factors equal to the bit (ties: arithmetic on
-powers of two) or within FP32 rounding (n u times an elimination growth below 4
+"""The FP32 block LU where its pivots tie, are zero or NaN, or have reciprocals
+outside the normal range, in every group of a block: identical pivots to the
+oracle's, factors equal to the bit (ties: arithmetic on powers of two) or
+within FP32 rounding, column by column (n u times an elimination growth below 4
 for the diagonally dominant matrices, as in the tests of the block LU)."""
 import numpy as np
 import pytest
@@ -48,6 +49,37 @@ def test_ties_in_every_group(n, maxblocksize):
     o = factors(s, p, M)
     assert np.array_equal(s.slvr.ipiv, o.ipiv)
     assert np.array_equal(s.slvr.lnz, o.lnz)
+
+
+def large(n):
+    """Factors that bring some of the diagonal entries of 2 n above 2^126."""
+    big = np.ones(n)
+    big[::9] = 2.0 ** (127 - np.floor(np.log2(2.0 * n)))
+    return big
+
+
+@pytest.mark.parametrize("n", [40, 128, 200])
+def test_reciprocals_outside_the_normal_range(n):
+    s, p = solver(n, 30)
+    M = np.random.default_rng(n).standard_normal((n, n)) + 2.0 * n * np.eye(n)
+    o = factors(s, p, M * large(n))
+    assert np.array_equal(s.slvr.ipiv, o.ipiv)
+    x = s.slvr.xlnz[:-1] - 1
+    assert np.all(np.maximum.reduceat(np.abs(s.slvr.lnz - o.lnz), x) <= 5e-5 * np.maximum.reduceat(np.abs(o.lnz), x))
+
+
+@pytest.mark.parametrize("n", [40, 128, 200])
+def test_reciprocals_outside_the_normal_range_spd(n):
+    s, p = solver(n, 30, spd=True)
+    M = np.random.default_rng(n).standard_normal((n, n))
+    M = np.tril(M) + np.tril(M, -1).T
+    np.fill_diagonal(M, 2.0 * n * large(n))
+    factors(s, p, M)
+    C = np.linalg.cholesky(M)
+    for j in range(n):
+        f = int(s.slvr.xsuper[s.slvr.snode[j] - 1]) - 1
+        got = s.slvr.lnz[s.slvr.xlnz[j] - 1: s.slvr.xlnz[j + 1] - 1][j - f:]
+        assert np.max(np.abs(got - C[j:, j])) <= 5e-5 * np.max(np.abs(C[j:, j]))
 
 
 @pytest.mark.parametrize("n", [40, 128])   # one block: the panels spread a NaN through their padded triangles
