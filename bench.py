@@ -510,7 +510,7 @@ def run_ours(args):
         """DRAM bytes per launch of the class's FP32 kernels from the committed ncu summaries: the block-LU
         class from sampled 64^3 launches (DRAM / algorithmic bytes of a one-block launch, scaled by the
         blocks a launch processes), the others from the 40^3 capture."""
-        p64 = os.path.join(ROOT, "profiles", "dram_traffic_k_block_lu_laplace3d64.md")
+        p64 = os.path.join(ROOT, "profiles", "dram_traffic_k_block_lu_f32_laplace3d64.md")
         if cls == "getrf" and alg_per_launch and os.path.exists(p64):
             ratio = None
             for line in open(p64):
@@ -518,16 +518,18 @@ def run_ours(args):
                     ratio = float(line.split()[1].rstrip("x"))
             if ratio:
                 return ratio * alg_per_launch, (
-                    f"64^3: ncu dram__bytes_read.sum + dram__bytes_write.sum of sampled one-block k_block_lu "
+                    f"64^3: ncu dram__bytes_read.sum + dram__bytes_write.sum of sampled one-block k_block_lu_f32 "
                     f"launches is {ratio:.2f}x their algorithmic bytes "
-                    f"(profiles/dram_traffic_k_block_lu_laplace3d64.md); scaled by the algorithmic bytes per "
+                    f"(profiles/dram_traffic_k_block_lu_f32_laplace3d64.md); scaled by the algorithmic bytes per "
                     f"launch of the class (the same ratio taken for its small-front kernels)")
-        names = {"getrf": ("k_block_lu<float>", "k_block_lu_small<float>", "k_leaf_factor<float>"),
+        names = {"getrf": ("k_block_lu_f32", "k_block_lu_small<float>", "k_leaf_factor"),
                  "panel": ("k_block_panel<float",),
                  "trail": ("k_block_trail<float>",), "schur": ("k_schur<float>",),
-                 "tc_trail": ("k_tc_update<0>",), "tc_schur": ("k_tc_update<1>",),
-                 "fwd": ("k_fwd<float>", "k_front_solve<float, 1,", "k_fwd_l21<float>", "k_solve_leaf<float, 1>"),
-                 "bwd": ("k_bwd<float>", "k_bwd_u12<float>", "k_front_solve<float, 0,", "k_solve_leaf<float, 0>")}.get(cls, ())
+                 "tc_trail": ("k_tc_update<0,",), "tc_schur": ("k_tc_update<1,",),
+                 "fwd": ("k_fwd<float>", "k_front_solve<float, 1,", "k_fwd_l21<float", "k_solve_leaf<float, 1,",
+                         "k_solve_leaf_set<float, 1,"),
+                 "bwd": ("k_bwd<float>", "k_bwd_u12<float", "k_front_solve<float, 0,", "k_solve_leaf<float, 0,",
+                         "k_solve_leaf_set<float, 0,")}.get(cls, ())
         path = os.path.join(ROOT, "profiles", "dram_traffic_laplace3d40_mixed_step.md")
         if not names or not os.path.exists(path):
             return None, None

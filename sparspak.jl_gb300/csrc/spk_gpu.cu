@@ -158,7 +158,7 @@ template <typename T>
 struct Storage {
     T* d = nullptr;
     T* inv2 = nullptr;      // whole-block forward / backward operators
-    unsigned char* pack = nullptr;   // packed panels of the tensor-core fronts (FP64: integer slices)
+    unsigned char* pack = nullptr;   // packed panels of the tensor-core fronts (FP64: integer slices, one level's at a time)
     ll slice_bytes = 0;     // FP64: what the slices take; no_slices: refused when last asked for
     bool no_slices = false;
     bool loaded = false;    // values assembled since the last factor
@@ -520,10 +520,12 @@ static int analyse(spk_handle* h, const int64_t* xsuper, const int64_t* snode, c
     // whole front in one launch, so a longer chain of smaller ones only adds
     // launches (a tridiagonal system of 1101 unknowns: 551 levels of one- and
     // two-column fronts without this, 4.7 ms a refactorisation and solve, 36
-    // levels with it, 1.8 ms; 512 batched systems: 1.44 M fronts in 18 levels,
-    // 17.8 ms, 451,000 in 14 levels, 14.3 ms).  Up to 8 columns takes 1.4 and
-    // 15.0 ms, up to 32 columns 2.6 and 14.9 ms, up to 64 rows below them 24.9
-    // instead of 24.1 ms for a 64^3 step.
+    // levels with it, 1.3 ms; 512 batched systems: 1.44 M fronts in 18 levels,
+    // 17.8 ms, 451,000 in 14 levels, 14.1 ms).  When the width was chosen: up to
+    // 8 columns 1.4 and 15.0 ms, 16 columns 1.8 and 14.3, 32 columns 2.6 and
+    // 14.9; up to 64 rows below them 24.9 instead of 24.1 ms for a 64^3 step.
+    // Entries stored against the exact storage: 3-D grids 1.01 to 1.04 times,
+    // 2-D and the batched systems 1.12 to 1.18, a tridiagonal system 6.0.
     h->col_front.assign(n, -1);
     h->fronts.clear();
     auto exact_entries = [&](i64 t) {

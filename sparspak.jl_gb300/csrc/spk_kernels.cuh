@@ -3362,13 +3362,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc_update(float* fac, const u
 // 32 (8 - i) columns, whose products are weights i .. 7: eight MMAs per 16
 // columns where one per pair was 36, of 95 cycles each up to 64 columns.  The
 // weights are joined and rounded by integer instructions (oz_join).  What
-// bounds it now is latency, no pipe is above a third: a tile's chain of copies
-// (160 KB), accumulator loads, joins and target accesses, 13,900 cycles per
-// 128 x 32 x 64 product; 12 TFLOP/s on a 4096 x 4096 x 64 update where the
-// multiply-add tiles give 1.05.  48^3 convection-diffusion, rank updates:
-// 131 -> 20.3 ms (23.5 with an MMA per pair and FP64 joins).  Two groups of
-// epilogue warps on alternate tiles, and eight warps with twice the registers,
-// took 21.1 and 22.4 ms.
+// bounds it now is latency: a tile's chain of copies (160 KB), accumulator
+// loads, joins and target accesses (issue slots 37 to 41% busy in the Schur
+// form, no pipe above 43%, ALU first).  48^3 convection-diffusion, rank updates:
+// 131 -> 17.9 ms (16.5 without the second sums; 23.5 with an MMA per pair and
+// FP64 joins, before there were any).  Two groups of epilogue warps on alternate
+// tiles, and eight warps with twice the registers, were 4 and 10% slower.
 // ---------------------------------------------------------------------------
 constexpr int OZ_D = 8, OZ_N = 32;                       // digits, tile columns
 constexpr int OZ_SLICE = umma::PCHUNK16;                 // one slice of a 128-line tile and 16 columns, 4 KB

@@ -76,19 +76,21 @@ SPK_HOST, SPK_DEVICE = 0, 1
 KERNEL_CLASSES = ["assemble", "getrf", "panel", "trail", "schur", "fwd", "bwd", "permute", "residual", "blockinv",
                   "tc_trail", "tc_schur"]
 KERNEL_NAMES = {"assemble": "k_scatter_values",
-                "getrf": "k_block_lu_pc+k_block_lu_f32+k_block_lu_f64+k_block_lu_small+k_leaf_factor+k_leaf_queue",
+                "getrf": "k_block_lu_pc+k_block_lu_f32+k_block_lu_f64+k_block_lu_small+k_leaf_factor+k_leaf_factor_set+k_leaf_queue",
                 "panel": "k_block_panel+k_block_panel_f64+k_oz_pack",
                 "trail": "k_block_trail", "schur": "k_schur",
-                "fwd": "k_fwd+k_front_solve<fwd>+k_fwd_l21+k_solve_leaf<fwd>",
-                "bwd": "k_bwd_u12+k_bwd+k_front_solve<bwd>+k_solve_leaf<bwd>", "permute": "k_permute+k_unpermute",
+                "fwd": "k_fwd+k_tfwd+k_front_solve<fwd>+k_front_gemv+k_front_gemv_t+k_fwd_l21+k_solve_leaf<fwd>+k_solve_leaf_set<fwd>",
+                "bwd": "k_bwd_u12+k_bwd+k_tbwd_l21+k_tbwd+k_front_solve<bwd>+k_front_gemv+k_front_gemv_t+k_solve_leaf<bwd>"
+                       "+k_solve_leaf_set<bwd>", "permute": "k_permute+k_unpermute",
                 "residual": "k_residual", "blockinv": "k_block_inv",
                 "tc_trail": "k_tc_update<TC_TRAIL>+k_oz_update<TC_TRAIL>",
                 "tc_schur": "k_tc_update<TC_SCHUR>+k_oz_update<TC_SCHUR>"}
-# How each class's FP32 form computes: tensor cores (tcgen05, 3xTF32) or CUDA cores.
-KERNEL_UNITS = {"tc_trail": "tcgen05 kind::tf32, 3xTF32 per term", "tc_schur": "tcgen05 kind::tf32, 3xTF32 per term",
+# How each class computes: tensor cores (tcgen05) or CUDA cores.
+_UPDATES = "tcgen05: FP32 kind::tf32, 3xTF32 per term; BF16S kind::f16; FP64 kind::f16 on eight BF16 digits per entry"
+KERNEL_UNITS = {"tc_trail": _UPDATES, "tc_schur": _UPDATES,
                 "trail": "FP32/FP64 FMA (fronts without a pack)", "schur": "FP32/FP64 FMA (fronts without a pack)",
-                "getrf": "FP32 FMA, latency-bound (one CTA per front, sequential pivot columns; small fronts a warp each)",
-                "panel": "FP32 FMA (register-line triangular sweeps)"}
+                "getrf": "FP32/FP64 FMA, latency-bound (one CTA per front, sequential pivot columns; small fronts a warp each)",
+                "panel": "FP32/FP64 FMA (register-line triangular sweeps; k_oz_pack: integer)"}
 SPK_FP64, SPK_FP32, SPK_BF16S = 0, 1, 2
 SPK_SPD = 16   # or-ed with a precision: the symmetric (SPD, Cholesky) form
 SPK_SOLVER_AUTO, SPK_SOLVER_IR, SPK_SOLVER_GMRES = 0, 1, 2
