@@ -136,3 +136,32 @@ def test_finite_columns_beside_a_non_finite_entry(bad):
     assert np.all(np.isfinite(F[:150, :150])) and np.all(np.isfinite(G[:150, :150]))
     both = np.isfinite(F) & np.isfinite(G)
     assert np.max(np.abs(F[both] / G[both] - 1.0)) <= n * 2.0 ** -53
+
+
+@pytest.mark.parametrize("spd", [False, True])
+@pytest.mark.parametrize("power", [20, 40])
+def test_large_columns_of_a_grid(power, spd):
+    # Schur complements over several blocks: some unknowns of a 3-D grid in other units (rows and columns in the
+    # symmetric form), against the oracle's solution in the old ones; 1e-12 is the accuracy asked of plain FP64 solves
+    # of these grids (condition number below 1e3)
+    k = 16
+    A = S.gallery.laplacian((k, k, k), shift=1e-3) if spd else S.gallery.convection_diffusion(k=k)
+    n = A.shape[0]
+    big = np.ones(n)
+    big[np.random.default_rng(3).choice(n, 40, replace=False)] = 2.0 ** power
+    B = sp.csc_matrix(A)
+    B.data = B.data * np.repeat(big, np.diff(B.indptr)) * (big[B.indices] if spd else 1.0)
+    s = S.SparseSolver(B, spd=spd)
+    S.findorder_(s, S.nd_grid(k, k, k))
+    S.symbolicfactor_(s)
+    S.inmatrix_(s)
+    s.slvr.engine.profile_reset()
+    S.factor_(s)
+    assert s.slvr.engine.profile_read()["tc_schur"]["launches"] > 0
+    o = oracle.OracleLU(s.slvr)
+    o.inmatrix_csc(*_matrix_arrays(sp.csc_matrix(A)))   # in the units it was in
+    assert o.factor() == 0
+    b = S.gallery.random_rhs(n, 1, seed=2).ravel()
+    x = s.slvr.engine.solve(b * (big if spd else 1.0), "fp64+spd" if spd else "fp64").ravel() * big
+    ref = o.solve(b).ravel()
+    assert np.max(np.abs(x - ref)) <= 1e-12 * np.max(np.abs(ref))
